@@ -137,7 +137,7 @@ class _Embed(torch.autograd.Function):
     @staticmethod
     def forward(ctx, wte, wpe, ids, first):
         b, s = ids.shape
-        flat = ids.reshape(-1)
+        flat = ids.reshape(-1).contiguous()   # a column of a wider tensor is a strided view, and the kernels read consecutive ids
         e = F.embedding(flat, wte)
         if wpe is not None:
             e.view(b, s, -1).add_(wpe[first:first + s])
