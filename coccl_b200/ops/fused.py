@@ -154,16 +154,41 @@ class _Embed(torch.autograd.Function):
         wte, wpe = ctx.tables
         b, s, first = ctx.meta
         T, H = b * s, wte.shape[1]
-        dy = dy.contiguous() if aligned16(dy) else dy.clone(memory_format=torch.contiguous_format)
-        order = torch.empty(T, dtype=torch.int32, device=dy.device)
+        (node_w, _), (node_p, _) = ctx.next_functions[:2]
+        grads, straight = [None, None], []
+        for i, (w, node) in enumerate(((wte, node_w), (wpe, node_p))):
+            want = _wanted_gradient(w, node)
+            straight.append(want == "buffer")
+            if want == "tensor" and i == 0:
+                grads[0] = torch.ops.aten.embedding_dense_backward(dy, flat, wte.shape[0], -1, False)
+            elif want == "tensor":
+                grads[1] = F.pad(dy.reshape(b, s, H).sum(0), (0, 0, first, wpe.shape[0] - first - s))
+        if any(straight):
+            dy = dy.contiguous() if aligned16(dy) else dy.clone(memory_format=torch.contiguous_format)
         lib, st = _lib.lib(), _lib.cur_stream()
-        _lib.check(lib.cocclkEmbedOrder(flat.data_ptr(), order.data_ptr(), T, st), "cocclkEmbedOrder")
-        _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), flat.data_ptr(), order.data_ptr(), wte.main_grad.data_ptr(), T, H, wte.shape[0], st),
-                   "cocclkEmbedBwd")
-        if wpe is not None:
+        if straight[0]:
+            order = torch.empty(T, dtype=torch.int32, device=dy.device)
+            _lib.check(lib.cocclkEmbedOrder(flat.data_ptr(), order.data_ptr(), T, st), "cocclkEmbedOrder")
+            _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), flat.data_ptr(), order.data_ptr(), wte.main_grad.data_ptr(), T, H,
+                                          wte.shape[0], st), "cocclkEmbedBwd")
+        if straight[1]:
             g = wpe.main_grad[first:first + s]
             _lib.check(lib.cocclkEmbedPositionsBwd(dy.data_ptr(), g.data_ptr(), b, s, H, st), "cocclkEmbedPositionsBwd")
-        return None, None, None, None
+        return grads[0], grads[1], None, None
+
+
+def _wanted_gradient(w, node) -> str:
+    """How this backward pass wants the gradient of table `w` (`node`: where autograd would accumulate it): "buffer" (straight
+    into `main_grad`), "tensor" (as a tensor: hooks on the table see and may change it, torch.autograd.grad returns it, a pass
+    with create_graph differentiates it) or "none" (backward(inputs=...) of other tensors)."""
+    if w is None or node is None:
+        return "none"
+    try:
+        if not torch._C._will_engine_execute_node(node):
+            return "none"
+    except RuntimeError:   # a leaf whose gradient torch.autograd.grad captures
+        return "tensor"
+    return "tensor" if torch.is_grad_enabled() or w._backward_hooks or w._post_accumulate_grad_hooks else "buffer"
 
 
 def embed_fits(ids, wte, wpe=None, first: int = 0) -> bool:
@@ -180,7 +205,7 @@ def embed_fits(ids, wte, wpe=None, first: int = 0) -> bool:
 
 def embed(ids, wte, wpe=None, first: int = 0):
     """wte[ids] (+ wpe[first + position]) as [tokens, hidden] for ids [batch, seq]; the gradients are added to the tables'
-    `main_grad` in fp32 (the caller has checked embed_fits)."""
+    `main_grad` in fp32 (the caller has checked embed_fits), or handed to autograd where something wants to see them."""
     return _Embed.apply(wte, wpe, ids, first)
 
 

@@ -4,6 +4,7 @@ import ctypes
 
 import pytest
 import torch
+import torch.nn.functional as F
 
 from coccl_b200 import _lib
 from coccl_b200.ops import fused
@@ -66,3 +67,42 @@ def test_embedding_gradient_follows_the_ids_whatever_their_strides(embed_kernels
     e.backward(dy)
     want = torch.zeros(40, 8).index_add_(0, ids.reshape(-1), dy.float())
     assert torch.allclose(wte.main_grad, want, atol=1e-5)
+
+
+def _embedded(embed_kernels):
+    """A pass through the tables with its gradients as autograd's own operations give them."""
+    k, wte, wpe = embed_kernels
+    ids = torch.tensor([[3, 3, 5], [0, 39, 5]])
+    dy = torch.randn(6, 8, generator=torch.Generator().manual_seed(5)).to(torch.bfloat16)
+    a, b = (t.detach().clone().requires_grad_(True) for t in (wte, wpe))
+    (F.embedding(ids, a) + b[2:5]).reshape(6, 8).backward(dy)
+    return k, wte, wpe, fused.embed(ids, wte, wpe, 2), dy, a.grad, b.grad
+
+
+def test_hooks_on_the_embedding_tables_see_and_change_the_gradient(embed_kernels):
+    k, wte, wpe, e, dy, gw, gp = _embedded(embed_kernels)
+    seen = []
+    handles = [wte.register_hook(lambda g: (seen.append(g.clone()), g * 0)[1]), wpe.register_post_accumulate_grad_hook(seen.append)]
+    e.backward(dy, retain_graph=True)
+    assert not k.calls and torch.equal(seen[0], gw) and seen[1] is wpe
+    assert torch.equal(wte.grad, torch.zeros_like(wte)) and torch.equal(wpe.grad, gp)
+    for h in handles:
+        h.remove()
+    wte.grad = wpe.grad = None
+    e.backward(dy)
+    assert k.calls == ["order", "rows", "positions"] and wte.grad is None and wpe.grad is None
+    assert torch.allclose(wte.main_grad, gw.float(), atol=2e-2, rtol=1e-2) and torch.allclose(wpe.main_grad, gp.float(), atol=2e-2, rtol=1e-2)
+
+
+def test_gradients_of_the_embedding_tables_can_be_asked_for(embed_kernels):
+    k, wte, wpe, e, dy, gw, gp = _embedded(embed_kernels)
+    a, b = torch.autograd.grad(e, (wte, wpe), dy, retain_graph=True)
+    assert torch.equal(a, gw) and torch.equal(b, gp) and not k.calls
+    e.backward(dy, inputs=[wpe], retain_graph=True)
+    assert k.calls == ["positions"] and wte.grad is None
+    # second derivatives: d/d(dy) of sum(gradient * c) is c looked up by the ids
+    d2 = dy.clone().requires_grad_(True)
+    (g,) = torch.autograd.grad(e, wte, d2, create_graph=True)
+    c = torch.randn(40, 8, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16)
+    (back,) = torch.autograd.grad(g, d2, c)
+    assert torch.equal(back, c[torch.tensor([3, 3, 5, 0, 39, 5])])
