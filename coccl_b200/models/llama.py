@@ -41,17 +41,22 @@ class _RMSNorm(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, weight, rstd = ctx.saved_tensors
-        wide = rstd.dtype
-        xhat = x.to(wide) * rstd
-        dyf = dy.to(wide)
-        dw = (dyf * xhat).reshape(-1, x.shape[-1]).sum(0)
-        g = dyf * weight.to(wide)
-        dx = (rstd * (g - xhat * (g * xhat).mean(-1, keepdim=True))).to(x.dtype)
+        dx, dw = rms_norm_gradients(x, weight, rstd, dy)
         mg = getattr(weight, "main_grad", None)
         if mg is not None:
             mg.add_(dw.to(mg.dtype))
             return dx, None, None
         return dx, dw.to(weight.dtype), None
+
+
+def rms_norm_gradients(x, weight, rstd, dy):
+    """(dx, fp32 dw) of y = x * rstd * weight with rstd = rsqrt(mean(x^2) + eps), as PyTorch operations."""
+    wide = rstd.dtype
+    xhat = x.to(wide) * rstd
+    dyf = dy.to(wide)
+    dw = (dyf * xhat).reshape(-1, x.shape[-1]).sum(0)
+    g = dyf * weight.to(wide)
+    return (rstd * (g - xhat * (g * xhat).mean(-1, keepdim=True))).to(x.dtype), dw
 
 
 def rms_norm(x, weight, eps: float, residual=None):

@@ -209,29 +209,48 @@ def embed(ids, wte, wpe=None, first: int = 0):
     return _Embed.apply(wte, wpe, ids, first)
 
 
+# The backward kernels' results are constants to autograd. Under create_graph (a backward pass with gradients enabled) the
+# backward functions below are PyTorch operations instead, written out: their results can be differentiated again.
+def _rms_norm_graph(x, weight, eps, dy):
+    """(dx, dw) of RMSNorm(x) * weight; dw is None where it went into `main_grad`."""
+    from ..models.llama import rms_norm_gradients
+    rstd = torch.rsqrt(x.float().square().mean(-1, keepdim=True) + eps)
+    dx, dw = rms_norm_gradients(x, weight, rstd, dy)
+    mg = getattr(weight, "main_grad", None)
+    if mg is not None:
+        mg.add_(dw.detach())
+        return dx, None
+    return dx, dw.to(weight.dtype)
+
+
 # --------------------------------------------------------------------------- RMSNorm (+ residual add)
 class _RmsNorm(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, res, weight, eps):
         H = x.shape[-1]
-        x2 = x.reshape(-1, H).contiguous()
-        r2 = res.reshape(-1, H).contiguous() if res is not None else None
-        M = x2.shape[0]
-        y = torch.empty_like(x2)
-        xo = torch.empty_like(x2) if res is not None else None
+        xc = x.contiguous()
+        r2 = res.contiguous() if res is not None else None
+        y = torch.empty_like(xc)
+        xo = torch.empty_like(xc) if res is not None else None
+        M = x.numel() // H
         rstd = torch.empty(M, dtype=torch.float32, device=x.device)
-        rc = _lib.lib().cocclkRmsNormFwd(x2.data_ptr(), _lib.ptr(r2), weight.data_ptr(), y.data_ptr(), _lib.ptr(xo),
+        rc = _lib.lib().cocclkRmsNormFwd(xc.data_ptr(), _lib.ptr(r2), weight.data_ptr(), y.data_ptr(), _lib.ptr(xo),
                                          rstd.data_ptr(), M, H, eps, _lib.cur_stream())
         _lib.check(rc, "cocclkRmsNormFwd")
-        xs = xo if res is not None else x2
-        ctx.save_for_backward(xs, weight, rstd)
-        ctx.has_res = res is not None
-        return y.reshape(x.shape), (xs.reshape(x.shape) if res is not None else None)
+        ctx.save_for_backward(xo if res is not None else x, weight, rstd)
+        ctx.has_res, ctx.eps = res is not None, eps
+        return y, xo
 
     @staticmethod
     def backward(ctx, dy, dxs):
         xs, weight, rstd = ctx.saved_tensors
-        M, H = xs.shape
+        if torch.is_grad_enabled():
+            dx, dw = _rms_norm_graph(xs, weight, ctx.eps, dy)
+            dx = dx + dxs if dxs is not None else dx
+            return dx, (dx if ctx.has_res else None), dw, None
+        xs = xs.contiguous()
+        H = xs.shape[-1]
+        M = xs.numel() // H
         dy2 = dy.reshape(-1, H).contiguous()
         dres = dxs.reshape(-1, H).contiguous() if dxs is not None else None
         if not (aligned16(dy2) and aligned16(dres)):
@@ -245,7 +264,6 @@ class _RmsNorm(torch.autograd.Function):
             _lib.check(rc, "cocclkRmsNormBwd")
 
         dw = _accum_param_grad(weight, None, run)
-        dx = dx.reshape(dy.shape)
         return dx, (dx if ctx.has_res else None), dw, None
 
 
@@ -290,6 +308,8 @@ class _RotateQkv(torch.autograd.Function):
         qkv, qw, kw, cos, sin = ctx.saved_tensors
         nh, nkv, eps = ctx.meta
         T, d = dq.shape[0], cos.shape[1]
+        if torch.is_grad_enabled():
+            return (*_rotate_graph(dq, dk, dv, qkv, qw, kw, cos, sin, eps), None, None, None, None, None)
         dq, dk, dv = (t.contiguous() if aligned16(t) else t.clone(memory_format=torch.contiguous_format) for t in (dq, dk, dv))
         dqkv = dq.new_empty(T, (nh + 2 * nkv) * d)
         mq, mk = getattr(qw, "main_grad", None), getattr(kw, "main_grad", None)
@@ -309,6 +329,24 @@ class _RotateQkv(torch.autograd.Function):
         if qw is not None and mq is None:
             return dqkv, gq.to(qw.dtype), gk.to(kw.dtype), None, None, None, None, None
         return dqkv, None, None, None, None, None, None, None
+
+
+def _rotate_graph(dq, dk, dv, qkv, qw, kw, cos, sin, eps):
+    """(dqkv, dqw, dkw) of the rotation under create_graph."""
+    T, d = dq.shape[0], cos.shape[1]
+    at = torch.arange(T, device=dq.device) % cos.shape[0]
+    c, s = cos[at][:, None], sin[at][:, None]
+
+    def back(g):   # the rotation by the opposite angle
+        g = g.float()
+        return g * c - torch.cat([-g[..., d // 2:], g[..., :d // 2]], -1) * s
+    gq, gk = back(dq).to(dq.dtype), back(dk).to(dk.dtype)
+    dqw = dkw = None
+    if qw is not None:
+        q, k, _ = (t.reshape(T, -1, d) for t in qkv.split([g.shape[1] * d for g in (dq, dk, dv)], -1))
+        gq, dqw = _rms_norm_graph(q, qw, eps, gq)
+        gk, dkw = _rms_norm_graph(k, kw, eps, gk)
+    return torch.cat([t.reshape(T, -1) for t in (gq, gk, dv)], -1), dqw, dkw
 
 
 def rotate_qkv_fits(qkv, d: int, qw=None, kw=None) -> bool:
@@ -346,6 +384,9 @@ class _Swiglu(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         (z,) = ctx.saved_tensors
+        if torch.is_grad_enabled():
+            gate, up = z.chunk(2, dim=-1)
+            return torch.autograd.grad(F.silu(gate) * up, z, dy, create_graph=True)[0]
         F_ = z.shape[-1] // 2
         dy = dy.contiguous() if aligned16(dy) else dy.clone(memory_format=torch.contiguous_format)
         dz = torch.empty_like(z)

@@ -1,12 +1,14 @@
 """Host side of the fused training operations, with the kernel library replaced by a stand-in that reads what the kernels would
 read (the pointers and sizes of each launch)."""
 import ctypes
+import math
 
 import pytest
 import torch
 import torch.nn.functional as F
 
 from coccl_b200 import _lib
+from coccl_b200.models import llama
 from coccl_b200.ops import fused
 
 
@@ -106,3 +108,116 @@ def test_gradients_of_the_embedding_tables_can_be_asked_for(embed_kernels):
     c = torch.randn(40, 8, generator=torch.Generator().manual_seed(6)).to(torch.bfloat16)
     (back,) = torch.autograd.grad(g, d2, c)
     assert torch.equal(back, c[torch.tensor([3, 3, 5, 0, 39, 5])])
+
+
+class LlamaKernels:
+    """What the Llama kernels compute; the backward kernels of the rotation and the gate write nothing."""
+
+    @staticmethod
+    def _bf16(ptr, *shape):
+        n = math.prod(shape)
+        return torch.frombuffer((ctypes.c_uint8 * (2 * n)).from_address(ptr), dtype=torch.bfloat16).view(*shape)
+
+    @staticmethod
+    def _fp32(ptr, *shape):
+        n = math.prod(shape)
+        return torch.frombuffer((ctypes.c_uint8 * (4 * n)).from_address(ptr), dtype=torch.float32).view(*shape)
+
+    def cocclkLayerNormBwdGrid(self, M):
+        return 1
+
+    cocclkRotateBwdGrid = cocclkLayerNormBwdGrid
+
+    def __getattr__(self, name):
+        if name.endswith("Bwd"):
+            return lambda *a: 0
+        raise AttributeError(name)
+
+    def cocclkRmsNormFwd(self, x, res, w, y, xo, rstd, M, H, eps, stream):
+        xs = self._bf16(x, M, H)
+        if res:
+            xs = self._bf16(xo, M, H).copy_(xs + self._bf16(res, M, H))
+        r = torch.rsqrt(xs.float().square().mean(-1, keepdim=True) + eps)
+        self._fp32(rstd, M, 1).copy_(r)
+        self._bf16(y, M, H).copy_(xs.float() * r * self._bf16(w, H).float())
+        return 0
+
+    def cocclkRmsNormBwd(self, dy, x, rstd, w, dres, dx, dw, accumulate, scratch, M, H, stream):
+        got = llama.rms_norm_gradients(self._bf16(x, M, H), self._bf16(w, H), self._fp32(rstd, M, 1), self._bf16(dy, M, H))
+        self._bf16(dx, M, H).copy_(got[0] + (self._bf16(dres, M, H) if dres else 0))
+        self._fp32(dw, H).copy_(got[1] + (self._fp32(dw, H) if accumulate else 0))
+        return 0
+
+    def cocclkRotateFwd(self, qkv, q, k, v, cos, sin, qw, kw, T, seq, nh, nkv, d, eps, stream):
+        heads = self._bf16(qkv, T, nh + 2 * nkv, d).float()
+        at = torch.arange(T) % seq
+        c, s = (self._fp32(p, seq, d)[at][:, None] for p in (cos, sin))
+        for out, x, w in ((q, heads[:, :nh], qw), (k, heads[:, nh:nh + nkv], kw)):
+            if w:
+                x = x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * self._bf16(w, d).float()
+            self._bf16(out, *x.shape).copy_(x * c + torch.cat([-x[..., d // 2:], x[..., :d // 2]], -1) * s)
+        self._bf16(v, T, nkv, d).copy_(heads[:, nh + nkv:])
+        return 0
+
+    def cocclkSwigluFwd(self, z, y, M, F_, stream):
+        gate, up = self._bf16(z, M, 2 * F_).chunk(2, -1)
+        self._bf16(y, M, F_).copy_(F.silu(gate.float()) * up.float())
+        return 0
+
+
+def _second(outputs, inputs, seed):
+    """Gradients of `inputs` under create_graph and, from a random weighting of those, the gradients once more."""
+    gen = torch.Generator().manual_seed(seed)
+    dys = [torch.randn(o.shape, generator=gen).to(o.dtype).requires_grad_(True) for o in outputs]
+    first = torch.autograd.grad(outputs, inputs, dys, create_graph=True)
+    total = sum((g * torch.randn(g.shape, generator=gen).to(g.dtype)).sum() for g in first)
+    second = torch.autograd.grad(total, [*inputs, *dys], allow_unused=True)
+    return [*first, *(torch.zeros(()) if g is None else g for g in second)]
+
+
+@pytest.mark.parametrize("case", ["norm", "norm + residual", "norm, rows apart", "rotation", "rotation + head norm", "gate"])
+def test_gradients_of_the_llama_functions_can_be_differentiated(monkeypatch, case):
+    """First and second derivatives against the same functions in 64 bits. bf16 results in a chain of a few operations: 2^-8 of
+    the largest value in each."""
+    k = LlamaKernels()
+    monkeypatch.setattr(_lib, "lib", lambda: k)
+    monkeypatch.setattr(_lib, "cur_stream", lambda: 0)
+    gen = torch.Generator().manual_seed(11)
+
+    def leaf(*shape):
+        return torch.randn(*shape, generator=gen).to(torch.bfloat16).requires_grad_(True)
+    eps, T, seq, nh, nkv, d = 1e-5, 6, 3, 2, 1, 8
+
+    def rms(x, w):
+        return x * torch.rsqrt(x.square().mean(-1, keepdim=True) + eps) * w
+    if case.startswith("norm"):
+        x, w, r = leaf(5, 32), leaf(16), leaf(5, 16)
+        inputs = [x, w] + ([r] if "residual" in case else [])
+        xin = x[:, ::2] if "apart" in case else x[:, :16].contiguous()
+        out = fused.rms_norm(xin, w, eps, r if "residual" in case else None)
+        out = out if isinstance(out, tuple) else (out,)
+        wide = [t.detach().double().requires_grad_(True) for t in inputs]
+        xw = wide[0][:, ::2] if "apart" in case else wide[0][:, :16]
+        xs = xw + wide[2] if "residual" in case else xw
+        ref = (rms(xs, wide[1]), xs)[:len(out)]
+    elif case.startswith("rotation"):
+        x, qw, kw = leaf(T, (nh + 2 * nkv) * d), leaf(d), leaf(d)
+        inputs = [x] + ([qw, kw] if "norm" in case else [])
+        cos, sin = llama._rope_tables(seq, d, 100.0, torch.device("cpu"))
+        out = fused.rotate_qkv(x, cos, sin, nh, nkv, *(inputs[1:] or (None, None)), eps)
+        wide = [t.detach().double().requires_grad_(True) for t in inputs]
+        heads = wide[0].view(T, -1, d)
+        at = torch.arange(T) % seq
+        parts = [heads[:, :nh], heads[:, nh:nh + nkv]]
+        if "norm" in case:
+            parts = [rms(p, w) for p, w in zip(parts, wide[1:])]
+        ref = [p * cos.double()[at][:, None] + torch.cat([-p[..., d // 2:], p[..., :d // 2]], -1) * sin.double()[at][:, None]
+               for p in parts] + [heads[:, nh + nkv:]]
+    else:
+        inputs = [leaf(4, 32)]
+        out = (fused._Swiglu.apply(inputs[0]),)
+        wide = [inputs[0].detach().double().requires_grad_(True)]
+        gate, up = wide[0].chunk(2, -1)
+        ref = (F.silu(gate) * up,)
+    for got, want in zip(_second(out, inputs, 21), _second(ref, wide, 21)):
+        assert (got.double() - want).abs().max() <= 3 * 2.0 ** -8 * max(1.0, want.abs().max().item())
