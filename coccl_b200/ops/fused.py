@@ -199,7 +199,7 @@ def embed_fits(ids, wte, wpe=None, first: int = 0) -> bool:
         mg = getattr(w, "main_grad", None)
         return (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and w.shape[1] % 8 == 0 and
                 w.requires_grad and mg is not None and mg.dtype == torch.float32 and mg.is_contiguous() and aligned16(mg))
-    return (ids.is_cuda and ids.dtype == torch.int64 and ids.dim() == 2 and 0 < ids.numel() <= 16384 and table(wte) and
+    return (ordinary(ids, wte, wpe) and ids.is_cuda and ids.dtype == torch.int64 and ids.dim() == 2 and 0 < ids.numel() <= 16384 and table(wte) and
             (wpe is None or (table(wpe) and wpe.shape[1] == wte.shape[1] and wpe.shape[0] >= first + ids.shape[1])))
 
 
@@ -267,6 +267,15 @@ class _RmsNorm(torch.autograd.Function):
         return dx, (dx if ctx.has_res else None), dw, None
 
 
+def ordinary(*ts) -> bool:
+    """Whether a kernel may stand in for PyTorch operations on these tensors (None counts): plain tensors, outside of function
+    transforms (vmap, jvp, ...), forward-mode levels and dispatch modes (fake tensors, tracing, counters), all of which work on
+    the operations and would not see a kernel."""
+    return (all(t is None or type(t) in (torch.Tensor, torch.nn.Parameter) for t in ts) and
+            not torch._C._are_functorch_transforms_active() and torch.autograd.forward_ad._current_level < 0 and
+            torch._C._len_torch_dispatch_stack() == 0)
+
+
 def aligned16(*ts) -> bool:
     """Whether every given tensor starts on a 16-byte boundary (None counts as aligned)."""
     return all(t is None or t.data_ptr() % 16 == 0 for t in ts)
@@ -278,7 +287,7 @@ def rms_norm_fits(x, weight, residual=None) -> bool:
     H = x.shape[-1] if x.dim() else 0
     same = residual is None or (residual.dtype == x.dtype and residual.shape == x.shape and residual.device == x.device)
     mg = getattr(weight, "main_grad", None)
-    return (x.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and weight.device == x.device and same and
+    return (ordinary(x, weight, residual) and x.is_cuda and x.dtype == weight.dtype == torch.bfloat16 and weight.device == x.device and same and
             0 < H <= 16384 and H % 8 == 0 and x.numel() > 0 and weight.shape == (H,) and weight.is_contiguous() and
             (mg is None or (mg.dtype == torch.float32 and mg.is_contiguous())) and aligned16(x, weight, residual))
 
@@ -352,7 +361,7 @@ def _rotate_graph(dq, dk, dv, qkv, qw, kw, cos, sin, eps):
 def rotate_qkv_fits(qkv, d: int, qw=None, kw=None) -> bool:
     """Whether the rotation kernel takes a packed projection: contiguous bf16 on the GPU, heads of 32, 64, 128 or 256 (a head
     is a power of two of lanes), norm weights both present with fp32 gradients of the same kind, or both absent."""
-    if not (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.is_contiguous() and qkv.numel() > 0 and
+    if not (ordinary(qkv, qw, kw) and qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.dim() == 2 and qkv.is_contiguous() and qkv.numel() > 0 and
             d in (32, 64, 128, 256) and aligned16(qkv)):
         return False
     if qw is None and kw is None:
@@ -398,7 +407,8 @@ class _Swiglu(torch.autograd.Function):
 def swiglu(z):
     """silu(gate) * up for z = [gate | up] along the last dimension: one kernel each way for contiguous bf16 CUDA tensors
     whose halves are whole 16-byte vectors, PyTorch operations otherwise."""
-    if z.is_cuda and z.dtype == torch.bfloat16 and z.is_contiguous() and z.shape[-1] % 16 == 0 and z.numel() > 0 and aligned16(z):
+    if (ordinary(z) and z.is_cuda and z.dtype == torch.bfloat16 and z.is_contiguous() and z.shape[-1] % 16 == 0 and z.numel() > 0 and
+            aligned16(z)):
         return _Swiglu.apply(z)
     gate, up = z.chunk(2, dim=-1)
     return F.silu(gate) * up

@@ -221,3 +221,59 @@ def test_gradients_of_the_llama_functions_can_be_differentiated(monkeypatch, cas
         ref = (F.silu(gate) * up,)
     for got, want in zip(_second(out, inputs, 21), _second(ref, wide, 21)):
         assert (got.double() - want).abs().max() <= 3 * 2.0 ** -8 * max(1.0, want.abs().max().item())
+
+
+@pytest.fixture
+def llama_as_on_the_gpu(monkeypatch):
+    """CPU tensors that the rules for the kernels take for CUDA ones; a kernel call fails."""
+    class No:
+        def __getattr__(self, name):
+            raise AssertionError(f"{name} called")
+    monkeypatch.setattr(_lib, "lib", lambda: No())
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True))
+
+
+def _llama_functions():
+    """(function of one bf16 tensor [4, 32], the same as PyTorch operations): what the Llama layers run on one tensor."""
+    w, table = torch.linspace(0.5, 1.5, 32).to(torch.bfloat16), _table(40, 8, 1)
+    return {"gate": (fused.swiglu, lambda z: F.silu(z[..., :16]) * z[..., 16:]),
+            "embedding": (lambda x: fused.embed_fits((x.reshape(-1, 32)[:, :2] * 0).long(), table), None),
+            "norm": (lambda x: fused.rms_norm_fits(x, w), None), "rotation": (lambda x: fused.rotate_qkv_fits(x, 32), None)}
+
+
+@pytest.mark.parametrize("around", ["vmap", "forward mode", "dispatch mode", "subclass"])
+@pytest.mark.parametrize("name", ["gate", "norm", "rotation", "embedding"])
+def test_transforms_and_modes_work_on_operations(llama_as_on_the_gpu, around, name):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Count(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    class Sub(torch.Tensor):
+        pass
+    fn, ref = _llama_functions()[name]
+    x = torch.randn(4, 32, generator=torch.Generator().manual_seed(1)).to(torch.bfloat16)
+    if ref is None:   # a rule: yes for plain tensors, no here
+        assert fn(x)
+        if around == "vmap":
+            assert torch.vmap(lambda t: t * (1 + int(fn(x))))(x).equal(x)
+        elif around == "forward mode":
+            with torch.autograd.forward_ad.dual_level():
+                assert not fn(x)
+        elif around == "dispatch mode":
+            with Count():
+                assert not fn(x)
+        else:
+            assert not fn(x.as_subclass(Sub))
+        return
+    if around == "vmap":
+        assert torch.equal(torch.vmap(fn)(x), ref(x))
+    elif around == "forward mode":
+        got, want = (torch.func.jvp(f, (x,), (torch.ones_like(x),)) for f in (fn, ref))
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    elif around == "dispatch mode":
+        with Count():
+            assert torch.equal(fn(x), ref(x))
+    else:
+        assert torch.equal(fn(x.as_subclass(Sub)), ref(x))
