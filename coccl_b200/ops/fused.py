@@ -490,7 +490,7 @@ class _CrossEntropy(torch.autograd.Function):
     def forward(ctx, logits, targets, scale, unit_grad):
         V = logits.shape[-1]
         lg = logits.reshape(-1, V)
-        tg = targets.reshape(-1)
+        tg = targets.reshape(-1).contiguous()   # the kernel reads consecutive targets
         M = lg.shape[0]
         if lg.is_cuda:
             assert lg.stride(1) == 1

@@ -277,3 +277,21 @@ def test_transforms_and_modes_work_on_operations(llama_as_on_the_gpu, around, na
             assert torch.equal(fn(x), ref(x))
     else:
         assert torch.equal(fn(x.as_subclass(Sub)), ref(x))
+
+
+@pytest.mark.parametrize("kind", ["one column", "every other column", "whole rows"])
+def test_cross_entropy_reads_its_targets_whatever_their_strides(monkeypatch, kind):
+    seen = []
+
+    class K:
+        def cocclkCrossEntropy(self, logits, targets, loss, M, V, ld, scale, stream):
+            seen.append(_read(targets, M, ctypes.c_int64, torch.int64))
+            return 0
+    tok = torch.arange(40).view(4, 10)
+    targets = {"one column": tok[:, 1:2], "every other column": tok[:1, ::2], "whole rows": tok}[kind]
+    logits = torch.zeros(targets.numel(), 64, dtype=torch.bfloat16)
+    monkeypatch.setattr(_lib, "lib", lambda: K())
+    monkeypatch.setattr(_lib, "cur_stream", lambda: 0)
+    monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True))
+    fused.cross_entropy(logits, targets, 1.0)
+    assert torch.equal(seen[0], targets.reshape(-1))
