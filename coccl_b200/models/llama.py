@@ -94,6 +94,14 @@ def rotate_positions(x, theta: float):
     return (xf * cos + rot * sin).to(x.dtype)
 
 
+def _attends_grouped(q, k, v) -> bool:
+    """Whether an attention kernel is enabled that serves grouped queries without a copy of the keys and values per query head:
+    flash and cuDNN attention do; the memory-efficient one refuses them and plain matrix products copy all the same. Heads wider
+    than 128 are copied always, which lets PyTorch choose among all of its kernels."""
+    p = torch.backends.cuda.SDPAParams(q, k, v, None, 0.0, True, True)
+    return torch.backends.cuda.can_use_flash_attention(p) or torch.backends.cuda.can_use_cudnn_attention(p)
+
+
 class LlamaLayer(TransformerLayer):
     def __init__(self, cfg, idx, store, tp):
         nn.Module.__init__(self)
@@ -154,11 +162,10 @@ class LlamaLayer(TransformerLayer):
         if getattr(self, "cp", None) is None and fused.rotate_qkv_fits(qkv, d, qw, kw):
             cos, sin = _rope_tables(seq, d, cfg.rope_theta, qkv.device)
             q, k, v = (x.view(batch, seq, -1, d).transpose(1, 2) for x in fused.rotate_qkv(qkv, cos, sin, nh, nkv, qw, kw, cfg.eps))
-            # grouped queries inside the attention kernel: keys and values are not copied per query head (heads wider than
-            # 128 keep the copies, which let PyTorch choose among all of its attention kernels)
-            if nkv != nh and d > 128:
+            grouped = nkv != nh and d <= 128 and _attends_grouped(q, k, v)
+            if nkv != nh and not grouped:
                 k, v = k.repeat_interleave(nh // nkv, dim=1), v.repeat_interleave(nh // nkv, dim=1)
-            o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=nkv != nh and d <= 128).transpose(1, 2)
+            o = F.scaled_dot_product_attention(q, k, v, is_causal=True, enable_gqa=grouped).transpose(1, 2)
             return o.reshape(batch * seq, nh * d)
         q, k, v = qkv.split([nh * d, nkv * d, nkv * d], dim=-1)
         q, k = q.reshape(batch, seq, nh, d), k.reshape(batch, seq, nkv, d)
