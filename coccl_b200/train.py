@@ -8,12 +8,14 @@ optimizer and returns the mean loss as a device scalar.
 """
 from __future__ import annotations
 
+import operator
+import warnings
 from dataclasses import dataclass
 
 import torch
 
 from . import _lib
-from .models.gpt import GPTConfig, GPTStage
+from .models.gpt import GPTConfig, GPTStage, ParamStore, TransformerLayer
 from .parallel.dp import DistributedOptimizer
 
 
@@ -45,6 +47,60 @@ def split_layers(n_layer: int, stages: int) -> list[tuple[int, int]]:
     return out
 
 
+def _own_code() -> list:
+    """(namespace, names, values) of the functions, classes and methods that a pass through a stage can reach by name, as this
+    package and PyTorch define them."""
+    from torch.nn.modules import module as nnm
+    from .models import gpt, llama
+    from .ops import fused, gemm
+    own = (gpt.GPTStage, gpt.TransformerLayer, gpt.NoTP, gpt.GPTConfig, llama.LlamaLayer, Trainer, fused._Linear, fused._LayerNorm,
+           fused._RmsNorm, fused._RotateQkv, fused._Swiglu, fused._Embed, fused._CrossEntropy)
+    spaces = [(vars(x), [k for k, v in vars(x).items() if callable(v) or isinstance(v, (staticmethod, classmethod, property))])
+              for x in (gpt, llama, fused, gemm, _lib, *own)]
+    spaces += [(vars(torch.nn.functional), ["scaled_dot_product_attention", "embedding", "silu"]), (vars(nnm.Module), ["__call__", "_call_impl"]),
+               (vars(torch.Tensor), ["backward"]), (vars(torch.autograd), ["backward"])]
+    return [(ns, keys, [ns[k] for k in keys]) for ns, keys in spaces]
+
+
+class _Snapshot:
+    """Everything a pass through a stage looks up in its modules, as it stood: their attributes, parameters and sub-modules, the
+    fields of the objects they hold (configuration, tensor-parallel context), the elements of lists. Taken and compared by
+    identity, and what is compared is kept alive, so that a new object can never pass for the old one."""
+
+    # hook tables of a module: their identity is compared, what is in them is MicroBatchGraph._plain_context's to look at
+    HOOKS = set(vars(torch.nn.Module())) - {"_parameters", "_buffers", "_modules"}
+
+    def __init__(self, *roots):
+        self.roots, self.parts, seen = roots, [], set()
+        for r in roots:
+            self._walk(r, seen)
+
+    def _walk(self, obj, seen):
+        if id(obj) in seen or isinstance(obj, (type, torch.Tensor, ParamStore)):
+            return
+        seen.add(id(obj))
+        module = isinstance(obj, torch.nn.Module)
+        if module or (type(obj).__module__.startswith(__package__) and hasattr(obj, "__dict__")):
+            obj = obj.__dict__
+        if isinstance(obj, (dict, list, tuple)):
+            self.parts.append((obj, self._content(obj)))
+            for v in [v for k, v in obj.items() if not (module and k in self.HOOKS)] if isinstance(obj, dict) else obj:
+                self._walk(v, seen)
+
+    @staticmethod
+    def _content(c):
+        return [*c, *c.values()] if isinstance(c, dict) else list(c)
+
+    def holds(self, *roots) -> bool:
+        if not all(map(operator.is_, roots, self.roots)):
+            return False
+        for c, was in self.parts:
+            now = self._content(c)
+            if len(now) != len(was) or not all(map(operator.is_, now, was)):
+                return False
+        return True
+
+
 class MicroBatchGraph:
     """Forward and backward of one micro-batch as a CUDA graph, for models whose kernels are shorter than the host code that
     launches them.
@@ -52,25 +108,42 @@ class MicroBatchGraph:
     A micro-batch is about 35 launches a layer through autograd, 1.2 ms of host time a layer; below that much device work a
     layer the GPU waits (2 layers 512 wide, two micro-batches of 512 tokens: 5.0 ms a step for 1.4 ms of kernels). Replayed,
     the launches cost the device only. Large models gain nothing and would keep a micro-batch's activations in the graph's
-    pool, so the rule is on size (`worth_it`). A graph is captured when a step has been seen twice with the same shapes and
-    the same parameter and gradient buffers, so first steps on new inputs run as ever; it holds what its kernels address
-    (the scratch buffers and tables as they were), and any change of those buffers, of the hooks on the modules or of the
-    autograd modes around the call sends the step back to the launches."""
+    pool, so the rule is on size (`worth_it`). A graph is captured when a step has been seen twice with nothing changed, so
+    first steps on new inputs run as ever; it holds what its kernels address (the scratch buffers and tables as they were).
+
+    A replay runs the kernels and none of the Python around them, so it stands in for a step only while that Python could not
+    have done anything else: the stage is built of this package's own dense layers, whose methods and functions are the
+    package's own; nothing the pass looks up has changed since the capture (`_Snapshot`), nor the buffers behind the parameters
+    and their gradients, nor PyTorch's switches for attention, matrix products and determinism; and no hook, mode or context
+    around the call would see the pass. Anything else goes back to the launches. Setting `enabled` to False does so for good,
+    and gives the graph's memory back at the next step."""
 
     MAX_TOKENS = 16384
     MAX_LAYER_FLOPS = 1.5e12    # 1.1 ms at the 1.37 PFLOP/s of sustained bf16 products, against 1.2 ms of host time
+    MAX_POOL_BYTES = 1 << 30    # the graph keeps the activations of a micro-batch beside the allocator's cache
 
     def __init__(self):   # no reference to the trainer: the two would keep each other's device memory until a collection
         self.enabled = True
         self._drop()
 
     def _drop(self):
-        self.key = self.seen = self.graph = self.tokens = self.keep = None
+        self.key = self.snapshot = self.sdp_order = self.seen = self.graph = self.tokens = self.keep = None
         self.launches = 0
 
     @classmethod
     def worth_it(cls, cfg: GPTConfig, n_tokens: int) -> bool:
-        return n_tokens <= cls.MAX_TOKENS and cfg.flops_per_token() * n_tokens <= cls.MAX_LAYER_FLOPS * max(1, cfg.n_layer)
+        # bf16 values a token leaves behind: 12 rows of the hidden size and 4 of the MLP's a layer, and its logits
+        pool = 2.0 * n_tokens * (cfg.n_layer * (12 * cfg.hidden + 4 * cfg.ffn) + cfg.vocab)
+        return (n_tokens <= cls.MAX_TOKENS and cfg.flops_per_token() * n_tokens <= cls.MAX_LAYER_FLOPS * max(1, cfg.n_layer) and
+                pool <= cls.MAX_POOL_BYTES)
+
+    @staticmethod
+    def own_code(stage) -> bool:
+        """Whether `stage` is built of this package's own dense modules, with none of their methods replaced."""
+        from .models.llama import LlamaLayer
+        return type(stage) is GPTStage and all(
+            type(m) in (GPTStage, TransformerLayer, LlamaLayer, torch.nn.ModuleList) and
+            not any(callable(getattr(type(m), k, None)) for k in vars(m)) for m in stage.modules())
 
     @staticmethod
     def _plain_context(stage) -> bool:
@@ -84,33 +157,58 @@ class MicroBatchGraph:
 
     @staticmethod
     def _key(t, shape, scale):
+        """What is compared by value; None where hooks on a parameter would see its gradient, or it has no gradient buffer."""
         from .ops import gemm as G
-        params = tuple((p.data_ptr(), p.main_grad.data_ptr(), p.requires_grad, bool(p._backward_hooks))
-                       for p in t.stage.store.params.values())
-        return tuple(shape), scale, G.get_variant(), torch.cuda.current_device(), t._loss_acc.data_ptr(), params
+        sdp, cudnn, mm = torch.backends.cuda, torch.backends.cudnn, torch.backends.cuda.matmul
+        switches = (sdp.flash_sdp_enabled(), sdp.mem_efficient_sdp_enabled(), sdp.math_sdp_enabled(), sdp.cudnn_sdp_enabled(),
+                    sdp.fp16_bf16_reduction_math_sdp_allowed(),
+                    torch.are_deterministic_algorithms_enabled(), torch.is_deterministic_algorithms_warn_only_enabled(),
+                    torch.utils.deterministic.fill_uninitialized_memory, cudnn.enabled, cudnn.deterministic, cudnn.benchmark,
+                    torch.get_float32_matmul_precision(), mm.allow_bf16_reduced_precision_reduction,
+                    torch.get_default_dtype(), torch.is_inference_mode_enabled())
+        params = [p for m in t.stage.modules() for p in m._parameters.values() if p is not None]
+        if any(p._backward_hooks or p._post_accumulate_grad_hooks or getattr(p, "main_grad", None) is None for p in params):
+            return None
+        params = [(p.data_ptr(), p.main_grad.data_ptr(), p.main_grad.dtype, p.shape, p.stride(), p.requires_grad) for p in params]
+        return tuple(shape), scale, G.get_variant(), torch.cuda.current_device(), t._loss_acc.data_ptr(), switches, params
 
     def ready(self, t: "Trainer", shape, scale) -> bool:
         """Whether trainer t's micro-batches of this step are to be replayed (captures the graph at the third equal step)."""
-        if not (self.enabled and torch.device(t.device).type == "cuda" and t.schedule is None and t.groups is None and not t.fsdp and
+        if not self.enabled:
+            self._drop()
+            return False
+        if not (torch.device(t.device).type == "cuda" and t.schedule is None and t.groups is None and not t.fsdp and
                 t.cfg.n_experts == 0 and self.worth_it(t.cfg, shape[0] * (shape[1] - 1)) and
-                self._plain_context(t.stage)):
+                self._plain_context(t.stage) and "_micro_batch" not in vars(t) and type(t)._micro_batch is Trainer._micro_batch and
+                all(all(map(operator.is_, map(ns.get, keys), was)) for ns, keys, was in _OWN_CODE)):
             return False
         key = self._key(t, shape, scale)
-        if any(k[3] for k in key[-1]):
+        if key is None:
             return False
-        if key != self.key:
+        order = torch._C._get_sdp_priority_order()   # PyTorch fills it in at its first attention call
+        if key != self.key or not self.snapshot.holds(t.stage, t.cfg) or (self.graph is not None and order != self.sdp_order):
             self._drop()
-            self.key, self.seen = key, 1
+            if self.own_code(t.stage):
+                self.key, self.snapshot, self.seen = key, _Snapshot(t.stage, t.cfg), 1
             return False
         if self.graph is None:
             self.seen += 1
             if self.seen > 2:
+                self.sdp_order = order
                 self._capture(t, shape, scale)
         return self.graph is not None
+
+    def _give_up(self, why: str):
+        self.enabled = False
+        self._drop()
+        warnings.warn(f"micro-batches of this trainer are launched kernel by kernel: {why}")
 
     def _capture(self, t, shape, scale):
         from .models import llama
         from .ops import fused, gemm
+        params = list(t.stage.parameters())
+        if any(p.grad is not None for p in params):
+            return
         tokens = torch.zeros(tuple(shape), dtype=torch.int64, device=t.device)
         graph, side, cur = torch.cuda.CUDAGraph(), torch.cuda.Stream(t.device), torch.cuda.current_stream(t.device)
         before = _lib.lib().cocclkLaunchCount()
@@ -122,16 +220,16 @@ class MicroBatchGraph:
                     t._micro_batch(tokens, scale)
                 finally:
                     graph.capture_end()
-        except RuntimeError:
-            self.enabled = False   # something in this model cannot be captured: nothing has run, the launches take over
+            if any(p.grad is not None for p in params):
+                self._give_up("autograd leaves a gradient in `.grad`, which only the capture would see")
+                return
+        except RuntimeError as e:   # nothing has run: the launches take over
+            self._give_up(f"the capture of the CUDA graph failed ({e})")
             return
         finally:
             cur.wait_stream(side)
-        if any(p.grad is not None for p in t.stage.parameters()):
-            for p in t.stage.parameters():
+            for p in params:
                 p.grad = None
-            self.enabled = False   # a gradient that autograd hands over in `.grad` would only be seen by the capture
-            return
         self.graph, self.tokens = graph, tokens
         self.launches = _lib.lib().cocclkLaunchCount() - before
         self.keep = (list(fused._scratch.values()), list(gemm._err_words.values()), list(llama._ROPE_CACHE.values()))
@@ -298,3 +396,6 @@ class Trainer:
         if wait:
             from .ops import gemm as G
             G.check_errors()
+
+
+_OWN_CODE = _own_code()

@@ -66,6 +66,122 @@ def test_hooks_modes_and_changed_buffers_take_the_launches(cuda):
     assert a.micro_graph.graph is None and float(p.main_grad.norm()) > 0
 
 
+def _set(obj, name, value):
+    setattr(obj, name, value)
+
+
+def _other_data(p):
+    p.data = (p.data.float() * 0.5).to(p.dtype)   # another buffer
+
+
+def _other_main_grad(p):
+    p.main_grad = p.main_grad.clone()
+
+
+def _plain_mlp(t):
+    layer = t.stage.layers[0]
+    layer.mlp = lambda y: type(layer).mlp(layer, y) * 0.5
+
+
+CHANGES = {
+    "weight of the joined projections": lambda t: _other_data(t.stage.layers[0].wqkv),
+    "weight of gate and up": lambda t: _other_data(t.stage.layers[1].w_gate_up),
+    "gradient buffer of the joined projections": lambda t: _other_main_grad(t.stage.layers[0].wqkv),
+    "eps": lambda t: _set(t.cfg, "eps", 0.5),
+    "rope_theta": lambda t: _set(t.cfg, "rope_theta", 7.0),
+    "method of a layer": _plain_mlp,
+}
+
+
+@pytest.mark.parametrize("change", sorted(CHANGES))
+def test_changes_after_the_capture_take_effect(cuda, change):
+    """The same change made to a replayed and to a launched trainer: their next steps agree up to the order of the attention's
+    atomic sums, and differ from what a step without the change gives."""
+    a, b = _pair("llama")
+    for step in range(4):
+        a.train_step(_tokens(step))
+        b.train_step(_tokens(step))
+    assert a.micro_graph.graph is not None
+    for t in (a, b):
+        CHANGES[change](t)
+    for step in range(4, 8):
+        la, lb = a.train_step(_tokens(step)).item(), b.train_step(_tokens(step)).item()
+        assert abs(la - lb) <= 2e-3 * abs(lb), (step, la, lb)
+        for pa, pb in zip(a.stage.parameters(), b.stage.parameters()):
+            assert (pa.main_grad - pb.main_grad).norm() <= 3e-2 * pb.main_grad.norm() + 1e-6, step
+    assert (a.micro_graph.graph is not None) == (change != "method of a layer")   # captured anew, or not at all
+
+
+@pytest.mark.parametrize("switch", ["attention kernels", "determinism"])
+def test_switches_of_pytorch_send_the_step_back_to_the_launches(cuda, switch):
+    from torch.nn.attention import SDPBackend, sdpa_kernel
+    a, _ = _pair("gpt")
+    for step in range(3):
+        a.train_step(_tokens(step))
+    graph = a.micro_graph.graph
+    assert graph is not None
+    if switch == "attention kernels":
+        with sdpa_kernel(SDPBackend.MATH):
+            a.train_step(_tokens(3))
+    else:
+        torch.use_deterministic_algorithms(True, warn_only=True)
+        try:
+            a.train_step(_tokens(3))
+        finally:
+            torch.use_deterministic_algorithms(False)
+    assert a.micro_graph.graph is None
+
+
+def test_disabling_gives_the_graph_back(cuda):
+    a, b = _pair("gpt")
+    for step in range(3):
+        a.train_step(_tokens(step))
+        b.train_step(_tokens(step))
+    assert a.micro_graph.graph is not None
+    a.micro_graph.enabled = False
+    la, lb = a.train_step(_tokens(3)).item(), b.train_step(_tokens(3)).item()
+    assert a.micro_graph.graph is None and abs(la - lb) <= 2e-3 * abs(lb)
+
+
+def test_failed_capture_is_reported_and_the_launches_take_over(cuda, monkeypatch):
+    a, b = _pair("gpt")
+
+    class Graph(torch.cuda.CUDAGraph):
+        def capture_begin(self, *args, **kw):
+            raise RuntimeError("no graph today")
+    for step in range(5):
+        with monkeypatch.context() as m:
+            m.setattr(torch.cuda, "CUDAGraph", Graph)
+            if step == 2:
+                with pytest.warns(UserWarning, match="no graph today"):
+                    la = a.train_step(_tokens(step)).item()
+            else:
+                la = a.train_step(_tokens(step)).item()
+        lb = b.train_step(_tokens(step)).item()
+        assert abs(la - lb) <= 2e-3 * abs(lb), step
+    assert a.micro_graph.graph is None and not a.micro_graph.enabled
+
+
+def test_gradients_that_autograd_hands_over_are_not_left_to_a_capture(cuda):
+    """An embedding whose gradient buffer the kernels do not take gets its gradient through `.grad`."""
+    a, b = _pair("llama")
+    for t in (a, b):
+        n = t.stage.wte.numel()
+        t.stage.wte.main_grad = torch.zeros(n + 1, device=cuda)[1:].view_as(t.stage.wte)
+    for step in range(5):
+        for t in (a, b):
+            t.stage.wte.main_grad.zero_()
+        if step == 2:
+            with pytest.warns(UserWarning, match="gradient"):
+                a.train_step(_tokens(step))
+        else:
+            a.train_step(_tokens(step))
+        b.train_step(_tokens(step))
+        ga, gb = a.stage.wte.main_grad, b.stage.wte.main_grad
+        assert gb.norm() > 0 and (ga - gb).norm() <= 3e-2 * gb.norm(), step
+    assert a.micro_graph.graph is None
+
+
 def test_size_rule(cuda):
     from coccl_b200.models.gpt import GPTConfig
     from coccl_b200.train import MicroBatchGraph
