@@ -229,6 +229,119 @@ __global__ void __launch_bounds__(kLnThreads) normBwdKernel(const bf16* dy, cons
   }
 }
 
+// The same for rows wider than 8192, where sums for two weights and a row of which some is prefetched do not fit the registers
+// (eight vectors a thread spilled 5.6 KB: 4096 x 16384 1430 us). The sums stay in shared memory, where a thread adds to its own
+// columns (131 KB at 16384, one CTA of 512 threads an SM), dy and x of the next row are on their way while this one is worked
+// on, the weight comes from the L1 cache twice a row. With the fold of the sums 4096 x 12288 and 4096 x 16384 take 112 and
+// 134 us (LayerNorm; with the row as fp32 in registers and no prefetch 275 and 374), 92 and 110 us (RMSNorm); 403 and 537 MB take
+// 62 and 82 us to copy.
+constexpr int kLnWideThreads = 512, kLnWideVec = 4;
+template <bool RMS>
+__global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf16* dy, const bf16* x, const float* mean,
+                                                                       const float* rstd, const bf16* gamma, const bf16* dres,
+                                                                       bf16* dx, float* partial, int M, int H) {
+  extern __shared__ float4 lnSums[];   // [dgamma | dbeta][vector of the thread][half][thread]
+  __shared__ float2 sm[2][kLnWideThreads / 32];
+  const int nvec = H / 8, warp = threadIdx.x >> 5, sums = (nvec + kLnWideThreads - 1) / kLnWideThreads * 2;
+  auto sum = [&](int which, int i, int half) -> float4& { return lnSums[(which * sums + i * 2 + half) * kLnWideThreads + threadIdx.x]; };
+  for (int k = 0; k < sums * (RMS ? 1 : 2); ++k) lnSums[k * kLnWideThreads + threadIdx.x] = make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint4* gv = reinterpret_cast<const uint4*>(gamma);
+  uint4 nd[kLnWideVec], nx[kLnWideVec];
+  float nmu = 0.f, nrs = 0.f;
+  auto fetch = [&](int row) {
+    const long base = (long)row * nvec;
+#pragma unroll
+    for (int i = 0; i < kLnWideVec; ++i) {
+      const int vi = threadIdx.x + i * kLnWideThreads;
+      if (vi < nvec) {
+        nd[i] = __ldg(reinterpret_cast<const uint4*>(dy) + base + vi);
+        nx[i] = __ldg(reinterpret_cast<const uint4*>(x) + base + vi);
+      }
+    }
+    if (!RMS) nmu = mean[row];
+    nrs = rstd[row];
+  };
+  auto add = [](float4& to, const float (&v)[8], int half) {
+    float4 t = to;
+    t.x += v[4 * half]; t.y += v[4 * half + 1]; t.z += v[4 * half + 2]; t.w += v[4 * half + 3];
+    to = t;
+  };
+  if (blockIdx.x < M) fetch(blockIdx.x);
+  int parity = 0;
+  for (int row = blockIdx.x; row < M; row += gridDim.x, parity ^= 1) {
+    uint4 cd[kLnWideVec], cx[kLnWideVec], cr[kLnWideVec];
+    const long base = (long)row * nvec;
+#pragma unroll
+    for (int i = 0; i < kLnWideVec; ++i) {
+      const int vi = threadIdx.x + i * kLnWideThreads;
+      cd[i] = nd[i];
+      cx[i] = nx[i];
+      if (dres && vi < nvec) cr[i] = __ldg(reinterpret_cast<const uint4*>(dres) + base + vi);
+    }
+    const float mu = nmu, rs = nrs;
+    if (row + (int)gridDim.x < M) fetch(row + gridDim.x);
+    float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+    for (int i = 0; i < kLnWideVec; ++i) {
+      const int vi = threadIdx.x + i * kLnWideThreads;
+      if (vi < nvec) {
+        float d[8], xv[8], g[8], p[8];
+        unpackBf16x8(cd[i], d);
+        unpackBf16x8(cx[i], xv);
+        unpackBf16x8(__ldg(gv + vi), g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = RMS ? xv[j] * rs : (xv[j] - mu) * rs, t = d[j] * g[j];
+          if (!RMS) s1 += t;
+          s2 += t * xh;
+          p[j] = d[j] * xh;
+        }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          add(sum(0, i, half), p, half);
+          if (!RMS) add(sum(1, i, half), d, half);
+        }
+      }
+    }
+    if (!RMS) s1 = warpSum(s1);
+    s2 = warpSum(s2);
+    if ((threadIdx.x & 31) == 0) sm[parity][warp] = make_float2(s1, s2);
+    __syncthreads();
+    float c1 = 0.f, c2 = 0.f;
+    for (int w = 0; w < kLnWideThreads / 32; ++w) { const float2 t = sm[parity][w]; c1 += t.x; c2 += t.y; }
+    c1 /= H;
+    c2 /= H;
+#pragma unroll
+    for (int i = 0; i < kLnWideVec; ++i) {
+      const int vi = threadIdx.x + i * kLnWideThreads;
+      if (vi < nvec) {
+        float d[8], xv[8], g[8], r[8], o[8];
+        unpackBf16x8(cd[i], d);
+        unpackBf16x8(cx[i], xv);
+        unpackBf16x8(__ldg(gv + vi), g);
+        if (dres) unpackBf16x8(cr[i], r);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float xh = RMS ? xv[j] * rs : (xv[j] - mu) * rs, t = d[j] * g[j];
+          o[j] = rs * (RMS ? t - xh * c2 : t - c1 - xh * c2);
+          if (dres) o[j] += r[j];
+        }
+        Vec8<bf16>::store(dx + (long)row * H + vi * 8, 8, true, o);
+      }
+    }
+  }
+  float* pg = partial + (long)blockIdx.x * (RMS ? 1 : 2) * H;
+  for (int i = 0; i < sums / 2; ++i) {
+    const int vi = threadIdx.x + i * kLnWideThreads;
+    if (vi >= nvec) break;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      reinterpret_cast<float4*>(pg + vi * 8)[half] = sum(0, i, half);
+      if (!RMS) reinterpret_cast<float4*>(pg + H + vi * 8)[half] = sum(1, i, half);
+    }
+  }
+}
+
 // out[c] (+)= sum_r partial[r][c]; `cols` columns, `rows` partial rows; columns from `split` on go to out2[c - split].
 // A CTA owns 32 columns; its 32 warps take every 32nd row (a warp reads 128 contiguous bytes of a row), four in flight, and
 // fold their sums through shared memory in a fixed order. Latency is all there is: 296 rows are three steps for a warp
@@ -643,11 +756,21 @@ static int launchNormBwd(const void* dy, const void* x, const float* mean, const
                          const void* dres, void* dx, float* dgamma, float* dbeta, int accumulate, float* scratch, int M, int H,
                          cudaStream_t s) {
   if (H % 8 || H <= 0 || H > kLnThreads * kLnMaxVec * 8 || M <= 0) return -1;
-  const int grid = cocclkLayerNormBwdGrid(M), threads = normThreads(H);
-  const int nv = (H / 8 + threads - 1) / threads;
+  int grid = cocclkLayerNormBwdGrid(M);
+  const int threads = normThreads(H), nv = (H / 8 + threads - 1) / threads;
 #define NORM_BWD(NV) normBwdKernel<NV, RMS><<<grid, threads, 0, s>>>((const bf16*)dy, (const bf16*)x, mean, rstd, \
       (const bf16*)gamma, (const bf16*)dres, (bf16*)dx, scratch, M, H)
-  if (nv <= 1) NORM_BWD(1); else if (nv <= 2) NORM_BWD(2); else if (nv <= 4) NORM_BWD(4); else NORM_BWD(8);
+  if (nv <= 1) NORM_BWD(1);
+  else if (nv <= 2) NORM_BWD(2);
+  else if (nv <= 4) NORM_BWD(4);
+  else {
+    const int rounds = (M + 147) / 148, smem = (H / 8 + kLnWideThreads - 1) / kLnWideThreads * kLnWideThreads * (RMS ? 32 : 64);
+    grid = (M + rounds - 1) / rounds;   // one CTA an SM, as many rows for each
+    const cudaError_t e = cudaFuncSetAttribute(normBwdWideKernel<RMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return (int)e;   // per device: a process may use several
+    normBwdWideKernel<RMS><<<grid, kLnWideThreads, smem, s>>>((const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)gamma,
+                                                              (const bf16*)dres, (bf16*)dx, scratch, M, H);
+  }
 #undef NORM_BWD
   // a scratch row is [dgamma | dbeta] (RMS: dgamma only): one fold for both
   const long cols = (RMS ? 1L : 2L) * H;

@@ -5,6 +5,7 @@ import pytest
 import torch
 import torch.nn.functional as F
 
+from coccl_b200 import _lib
 from coccl_b200.ops import fused
 
 pytestmark = pytest.mark.gpu
@@ -338,3 +339,62 @@ def test_cross_entropy_prefetched_rows(cuda, M, V):
     want[torch.arange(M, device=cuda), tgt.clamp(min=0)] -= 1
     want = want * valid[:, None] * 0.5
     assert ((logits.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("M,H", [(1, 8200), (2, 12288), (300, 8200), (149, 16384)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_wide_layer_norm_backward(cuda, M, H, residual):
+    """Rows that a CTA holds in parts (three and four vectors a thread, the last ones ragged), fewer and more rows than CTAs.
+    bf16 results carry 2^-9; the weight gradients sum M fp32 products."""
+    torch.manual_seed(M + H)
+    x, dy, r = (torch.randn(M, H, device=cuda).to(torch.bfloat16) for _ in range(3))
+    x.requires_grad_(True)
+    g = (1 + 0.1 * torch.randn(H, device=cuda)).to(torch.bfloat16).requires_grad_(True)
+    b = torch.randn(H, device=cuda).to(torch.bfloat16).requires_grad_(True)
+    g.main_grad, b.main_grad = torch.full((H,), 0.5, device=cuda), torch.zeros(H, device=cuda)
+    if residual:
+        y, xs = fused.layer_norm(x, g, b, 1e-5, r)
+        torch.autograd.backward([y, xs], [dy, r])
+    else:
+        fused.layer_norm(x, g, b, 1e-5).backward(dy)
+    s = (x + r if residual else x).detach().double().requires_grad_(True)
+    gd, bd = (t.detach().double().requires_grad_(True) for t in (g, b))
+    F.layer_norm(s, (H,), gd, bd, 1e-5).backward(dy.double())
+    ds = s.grad + (r.double() if residual else 0)
+    assert ((x.grad.double() - ds).abs() <= 2 ** -8 * ds.abs() + 1e-4).all()
+    assert torch.allclose(g.main_grad.double() - 0.5, gd.grad, rtol=1e-4, atol=1e-5 * M ** 0.5 + 1e-5)
+    assert torch.allclose(b.main_grad.double(), bd.grad, rtol=1e-4, atol=1e-5 * M ** 0.5 + 1e-5)
+
+
+def _device_us(fn, n=20):
+    """Device time of one call of many, the least of five rounds."""
+    for _ in range(3):
+        fn()
+    best = float("inf")
+    for _ in range(5):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(n):
+            fn()
+        b.record()
+        b.synchronize()
+        best = min(best, a.elapsed_time(b) / n * 1e3)
+    return best
+
+
+@pytest.mark.parametrize("rms", [False, True])
+def test_norm_backward_has_no_cliff_at_wide_rows(cuda, rms):
+    """One more vector a row must not cost several times the time (a kernel whose row does not fit the registers did: 20 times)."""
+    lib, M = _lib.lib(), 4096
+
+    def us(H):
+        x, dy, dr = (torch.randn(M, H, device=cuda).to(torch.bfloat16) for _ in range(3))
+        dx, g = torch.empty_like(x), torch.ones(H, device=cuda, dtype=torch.bfloat16)
+        mean, rstd, dg, db = torch.zeros(M, device=cuda), torch.ones(M, device=cuda), torch.zeros(H, device=cuda), torch.zeros(H, device=cuda)
+        sc = torch.empty(lib.cocclkLayerNormBwdGrid(M) * 2 * H, device=cuda)
+        p = [t.data_ptr() for t in (dy, x, mean, rstd, g, dr, dx, dg, db, sc)]
+        st = _lib.cur_stream()
+        if rms:
+            return _device_us(lambda: lib.cocclkRmsNormBwd(p[0], p[1], p[3], p[4], p[5], p[6], p[7], 1, p[9], M, H, st))
+        return _device_us(lambda: lib.cocclkLayerNormBwd(*p[:9], 1, p[9], M, H, st))
+    assert us(8200) <= 3 * us(8192)
