@@ -343,26 +343,28 @@ __global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf1
 }
 
 // out[c] (+)= sum_r partial[r][c]; `cols` columns, `rows` partial rows; columns from `split` on go to out2[c - split].
-// A CTA owns 32 columns; its 32 warps take every 32nd row (a warp reads 128 contiguous bytes of a row), four in flight, and
-// fold their sums through shared memory in a fixed order. Latency is all there is: 296 rows are three steps for a warp
-// (ten with 8 warps: 3.2 us a fold, now 2.5).
-constexpr int kColReduceCols = 32, kColReduceWarps = 32;
-__global__ void __launch_bounds__(32 * kColReduceWarps) colReduceKernel(const float* partial, float* out, float* out2, long split, int rows,
-                                                                       long cols, long stride, int accumulate) {
-  __shared__ float red[kColReduceWarps][33];
+// A CTA owns 32 columns; its WARPS warps take every WARPS-th row (a warp reads 128 contiguous bytes of a row), four in flight,
+// and fold their sums through shared memory in a fixed order. Latency is all there is: with 32 warps 296 rows are three steps for
+// a warp (ten with 8 warps: 3.2 us a fold, then 2.5). Few rows leave most of 32 warps idle, and more CTAs than the 296 of that size
+// that the GPU holds are a second wave, so such folds have 8 (column sum of 1 x 16384 in all: 5.5 us with 32, 3.9 with 8).
+constexpr int kColReduceCols = 32;
+template <int WARPS>
+__global__ void __launch_bounds__(32 * WARPS) colReduceKernel(const float* partial, float* out, float* out2, long split, int rows,
+                                                             long cols, long stride, int accumulate) {
+  __shared__ float red[WARPS][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const long c = (long)blockIdx.x * kColReduceCols + lane;
   float s = 0.f;
   if (c < cols) {
     int r = wy;
-    for (; r + 3 * kColReduceWarps < rows; r += 4 * kColReduceWarps) {
-      const float a0 = partial[(long)r * stride + c], a1 = partial[(long)(r + kColReduceWarps) * stride + c];
-      const float a2 = partial[(long)(r + 2 * kColReduceWarps) * stride + c], a3 = partial[(long)(r + 3 * kColReduceWarps) * stride + c];
+    for (; r + 3 * WARPS < rows; r += 4 * WARPS) {
+      const float a0 = partial[(long)r * stride + c], a1 = partial[(long)(r + WARPS) * stride + c];
+      const float a2 = partial[(long)(r + 2 * WARPS) * stride + c], a3 = partial[(long)(r + 3 * WARPS) * stride + c];
       s += (a0 + a1) + (a2 + a3);
     }
     float t[3];
 #pragma unroll
-    for (int u = 0; u < 3; ++u) t[u] = r + u * kColReduceWarps < rows ? partial[(long)(r + u * kColReduceWarps) * stride + c] : 0.f;
+    for (int u = 0; u < 3; ++u) t[u] = r + u * WARPS < rows ? partial[(long)(r + u * WARPS) * stride + c] : 0.f;
     s += (t[0] + t[1]) + t[2];
   }
   red[wy][lane] = s;
@@ -370,7 +372,7 @@ __global__ void __launch_bounds__(32 * kColReduceWarps) colReduceKernel(const fl
   if (wy == 0 && c < cols) {
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < kColReduceWarps; ++w) t += red[w][lane];
+    for (int w = 0; w < WARPS; ++w) t += red[w][lane];
     float* o = c < split ? out + c : out2 + (c - split);
     *o = accumulate ? *o + t : t;
   }
@@ -379,8 +381,9 @@ __global__ void __launch_bounds__(32 * kColReduceWarps) colReduceKernel(const fl
 // shared with llama_kernels.cu
 void launchColReduce(const float* partial, float* out, float* out2, long split, int rows, long cols, long stride, int accumulate,
                      cudaStream_t s) {
-  colReduceKernel<<<(unsigned)((cols + kColReduceCols - 1) / kColReduceCols), 32 * kColReduceWarps, 0, s>>>(partial, out, out2, split, rows, cols,
-                                                                                          stride, accumulate);
+  const unsigned grid = (unsigned)((cols + kColReduceCols - 1) / kColReduceCols);
+  if (rows > 64 && grid <= 2 * 148) colReduceKernel<32><<<grid, 32 * 32, 0, s>>>(partial, out, out2, split, rows, cols, stride, accumulate);
+  else colReduceKernel<8><<<grid, 32 * 8, 0, s>>>(partial, out, out2, split, rows, cols, stride, accumulate);
   cocclkCountLaunches(1);
 }
 
@@ -797,12 +800,21 @@ extern "C" int cocclkRmsNormBwd(const void* dy, const void* x, const float* rstd
   return launchNormBwd<true>(dy, x, nullptr, rstd, gamma, dres, dx, dgamma, nullptr, accumulate, scratch, M, H, s);
 }
 
-// 32 rows a block up to 64 blocks: a warp then has its (at most) four rows in flight at once
+// The most row blocks of a column sum (what its scratch holds): 32 rows a block up to 64 blocks.
 extern "C" int cocclkColSumBlocks(int M) { int b = (M + 31) / 32; return b > 64 ? 64 : (b < 1 ? 1 : b); }
+
+// Row blocks: 32 rows each (a warp then has its at most four rows in flight at once) while that leaves the GPU room, down to 128
+// rows where the column blocks fill it: more partial rows are more to write and fold (4096 x 4096: 7.5 us with 64 blocks, 6.6 with
+// 32; 512 x 16384: 7.7 with 16, 5.9 with 4).
+static int colSumBlocks(int M, int N) {
+  const int most = cocclkColSumBlocks(M), least = (M + 127) / 128 < most ? (M + 127) / 128 : most, colBlocks = (N / 8 + 31) / 32;
+  const int fill = 2 * 148 / colBlocks;
+  return fill < least ? least : (fill > most ? most : fill);
+}
 
 extern "C" int cocclkColSum(const void* x, float* out, int accumulate, float* scratch, int M, int N, cudaStream_t s) {
   if (N % 8 || M <= 0) return -1;
-  const int by = cocclkColSumBlocks(M);
+  const int by = colSumBlocks(M, N);
   const int rowsPer = (M + by - 1) / by;
   dim3 grid((N / 8 + 31) / 32, by);
   colSumPartialKernel<<<grid, 256, 0, s>>>((const bf16*)x, scratch, M, N, rowsPer);
@@ -947,7 +959,7 @@ extern "C" int cocclkColSumNoAlloc(const void* x, float* out, int accumulate, in
     }
     scratch = gColSumScratchAddr[dev];
   }
-  const int by = cocclkColSumBlocks(M);  // <= kNoAllocRows
+  const int by = colSumBlocks(M, N);  // <= kNoAllocRows
   const int rowsPer = (M + by - 1) / by;
   dim3 grid((N / 8 + 31) / 32, by);
   colSumPartialKernel<<<grid, 256, 0, s>>>((const bf16*)x, scratch, M, N, rowsPer);

@@ -398,3 +398,32 @@ def test_norm_backward_has_no_cliff_at_wide_rows(cuda, rms):
             return _device_us(lambda: lib.cocclkRmsNormBwd(p[0], p[1], p[3], p[4], p[5], p[6], p[7], 1, p[9], M, H, st))
         return _device_us(lambda: lib.cocclkLayerNormBwd(*p[:9], 1, p[9], M, H, st))
     assert us(8200) <= 3 * us(8192)
+
+
+@pytest.mark.parametrize("M,N", [(1, 16384), (129, 16384), (2049, 264), (4096, 2048), (64 * 32 + 1, 9472)])
+def test_column_sum_block_rules(cuda, M, N):
+    """Both folds (few and many partial rows, few and many columns) and both ends of the rule for the row blocks."""
+    torch.manual_seed(M)
+    x = torch.randn(M, N, device=cuda).to(torch.bfloat16)
+    lib = _lib.lib()
+    sc = torch.full((lib.cocclkColSumBlocks(M) * N + 8,), float("nan"), device=cuda)
+    out = torch.ones(N, device=cuda)
+    _lib.check(lib.cocclkColSum(x.data_ptr(), out.data_ptr(), 1, sc.data_ptr(), M, N, _lib.cur_stream()), "colsum")
+    # fp32 sums of M terms of size 1
+    assert ((out.double() - 1 - x.double().sum(0)).abs() <= M * 2.0 ** -24 * x.double().abs().sum(0) + 1e-6).all()
+    assert sc[-8:].isnan().all()
+
+
+def test_column_sum_of_wide_matrices_is_not_bound_by_its_fold(cuda):
+    """A column sum of few rows writes and folds more than it reads; it must cost about what a copy of one row's launches does."""
+    lib = _lib.lib()
+
+    def us(M, N):
+        x, out = torch.zeros(M, N, device=cuda, dtype=torch.bfloat16), torch.zeros(N, device=cuda)
+        sc = torch.empty(lib.cocclkColSumBlocks(M) * N, device=cuda)
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            for _ in range(50):
+                lib.cocclkColSum(x.data_ptr(), out.data_ptr(), 1, sc.data_ptr(), M, N, _lib.cur_stream())
+        return _device_us(g.replay, 3) / 50
+    assert us(1, 16384) <= 1.6 * us(1, 512)
