@@ -482,6 +482,7 @@ __global__ void __launch_bounds__(256) geluBwdKernel(const bf16* dy, const bf16*
 // ---------------------------------------------------------------- cross-entropy
 constexpr int kCeThreads = 1024;
 constexpr int kCeMaxVec = 7;  // V <= 1024*7*8 = 57344 held in registers
+constexpr int kCeNarrow = 256 * 4 * 8;
 
 __device__ __forceinline__ void cpAsync16(uint32_t smem, const void* g) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(g) : "memory");
@@ -494,8 +495,11 @@ __device__ __forceinline__ void cpAsync16(uint32_t smem, const void* g) {
 // row followed one another with the memory idle in between (4096 rows 336 us, 824 MB: 126 us to copy). The next row is now
 // on its way into shared memory while this one is worked on; a thread copies exactly the vectors it reads back, so the copy
 // needs no barrier, only the thread's own wait; and only the one vector that holds the target looks at it. 254 us, bound by
-// the exponentials and the two block reductions of the one CTA an SM has room for.
-__global__ void __launch_bounds__(kCeThreads) crossEntropyKernel(bf16* logits, const long* targets, float* loss,
+// the exponentials and the two block reductions of the one CTA an SM has room for. Rows of up to 8192 logits leave most of 1024
+// threads without one and take 256, four CTAs an SM, so that one row's
+// reductions run beside another's arithmetic: 4096 x 512 71 us with 1024 threads, 12.5 with 256, 4096 x 8192 85 and 26 us.
+template <int THREADS, int VECS>
+__global__ void __launch_bounds__(THREADS) crossEntropyKernel(bf16* logits, const long* targets, float* loss,
                                                                  int M, int V, long ld, float gscale) {
   extern __shared__ __align__(16) uint8_t ceRow[];
   __shared__ float sm[32];
@@ -504,9 +508,9 @@ __global__ void __launch_bounds__(kCeThreads) crossEntropyKernel(bf16* logits, c
   auto fetch = [&](int row) {
     const bf16* src = logits + (long)row * ld;
 #pragma unroll
-    for (int i = 0; i < kCeMaxVec; ++i) {
-      const int vi = threadIdx.x + i * kCeThreads;
-      if (vi < nvec) cpAsync16(mine + i * kCeThreads * 16, src + vi * 8);
+    for (int i = 0; i < VECS; ++i) {
+      const int vi = threadIdx.x + i * THREADS;
+      if (vi < nvec) cpAsync16(mine + i * THREADS * 16, src + vi * 8);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -515,11 +519,11 @@ __global__ void __launch_bounds__(kCeThreads) crossEntropyKernel(bf16* logits, c
     bf16* lr = logits + (long)row * ld;
     const long tgt = targets[row];
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    float v[kCeMaxVec][8];
+    float v[VECS][8];
     float mx = -INFINITY;
 #pragma unroll
-    for (int i = 0; i < kCeMaxVec; ++i) {
-      const int vi = threadIdx.x + i * kCeThreads;
+    for (int i = 0; i < VECS; ++i) {
+      const int vi = threadIdx.x + i * THREADS;
       if (vi < nvec) {
         unpackBf16x8(*reinterpret_cast<const uint4*>(ceRow + (size_t)vi * 16), v[i]);
 #pragma unroll
@@ -530,8 +534,8 @@ __global__ void __launch_bounds__(kCeThreads) crossEntropyKernel(bf16* logits, c
     mx = blockMax(mx, sm);
     float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < kCeMaxVec; ++i) {
-      const int vi = threadIdx.x + i * kCeThreads;
+    for (int i = 0; i < VECS; ++i) {
+      const int vi = threadIdx.x + i * THREADS;
       if (vi < nvec) {
 #pragma unroll
         for (int j = 0; j < 8; ++j) { v[i][j] = __expf(v[i][j] - mx); s += v[i][j]; }
@@ -543,8 +547,8 @@ __global__ void __launch_bounds__(kCeThreads) crossEntropyKernel(bf16* logits, c
     if (threadIdx.x == 0 && ignore) loss[row] = 0.f;
     const int tvec = ignore ? -1 : (int)(tgt >> 3), tj = (int)(tgt & 7);   // the one vector that holds the target
 #pragma unroll
-    for (int i = 0; i < kCeMaxVec; ++i) {
-      const int vi = threadIdx.x + i * kCeThreads;
+    for (int i = 0; i < VECS; ++i) {
+      const int vi = threadIdx.x + i * THREADS;
       if (vi < nvec) {
         float o[8];
 #pragma unroll
@@ -839,13 +843,15 @@ extern "C" int cocclkGeluBwd(const void* dy, const void* z, void* dz, long n, cu
 extern "C" int cocclkCrossEntropy(void* logits, const long* targets, float* loss, int M, int V, long ld,
                                   float gscale, cudaStream_t s) {
   if (V % 8 || V > kCeThreads * kCeMaxVec * 8 || ld % 8 || M <= 0) return -1;
-  // one CTA an SM walks the rows (the next one prefetched): as many rows for each
-  const int rounds = (M + 147) / 148, grid = (M + rounds - 1) / rounds;
+  // the resident CTAs walk the rows (the next one prefetched): as many rows for each
+  const bool narrow = V <= kCeNarrow;
+  const int resident = 148 * (narrow ? 4 : 1), rounds = (M + resident - 1) / resident, grid = (M + rounds - 1) / rounds;
   if (V * 2 > 40 * 1024) {   // per device: a process may use several
-    const cudaError_t e = cudaFuncSetAttribute(crossEntropyKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeThreads * kCeMaxVec * 16);
+    const cudaError_t e = cudaFuncSetAttribute(crossEntropyKernel<kCeThreads, kCeMaxVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeThreads * kCeMaxVec * 16);
     if (e != cudaSuccess) return (int)e;
   }
-  crossEntropyKernel<<<grid, kCeThreads, (size_t)V * 2, s>>>((bf16*)logits, targets, loss, M, V, ld, gscale);
+  if (narrow) crossEntropyKernel<256, 4><<<grid, 256, (size_t)V * 2, s>>>((bf16*)logits, targets, loss, M, V, ld, gscale);
+  else crossEntropyKernel<kCeThreads, kCeMaxVec><<<grid, kCeThreads, (size_t)V * 2, s>>>((bf16*)logits, targets, loss, M, V, ld, gscale);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }

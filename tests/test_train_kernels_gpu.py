@@ -427,3 +427,24 @@ def test_column_sum_of_wide_matrices_is_not_bound_by_its_fold(cuda):
                 lib.cocclkColSum(x.data_ptr(), out.data_ptr(), 1, sc.data_ptr(), M, N, _lib.cur_stream())
         return _device_us(g.replay, 3) / 50
     assert us(1, 16384) <= 1.6 * us(1, 512)
+
+
+@pytest.mark.parametrize("M,V", [(1, 8), (3, 2048), (593, 8192), (1300, 512), (600, 8200)])
+def test_cross_entropy_narrow_rows(cuda, M, V):
+    """The CTA of 256 threads: less than one vector a thread, the widest row it takes (and the first it does not), fewer and
+    more rows than resident CTAs."""
+    torch.manual_seed(M)
+    logits = (torch.randn(M, V, device=cuda) * 3).to(torch.bfloat16)
+    tgt = torch.randint(0, V, (M,), device=cuda)
+    tgt[0], tgt[-1] = 0, V - 1
+    if M > 2:
+        tgt[1] = -1
+    x = logits.double()
+    loss = fused.cross_entropy(logits, tgt, 0.25)
+    valid = tgt >= 0
+    nll = torch.logsumexp(x, -1) - x.gather(1, tgt.clamp(min=0)[:, None])[:, 0]
+    assert abs(loss.item() - 0.25 * nll[valid].sum().item()) <= 1e-5 * max(1.0, nll.sum().item())
+    want = torch.softmax(x, -1)
+    want[torch.arange(M, device=cuda), tgt.clamp(min=0)] -= 1
+    want = want * valid[:, None] * 0.25
+    assert ((logits.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
