@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kLnThreads) normFwdKernel(const bf16* x, const
     float s = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int vi = threadIdx.x + i * blockDim.x;
+      const int vi = threadIdx.x + i * kLnThreads;
       if (vi < nvec) {
         Vec8<bf16>::load(xr + vi * 8, 8, true, v[i]);
         if (res) {
@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kLnThreads) normFwdKernel(const bf16* x, const
       mu = blockSum(s, sm) / H;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        const int vi = threadIdx.x + i * blockDim.x;
+        const int vi = threadIdx.x + i * kLnThreads;
         if (vi < nvec) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) { const float d = v[i][j] - mu; q += d * d; }
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kLnThreads) normFwdKernel(const bf16* x, const
     if (threadIdx.x == 0) { if (!RMS) mean[row] = mu; rstd[row] = rs; }
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
-      const int vi = threadIdx.x + i * blockDim.x;
+      const int vi = threadIdx.x + i * kLnThreads;
       if (vi < nvec) {
         float g[8], b[8], o[8];
         Vec8<bf16>::load(gamma + vi * 8, 8, true, g);
