@@ -167,10 +167,10 @@ class _Embed(torch.autograd.Function):
             dy = dy.contiguous() if aligned16(dy) else dy.clone(memory_format=torch.contiguous_format)
         lib, st = _lib.lib(), _lib.cur_stream()
         if straight[0]:
-            order = torch.empty(T, dtype=torch.int32, device=dy.device)
-            _lib.check(lib.cocclkEmbedOrder(flat.data_ptr(), order.data_ptr(), T, st), "cocclkEmbedOrder")
-            _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), flat.data_ptr(), order.data_ptr(), wte.main_grad.data_ptr(), T, H,
-                                          wte.shape[0], st), "cocclkEmbedBwd")
+            sc = torch.empty(lib.cocclkEmbedScratchBytes(T, H), dtype=torch.uint8, device=dy.device)
+            _lib.check(lib.cocclkEmbedOrder(flat.data_ptr(), sc.data_ptr(), T, H, st), "cocclkEmbedOrder")
+            _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), sc.data_ptr(), wte.main_grad.data_ptr(), T, H, wte.shape[0], st),
+                       "cocclkEmbedBwd")
         if straight[1]:
             g = wpe.main_grad[first:first + s]
             _lib.check(lib.cocclkEmbedPositionsBwd(dy.data_ptr(), g.data_ptr(), b, s, H, st), "cocclkEmbedPositionsBwd")
@@ -194,7 +194,7 @@ def _wanted_gradient(w, node) -> str:
 def embed_fits(ids, wte, wpe=None, first: int = 0) -> bool:
     """Whether the embedding gradient can go straight into the parameters' gradient buffers: bf16 tables on the GPU with fp32
     `main_grad` buffers, rows of whole 16-byte vectors, and at most 16384 tokens (the kernel that sorts them compares every
-    pair: 45 us at that size, and a run of equal ids is summed by one CTA; larger batches take PyTorch's gradient)."""
+    pair: 72 us at that size; larger batches take PyTorch's gradient)."""
     def table(w):
         mg = getattr(w, "main_grad", None)
         return (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and w.shape[1] % 8 == 0 and

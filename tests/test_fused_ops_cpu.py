@@ -23,14 +23,18 @@ class EmbedKernels:
         self.grads = {t.main_grad.data_ptr(): t.main_grad for t in tables}
         self.calls = []
 
-    def cocclkEmbedOrder(self, ids, order, T, stream):
+    def cocclkEmbedScratchBytes(self, T, H):
+        return 16 * T
+
+    def cocclkEmbedOrder(self, ids, scratch, T, H, stream):
         self.calls.append("order")
+        self.ids = _read(ids, T, ctypes.c_int64, torch.int64)
         return 0
 
-    def cocclkEmbedBwd(self, dy, ids, order, grad, T, H, vocab, stream):
+    def cocclkEmbedBwd(self, dy, scratch, grad, T, H, vocab, stream):
         self.calls.append("rows")
         rows = _read(dy, T * H, ctypes.c_uint16, torch.int32).to(torch.int16).view(torch.bfloat16).view(T, H)
-        self.grads[grad].index_add_(0, _read(ids, T, ctypes.c_int64, torch.int64), rows.float())
+        self.grads[grad].index_add_(0, self.ids, rows.float())
         return 0
 
     def cocclkEmbedPositionsBwd(self, dy, grad, batch, seq, H, stream):

@@ -448,3 +448,40 @@ def test_cross_entropy_narrow_rows(cuda, M, V):
     want[torch.arange(M, device=cuda), tgt.clamp(min=0)] -= 1
     want = want * valid[:, None] * 0.25
     assert ((logits.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
+
+
+@pytest.mark.parametrize("H", [8, 1032])
+@pytest.mark.parametrize("lengths", [(63, 64, 65), (1, 64, 64, 1, 128), (129, 130, 65, 65, 700), (7, 2000, 3)])
+def test_embedding_gradient_of_long_runs(cuda, H, lengths):
+    """Runs of equal ids around the length that is summed in one piece, long ones next to one another, their tokens shuffled."""
+    torch.manual_seed(sum(lengths))
+    T = sum(lengths)
+    ids = torch.repeat_interleave(torch.arange(len(lengths), device=cuda) * 2, torch.tensor(lengths, device=cuda))
+    ids = ids[torch.randperm(T, device=cuda)].view(1, T)
+    wte = torch.zeros(2 * len(lengths), H, device=cuda, dtype=torch.bfloat16).requires_grad_(True)
+    dy = torch.randn(T, H, device=cuda).to(torch.bfloat16)
+    grads = []
+    for _ in range(3):
+        wte.main_grad = torch.ones(2 * len(lengths), H, device=cuda)
+        fused.embed(ids, wte).backward(dy)
+        grads.append(wte.main_grad)
+    assert torch.equal(grads[0], grads[1]) and torch.equal(grads[0], grads[2])
+    want = torch.ones(2 * len(lengths), H, device=cuda, dtype=torch.float64).index_add_(0, ids[0], dy.double())
+    size = torch.ones_like(want).index_add_(0, ids[0], dy.double().abs())
+    assert ((grads[0].double() - want).abs() <= T * 2.0 ** -24 * size + 1e-6).all()
+
+
+@pytest.mark.parametrize("V,H", [(512, 128), (8192, 512)])
+def test_embedding_gradient_of_padded_batches_costs_no_more(cuda, V, H):
+    """Half of the tokens one id (padding) against all of them random (one CTA for a run took 6.5 times as long)."""
+    wte = torch.zeros(V, H, device=cuda, dtype=torch.bfloat16).requires_grad_(True)
+    wte.main_grad = torch.zeros(V, H, device=cuda)
+    dy = torch.randn(16384, H, device=cuda).to(torch.bfloat16)
+    us = []
+    for padded in (False, True):
+        ids = torch.randint(0, V, (2, 8192), device=cuda)
+        if padded:
+            ids[:, 4096:] = 0
+        e = fused.embed(ids, wte)
+        us.append(_device_us(lambda: e.backward(dy, retain_graph=True)))
+    assert us[1] <= 2 * us[0], us
