@@ -365,20 +365,29 @@ extern "C" int cocclkGemmBf16Single(const void* A, long lda, int aMN, const void
 extern "C" int cocclkGemmBf16Small(const void* A, long lda, int aMN, const void* B, long ldb, int bMN, void* C, long ldc, int M, int N,
                                    int K, int epi, const void* bias, void* Z, unsigned int* err, int ranks, cudaStream_t stream);
 
-// Cluster ranks that share a 128 x 64 tile's contraction in gemm_small_kernels.cu, or 0 where the 256 x 256 tiles of the pair
-// kernel are faster. The lines are where a sweep over M, N, K = 65 .. 8192 changed sides (time per call, back to back, bf16
-// out; small against pair): what counts is how much of the GPU the tiles fill (two CTAs an SM: 296) and how long the
-// contraction is. 512 x 512 x 8192 (32 tiles) 15.3 us with 4 ranks, 42.5; 512 x 1536 x 512 (96) 6.6 with 1, 10.8;
-// 512 x 2048 x 4096 (128) 17.9 with 2, 24.9; 1024 x 2048 x 1024 (256) 11.2 with 1, 11.7; 1024 x 2048 x 2048 17.1, 16.4;
-// 512 x 8192 x 512 (512 tiles) 13.8, 9.6. Eight ranks pay only for the fewest tiles: 65 x 256 x 8192 9.4, 12.7 with 4.
-static int smallRanks(int M, int N, int K) {
+// Cluster ranks that share a 128 x 64 tile's contraction in gemm_small_kernels.cu, or 0 where the larger tiles (the pair kernel, up
+// to 128 rows the single-CTA one) are faster. The lines are where a sweep over M = 8 .. 1024, N = 64 .. 16384, K = 64 .. 8192 and
+// the three products of a linear layer changed sides (us a call, back to back; small against large tiles): what counts is how much
+// of the GPU the tiles fill (two CTAs an SM: 296) and how long the contraction is. 512 x 512 x 8192 (32 tiles) 15.3 with 4 ranks,
+// 42.5; 512 x 1536 x 512 (96) 6.6 with 1, 10.8; 512 x 2048 x 4096 (128) 17.9 with 2, 24.9. Eight ranks pay only for the fewest
+// tiles: 65 x 256 x 8192 9.4, 12.7 with 4. Beyond 128 tiles it is ahead only with A along the contraction and full tiles: 1024 x
+// 2048 x 1024 (256) 11.7, 12.1, but the weight gradient 13.1, 12.0, and with few rows, which every column of tiles loads again, 8 x
+// 16384 x 1024 18.4, 12.1 (as a weight gradient, whose 16-byte rows are slow copies, 38.2, 15.1). Few rows lose earlier: 8 x 8192 x
+// 2048 (128) 19.0, 15.3, weight gradients 48 x 8192 x 1024 11.9, 10.6, 136 x 4096 x 4096 27.0, 25.2 and 8 x 4096 x 512 (64) 9.9,
+// 8.2. A short contraction into one column of tiles is all epilogue: 128 x 64 x 64 4.8, 4.5, weight gradient 1024 x 64 x 64 6.2, 5.4.
+static int smallRanks(int M, int N, int K, bool aMN) {
   const long tiles = (long)((M + 127) / 128) * ((N + 63) / 64);
   const int kb = (K + 63) / 64;
+  const bool oneRow = M > 64 && M <= 128;   // one row of tiles, at least half full
+  if (kb <= 4 && (N <= 64 ? oneRow || (aMN && M >= 48) : aMN && oneRow && N <= 128)) return 0;
   if (tiles <= 8 && kb >= 64) return 8;
   if (tiles <= 32) return kb >= 16 ? 4 : (kb >= 8 ? 2 : 1);
-  if (tiles <= 64) return kb >= 64 ? 4 : (kb >= 16 ? 2 : 1);
-  if (tiles <= 128) return kb >= 32 ? 2 : 1;
-  if (tiles <= 256) return kb <= 16 ? 1 : 0;
+  if (tiles <= 64) return aMN && M < 16 && kb <= 16 ? 0 : (kb >= 64 ? 4 : (kb >= 16 ? 2 : 1));
+  if (tiles <= 128) {
+    const bool thin = aMN ? M <= 48 || (kb >= 32 && M % 128 > 0 && M % 128 <= 16) : M <= 16 && kb >= 16 && kb < 64;
+    return thin ? 0 : (kb >= 32 ? 2 : 1);
+  }
+  if (tiles <= 256) return !aMN && M > 128 && kb <= 16 ? 1 : 0;
   return 0;
 }
 // The small kernel stores 16-byte vectors straight from registers.
@@ -393,7 +402,7 @@ extern "C" int cocclkGemmBf16(const void* A, long lda, int aMN, const void* B, l
                               int maxCtas, cudaStream_t stream) {
   const int v = cocclkGemmGetVariant();
   if (v == 0 && maxCtas <= 0 && M > 0 && N > 0 && K > 0 && smallStoresFit(C, ldc, epi, bias, Z)) {
-    const int ranks = smallRanks(M, N, K);
+    const int ranks = smallRanks(M, N, K, aMN != 0);
     if (ranks > 0) return cocclkGemmBf16Small(A, lda, aMN, B, ldb, bMN, C, ldc, M, N, K, epi, bias, Z, err, ranks, stream);
   }
   // The pair kernel works on 256-row tiles: below that half of each pair would idle. A CTA limit of one

@@ -42,3 +42,45 @@ def test_small_outputs_all_epilogues(cuda, M, N, K, a_mn, b_mn):
     G.gemm(a, b, out=wide[:, :N])
     assert ((wide[:, :N].double() - ref).abs() <= tol).all() and (wide[:, N:] == 0).all()
     G.check_errors()
+
+
+@pytest.mark.parametrize("M,N,K,grad", [(8, 16384, 1024, True), (8, 16384, 1024, False), (8, 8192, 1024, True), (136, 8192, 1024, True),
+                                        (8, 8192, 2048, False), (1024, 64, 64, True), (512, 2048, 2048, True), (512, 512, 4096, False)])
+def test_the_rule_picks_no_kernel_that_is_far_behind(cuda, M, N, K, grad):
+    """The kernel chosen by size against the single-CTA one (few rows of a weight gradient took 2.5 times as long on the wrong
+    one), also where the small tiles are far ahead."""
+    if grad:
+        a, b = (torch.randn(K, n, device=cuda).to(torch.bfloat16).t() for n in (M, N))
+        out = torch.zeros(M, N, device=cuda)
+
+        def call():
+            G.gemm(a, b, out=out, accumulate=True)
+    else:
+        a, b = (torch.randn(n, K, device=cuda).to(torch.bfloat16) for n in (M, N))
+        out = torch.zeros(M, N, device=cuda, dtype=torch.bfloat16)
+
+        def call():
+            G.gemm(a, b, out=out)
+
+    def us(variant):
+        G.set_variant(variant)
+        try:
+            call()
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g):
+                for _ in range(20):
+                    call()
+        finally:
+            G.set_variant("auto")
+        best = float("inf")
+        for _ in range(5):
+            s, e = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            s.record()
+            g.replay()
+            e.record()
+            e.synchronize()
+            best = min(best, s.elapsed_time(e) / 20 * 1e3)
+        return best
+    single, auto = us("1cta"), us("auto")
+    assert auto <= 1.25 * single, (auto, single)
+    G.check_errors()
