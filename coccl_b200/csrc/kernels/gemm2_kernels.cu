@@ -14,6 +14,7 @@
 // CTAs, and both leave through the common cluster barrier after freeing TMEM.
 #include "gemm_epilogue.cuh"
 #include "launch_count.h"
+#include "per_device.h"
 
 #include <stdio.h>
 
@@ -228,8 +229,6 @@ extern "C" int cocclkGemmBf16Pair(const void* A, long lda, int aMN, const void* 
   if (rc) return rc;
   rc = bMN ? makeBf16TensorMap(&tb, B, N, K, ldb, 64, 64) : makeBf16TensorMap(&tb, B, K, N, ldb, BK, BNH);
   if (rc) return rc;
-  static int maxClusters = 0;
-  static bool attrSet = false;
   const bool f32 = epi == GEMM_EPI_F32 || epi == GEMM_EPI_F32_ACC;
   CUtensorMap tc = ta;  // placeholder for bf16 outputs (direct stores)
   if (f32) {
@@ -238,9 +237,12 @@ extern "C" int cocclkGemmBf16Pair(const void* A, long lda, int aMN, const void* 
   }
   const int stages = f32 ? kStages - 1 : kStages;
   const int smemBytes = stages * kStageBytes + (f32 ? kEpiStageBytes : 0) + (int)sizeof(Barriers) + 1024;
-  if (!attrSet) {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
+  static PerDevice<int> pairs;
+  const int* maxClusters;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  rc = pairs.get(dev, &maxClusters, [&](int& most) {
+    int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaError_t e = cudaFuncSetAttribute(gemmBf16PairKernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          kStages * kStageBytes + (int)sizeof(Barriers) + 1024);
@@ -248,7 +250,7 @@ extern "C" int cocclkGemmBf16Pair(const void* A, long lda, int aMN, const void* 
       e = cudaFuncSetAttribute(gemmBf16PairKernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                (kStages - 1) * kStageBytes + kEpiStageBytes + (int)sizeof(Barriers) + 1024);
     if (e != cudaSuccess) return (int)e;
-    maxClusters = sms / 2;
+    most = sms / 2;
     // how many pairs the device can hold at once (SMs pair up inside a GPC)
     cudaLaunchConfig_t q = {};
     q.gridDim = dim3((unsigned)(sms / 2) * 2, 1, 1);
@@ -259,14 +261,15 @@ extern "C" int cocclkGemmBf16Pair(const void* A, long lda, int aMN, const void* 
     qa[0].val.clusterDim.x = 2; qa[0].val.clusterDim.y = 1; qa[0].val.clusterDim.z = 1;
     q.attrs = qa; q.numAttrs = 1;
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemmBf16PairKernel<false>, &q) == cudaSuccess && n > 0 && n < maxClusters) maxClusters = n;
+    if (cudaOccupancyMaxActiveClusters(&n, gemmBf16PairKernel<false>, &q) == cudaSuccess && n > 0 && n < most) most = n;
     (void)cudaGetLastError();
-    attrSet = true;
-  }
+    return 0;
+  });
+  if (rc) return rc;
   GemmArgs g;
   g.C = C; g.Z = Z; g.bias = bias; g.M = M; g.N = N; g.K = K; g.ldc = ldc; g.epi = epi; g.aMN = aMN; g.bMN = bMN; g.err = err;
   const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
-  int clusters = maxClusters;
+  int clusters = *maxClusters;
   if (tiles < clusters) clusters = tiles;
   if (maxCtas > 1 && clusters > maxCtas / 2) clusters = maxCtas / 2;
   cudaLaunchConfig_t cfg = {};

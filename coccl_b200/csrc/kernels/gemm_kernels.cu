@@ -12,6 +12,7 @@
 // frees TMEM and returns.
 #include <atomic>
 #include "launch_count.h"
+#include "per_device.h"
 #include "gemm_epilogue.cuh"
 #include <stdio.h>
 #include <string.h>
@@ -336,25 +337,24 @@ extern "C" int cocclkGemmBf16Single(const void* A, long lda, int aMN, const void
   if (rc) return rc;
   rc = bMN ? makeMap(&tb, B, N, K, ldb, 64, 64) : makeMap(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc;
-  static int sms = 0;
-  static bool attrSet = false;
   CUtensorMap tc;
   rc = makeOutputMap(&tc, C, N, M, ldc, epi == GEMM_EPI_F32 || epi == GEMM_EPI_F32_ACC);
   if (rc) return rc;
   const int smemBytes = kStages * kStageBytes + kEpiStageBytes + (int)sizeof(GemmBarriers) + 1024;
-  if (!attrSet) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = cudaFuncSetAttribute(gemmBf16Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes);
-    if (e != cudaSuccess) return (int)e;
-    attrSet = true;
-  }
+  static PerDevice<int> smCount;
+  const int* sms;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  rc = smCount.get(dev, &sms, [&](int& n) {
+    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    return (int)cudaFuncSetAttribute(gemmBf16Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes);
+  });
+  if (rc) return rc;
   GemmArgs g;
   g.C = C; g.Z = Z; g.bias = bias; g.M = M; g.N = N; g.K = K; g.ldc = ldc; g.epi = epi; g.aMN = aMN; g.bMN = bMN;
   g.err = err;
   const int tiles = ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  int grid = tiles < sms ? tiles : sms;
+  int grid = tiles < *sms ? tiles : *sms;
   if (maxCtas > 0 && grid > maxCtas) grid = maxCtas;
   g.stages = kStages;
   gemmBf16Kernel<<<grid, kGemmThreads, smemBytes, stream>>>(ta, tb, tc, g);

@@ -13,6 +13,7 @@
 // Waits are bounded as in gemm_kernels.cu; every thread reaches both cluster barriers whatever happened before.
 #include "gemm_epilogue.cuh"
 #include "launch_count.h"
+#include "per_device.h"
 
 namespace coccl {
 using namespace sm100;
@@ -241,12 +242,14 @@ extern "C" int cocclkGemmBf16Small(const void* A, long lda, int aMN, const void*
   rc = bMN ? makeBf16TensorMap(&tb, B, N, K, ldb, 64, 64) : makeBf16TensorMap(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc;
   const int smemBytes = kStages * kStageBytes + (int)sizeof(Barriers) + 1024;
-  static bool attrSet = false;
-  if (!attrSet) {
-    cudaError_t e = cudaFuncSetAttribute(gemmSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes);
-    if (e != cudaSuccess) return (int)e;
-    attrSet = true;
-  }
+  static PerDevice<bool> allowed;
+  const bool* unused;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  rc = allowed.get(dev, &unused, [&](bool&) {
+    return (int)cudaFuncSetAttribute(gemmSmallKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smemBytes);
+  });
+  if (rc) return rc;
   GemmArgs g;
   g.C = C; g.Z = Z; g.bias = bias; g.M = M; g.N = N; g.K = K; g.ldc = ldc; g.epi = epi; g.aMN = aMN; g.bMN = bMN; g.err = err;
   g.stages = kStages;
