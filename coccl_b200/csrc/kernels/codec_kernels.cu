@@ -71,6 +71,10 @@ extern "C" int cocclkEncode(const void* in, void* out, long count, long chunks, 
   return (int)cudaGetLastError();
 }
 
+// Codecs whose sums take the registers of fewer CTAs only where the tiles are one round of them (cocclkDecodeReduce).
+template <class C> constexpr bool kSumsOneRound = false;
+template <bool ASYM, bool HAD> constexpr bool kSumsOneRound<SdpCodec<4, ASYM, HAD, false>> = true;
+
 extern "C" int cocclkDecodeReduce(const void* in, void* out, long count, long chunks, long reduce, long rawPitch,
                                   long encStride, int dtype, const cocclkCodec* codec, cudaStream_t stream) {
   CodecArgs a{};
@@ -80,10 +84,17 @@ extern "C" int cocclkDecodeReduce(const void* in, void* out, long count, long ch
   const long tiles = (count + kTileElems - 1) / kTileElems;
   bool ok = dispatchCodec(a.codec, [&](auto codecTag) {
     using C = decltype(codecTag);
-    const int grid = gridFor(tiles * chunks, C::kDecodeBlocks);
+    // Sums hold the words of several copies in flight and are faster with the registers of one CTA an SM fewer (8 x 262,147 bf16:
+    // 4 bits, groups of 128 6.4 -> 5.9 us, asymmetric groups of 16 8.3 -> 5.8, TACO 7.5 -> 6.6), unless that means one more round
+    // of tiles (8 x 3,000,008 fp16 TACO, 367 tiles on 296 places: 13.2 us, on 444 10.5) or, for 4-bit digits in groups of 32 and
+    // more, more than one round (8 x 4 Mi bf16, 512 tiles: 12.9 us, 12.5 with three). ZFP, integer work throughout: always.
+    const long items = tiles * chunks, few = (long)smCount() * C::kSumBlocks, many = (long)smCount() * C::kDecodeBlocks;
+    const bool sum = reduce > 1 && (a.codec.kind == kCodecZfp || items <= few ||
+                                    (!kSumsOneRound<C> && (items + few - 1) / few == (items + many - 1) / many));
     dispatchDtype(dtype, [&](auto t) {
       using T = decltype(t);
-      decodeReduceKernel<T, C><<<grid, kTileThreads, 0, stream>>>(a);
+      if (sum) decodeReduceKernel<T, C, C::kSumBlocks><<<gridFor(items, C::kSumBlocks), kTileThreads, 0, stream>>>(a);
+      else decodeReduceKernel<T, C, C::kDecodeBlocks><<<gridFor(items, C::kDecodeBlocks), kTileThreads, 0, stream>>>(a);
     });
   });
   if (!ok) return -1;

@@ -220,7 +220,11 @@ struct SdpCodec {
   static constexpr int kParams = SMALLG ? 4 : 1;
   static constexpr bool kRotated = HAD;
   static constexpr int kMinBlocks = 3;  // resident CTAs per SM the fused kernels are compiled for
-  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3;  // the same for the stand-alone kernels
+  // The same for the stand-alone kernels: encode, decode of one copy, sum of several (codec_kernels.cu says which sums). Eight
+  // chunks of 4 Mi bf16, one CTA an SM fewer against these: 4 bits, groups of 128: encode 19.4 against 19.1 us, decode 22.2
+  // against 20.3; 4 bits, groups of 8: 29.5 (three) and 31.2 (four), 26.1 and 23.1; 8 bits, asymmetric groups of 8, whose
+  // parameters do not fit 80 registers beside a run: 35.6 (three) and 39.8 (four), 28.9 (two) and 32.8 (three).
+  static constexpr int kEncodeBlocks = SMALLG ? 3 : 4, kDecodeBlocks = BITS == 8 && SMALLG && ASYM ? 2 : 3, kSumBlocks = 2;
   static constexpr int kSmemFloats = 8; // shared scratch every kernel passes as `sm` (group reductions wider than a warp)
   static __device__ __forceinline__ void initShared(float*) {}
   static constexpr uint32_t kSignBits = BITS == 4 ? 0x88888888u : 0x80808080u;
@@ -503,7 +507,8 @@ struct MxFp8Codec {
   static constexpr int kWords = 8;
   static constexpr bool kRotated = false;
   static constexpr int kMinBlocks = 3;
-  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3;
+  // 4 x 16 Mi bf16: decode 42.8 us with four, 35.7 with three; 8 x 4 Mi encode 15.7 us with three, 14.6 with four
+  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3, kSumBlocks = 2;
   static constexpr int kSmemFloats = 8;
   static __device__ __forceinline__ void initShared(float*) {}
 
@@ -610,7 +615,7 @@ struct TacoCodec {
   static constexpr bool kRotated = true;
   // stand-alone kernels: 61 and 79 registers, 8 x 3,000,008 fp16 encode 28.3 -> 25.5 us, decode + sum 13.2 -> 10.5 us against
   // one CTA fewer (367 tiles then fit the GPU at once)
-  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3;
+  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3, kSumBlocks = 2;
   static constexpr int kMinBlocks = 2;  // the lane butterflies keep two copies of a run live: 128 registers, no spills
   static constexpr int kSmemFloats = 8;
   static __device__ __forceinline__ void initShared(float*) {}
@@ -748,9 +753,11 @@ struct ZfpCodec {
   static constexpr int kWords = RATE;
   static constexpr bool kRotated = false;
   static constexpr int kMinBlocks = 2;
-  // the coder is a chain of dependent integer work: it needs the warps more than the registers (64 of them: rate 8 encode
-  // 66 us, decode 88 us for 16 Mi values; with 80 and 100 registers 79 and 99 us)
-  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 4;
+  // The coder is a chain of dependent integer work that neither warps nor registers shorten by much: eight chunks of 4 Mi fp32,
+  // encode 72.5 us at rate 8 with four CTAs an SM and 71.3 with three, decode 122.0 and 122.7; rate 4 56.0 and 56.0, 77.2 and
+  // 76.2; rate 16 103.5 and 104.2, 189.0 and 186.7 (64 registers spill there: 8 x 4096 values 15.3 against 13.5 us). Sums, which
+  // hold a second run: 79.0 and 73.2 at rate 4, 130.2 and 126.3 at 8, 207.1 and 201.5 at 16.
+  static constexpr int kEncodeBlocks = 4, kDecodeBlocks = RATE == 16 ? 3 : 4, kSumBlocks = 3;
   static constexpr int kMaxBits = 4 * RATE;
   // the plane tables of oracle/zfp1d_planes.h live in the kernel's shared scratch, behind its first 8 floats
   static constexpr int kSmemFloats = 8 + (int)sizeof(zfp1d::PlaneTables) / 4;

@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKern
 }
 
 // out chunk j = sum_{i<reduce} decode(in chunk i*chunks + j)
-template <typename T, class Codec>
-__global__ void __launch_bounds__(kTileThreads, Codec::kDecodeBlocks) decodeReduceKernel(const CodecArgs a) {
+template <typename T, class Codec, int BLOCKS>
+__global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const CodecArgs a) {
   __shared__ TileStage<T> stage;
   __shared__ float sm[Codec::kSmemFloats];
   Codec::initShared(sm);

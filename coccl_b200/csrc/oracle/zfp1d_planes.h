@@ -5,7 +5,7 @@
 //  * while some value is not yet significant the encoder takes two planes per table look-up, the decoder one;
 //  * from the plane on in which all four values are significant a plane's code is its four bits, so the rest of the string
 //    IS the rest of the stream and is appended (or taken off) with one shift.
-// Integer work bounds it (16 Mi values at 8 bits each: 336 MB that take 51 us to copy): plane by plane, with one table look-up
+// Integer work bounds it (16 Mi values at 8 bits each: 84 MB each way, 13 us to copy): plane by plane, with one table look-up
 // each, 66 us to encode and 89 us to decode them; as strings 42 and 67 us.
 #pragma once
 #include "oracle/zfp1d.h"

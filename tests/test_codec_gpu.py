@@ -185,3 +185,21 @@ def test_mxfp8_chunk_padding_is_zero(cuda, groups):
     del keep   # the encoder's output is allocated over these bytes, or over others that were never written
     enc = C.encode(torch.randn(64 * groups, device=cuda).to(torch.bfloat16), C.MXFP8, 2)
     assert (enc[:, 33 * groups:] == 0).all()
+
+
+@pytest.mark.parametrize("tiles", [1, 296, 297, 445, 593])
+@pytest.mark.parametrize("cfg", [C.SDP4BIT_G128, C.CodecConfig("sdp4bit", 4, 8, False, False), C.CodecConfig("sdp4bit", 4, 16, True, False),
+                                 C.CodecConfig("sdp4bit", 8, 8, True, False), C.CodecConfig("sdp4bit", 8, 512, False, True), C.MXFP8,
+                                 C.TACO_G128, C.ZFP_RATE8, C.CodecConfig("zfp", 16, 4, False, False)],
+                         ids=lambda c: f"{c.kind}{c.bits}g{c.group}{'a' if c.asym else 's'}")
+def test_sums_on_both_sides_of_the_rounds_of_tiles(cuda, cfg, tiles):
+    """One copy and the sum of three, with as many tiles as one more or less than the GPU's places for either kernel, the last
+    tile ragged. The sum is formed in fp32 before the way out of the rotated domain: a few fp32 steps of the values' sizes."""
+    torch.manual_seed(tiles)
+    count = tiles * 8192 - 24
+    x = torch.randn(3 * count, device=cuda)
+    enc = C.encode(x, cfg, 3)
+    one = C.decode(enc, cfg, count, torch.float32, 3).double()
+    got = C.decode_reduce(enc, cfg, count, torch.float32, 1, 3)[0].double()
+    size = one.abs().sum(0).amax()
+    assert ((got - one.sum(0)).abs() <= 64 * 2.0 ** -24 * size).all()
