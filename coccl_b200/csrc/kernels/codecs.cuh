@@ -437,7 +437,7 @@ struct SdpCodec {
   // power is exact unless the scaled parameter leaves the normal range: such groups (|values| < 1e-32) shift instead.
   static __device__ __forceinline__ void accumulate(const Raw& r, float (&acc)[32]) {
     if (!r.valid) return;
-    if (BITS == 4) {
+    if constexpr (BITS == 4) {
       bool tiny = false;
 #pragma unroll
       for (int j = 0; j < kParams; ++j) tiny = tiny || !(r.inv[j] >= 7.8e-34f);   // 2^-110; NaN counts as tiny
@@ -457,10 +457,8 @@ struct SdpCodec {
         const int b = k * kPerWord;
         add(digits2(x & 0xfu, x & 0xf0u), offs2(0, 1), m01, r.off[pj], acc[b], acc[b + 1]);
         add(digits2(x & 0xf00u, x & 0xf000u), offs2(2, 3), m23, r.off[pj], acc[b + 2], acc[b + 3]);
-        if (BITS == 4) {
-          add(digits2(x & 0xf0000u, y & 0xfu), offs2(4, 0), m40, r.off[pj], acc[b + 4], acc[b + 5]);
-          add(digits2(y & 0xf0u, y & 0xf00u), offs2(1, 2), m12, r.off[pj], acc[b + 6], acc[b + 7]);
-        }
+        add(digits2(x & 0xf0000u, y & 0xfu), offs2(4, 0), m40, r.off[pj], acc[b + 4], acc[b + 5]);
+        add(digits2(y & 0xf0u, y & 0xf00u), offs2(1, 2), m12, r.off[pj], acc[b + 6], acc[b + 7]);
       }
     } else {
       accumulateShifted(r, acc);

@@ -296,12 +296,8 @@ struct TileWalk {
   long tiles, chunks, ch, t, stepCh, stepT;
   __device__ __forceinline__ TileWalk(long count, long chunks_) : chunks(chunks_) {
     tiles = (count + kTileElems - 1) / kTileElems;
-    if (tiles <= 0x7fffffffL) {
-      const unsigned n = (unsigned)tiles;
-      ch = blockIdx.x / n; t = blockIdx.x % n; stepCh = gridDim.x / n; stepT = gridDim.x % n;
-    } else {
-      ch = 0; t = blockIdx.x; stepCh = 0; stepT = gridDim.x;   // the grid is smaller than that
-    }
+    const unsigned n = (unsigned)tiles;   // 2^32 tiles would be 2^45 elements
+    ch = blockIdx.x / n; t = blockIdx.x % n; stepCh = gridDim.x / n; stepT = gridDim.x % n;
   }
   __device__ __forceinline__ bool more() const { return ch < chunks; }
   __device__ __forceinline__ void next() {

@@ -92,14 +92,6 @@ __host__ __device__ __forceinline__ uint32_t hash32(uint32_t x) {
   x ^= x >> 16;
   return x;
 }
-__host__ __device__ __forceinline__ uint32_t rngWord(uint32_t seed, uint64_t quadIndex) {
-  uint32_t lo = (uint32_t)quadIndex, hi = (uint32_t)(quadIndex >> 32);
-  return hash32(lo ^ hash32(seed + 0x9e3779b9u * (hi + 1u)));
-}
-// uniform in (0,1) with 8-bit resolution, centred so that E[floor(y+u)] = y up to 2^-9.
-__host__ __device__ __forceinline__ float rngUnit(uint32_t word, int k) {
-  return ((float)((word >> (8 * k)) & 0xffu) + 0.5f) * (1.0f / 256.0f);
-}
 
 // ---------------------------------------------------------------------------
 // 8-element loads/stores with tail guards. `n` = elements still valid from p.
