@@ -186,15 +186,14 @@ class MicroBatchGraph:
         if key is None:
             return False
         order = torch._C._get_sdp_priority_order()   # PyTorch fills it in at its first attention call
-        if key != self.key or not self.snapshot.holds(t.stage, t.cfg) or (self.graph is not None and order != self.sdp_order):
+        if key != self.key or (self.graph is not None and not (self.snapshot.holds(t.stage, t.cfg) and order == self.sdp_order)):
             self._drop()
-            if self.own_code(t.stage):
-                self.key, self.snapshot, self.seen = key, _Snapshot(t.stage, t.cfg), 1
+            self.key, self.seen = key, 1
             return False
         if self.graph is None:
             self.seen += 1
-            if self.seen > 2:
-                self.sdp_order = order
+            if self.seen > 2 and self.own_code(t.stage):
+                self.snapshot, self.sdp_order = _Snapshot(t.stage, t.cfg), order
                 self._capture(t, shape, scale)
         return self.graph is not None
 
