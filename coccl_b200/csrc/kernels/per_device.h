@@ -10,11 +10,16 @@ class PerDevice {
  public:
   static constexpr int kDevices = 64;
 
-  // *out = the value of device `dev`, filled in by init(value) at its first use. init returns an error code; after an error the
-  // next use tries again. Returns that code, or 101 (invalid device) for an index out of range.
+  // *out = the value of device `dev`, filled in by init(value) at its first use. init returns an error code, which is returned;
+  // after an error the next use tries again. Devices beyond the table are initialised at every use.
   template <class Init>
   int get(int dev, const T** out, Init init) {
-    if (dev < 0 || dev >= kDevices) return 101;
+    if (dev < 0 || dev >= kDevices) {
+      static thread_local T other;
+      other = T{};
+      *out = &other;
+      return init(other);
+    }
     if (!ready_[dev].load(std::memory_order_acquire)) {
       std::lock_guard<std::mutex> lock(mutex_);
       if (!ready_[dev].load(std::memory_order_relaxed)) {

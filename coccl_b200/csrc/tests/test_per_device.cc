@@ -26,8 +26,17 @@ TEST(per_device_a_failure_is_returned_and_tried_again) {
   EXPECT(p.get(2, &v, [](int&) { return 7; }) == 7);
   EXPECT(v == nullptr);
   EXPECT(p.get(2, &v, [](int& x) { x = 5; return 0; }) == 0 && *v == 5);
-  EXPECT(p.get(-1, &v, [](int&) { return 0; }) == 101);
-  EXPECT(p.get(PerDevice<int>::kDevices, &v, [](int&) { return 0; }) == 101);
+}
+
+TEST(per_device_devices_beyond_the_table_are_initialised_at_every_use) {
+  PerDevice<int> p;
+  int calls = 0;
+  for (int dev : {PerDevice<int>::kDevices, -1, PerDevice<int>::kDevices}) {
+    const int* v = nullptr;
+    EXPECT(p.get(dev, &v, [&](int& x) { x += 3; ++calls; return 0; }) == 0);
+    EXPECT(v != nullptr && *v == 3);
+  }
+  EXPECT(calls == 3);
 }
 
 TEST(per_device_threads_share_one_initialisation) {
