@@ -114,8 +114,7 @@ _PROTOS = {
     "cocclkSwigluFwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "cocclkSwigluBwd": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_void_p]),
     "cocclkEmbedScratchBytes": (c_long, [c_int, c_int]),
-    "cocclkEmbedOrder": (c_int, [c_void_p, c_void_p, c_int, c_int, c_void_p]),
-    "cocclkEmbedBwd": (c_int, [c_void_p] * 3 + [c_int, c_int, c_long, c_void_p]),
+    "cocclkEmbedBwd": (c_int, [c_void_p] * 4 + [c_int, c_int, c_long, c_void_p]),
     "cocclkEmbedPositionsBwd": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_void_p]),
     "cocclkColSumBlocks": (c_int, [c_int]),
     "cocclkColSum": (c_int, [c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_void_p]),

@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) embedPositionsKernel(const bf16* dy, floa
 
 using namespace coccl;
 
-// Scratch of the two: places, then the parts of long runs, then a counter per window and block of columns.
+// Scratch: places, then the parts of long runs, then a counter per window and block of columns.
 struct EmbedScratch {
   long windows, colBlocks, partsAt, countersAt, bytes;
   EmbedScratch(int T, int H) : windows(((long)T + kEmbPiece - 1) / kEmbPiece), colBlocks((H + kEmbCols - 1) / kEmbCols) {
@@ -196,22 +196,16 @@ struct EmbedScratch {
 };
 extern "C" long cocclkEmbedScratchBytes(int T, int H) { return T > 0 && H > 0 ? EmbedScratch(T, H).bytes : 0; }
 
-extern "C" int cocclkEmbedOrder(const long* ids, void* scratch, int T, int H, cudaStream_t s) {
+extern "C" int cocclkEmbedBwd(const void* dy, const long* ids, void* scratch, float* grad, int T, int H, long vocab, cudaStream_t s) {
   if (T <= 0 || H <= 0 || H % 8) return -1;
   const EmbedScratch L(T, H);
   char* b = (char*)scratch;
-  embedOrderKernel<<<(T + 7) / 8, 256, 0, s>>>(ids, (int4*)b, (unsigned*)(b + L.countersAt), (int)(L.windows * L.colBlocks), T);
-  cocclkCountLaunches(1);
-  return (int)cudaGetLastError();
-}
-
-extern "C" int cocclkEmbedBwd(const void* dy, void* scratch, float* grad, int T, int H, long vocab, cudaStream_t s) {
-  if (T <= 0 || H <= 0 || H % 8) return -1;
-  const EmbedScratch L(T, H);
-  char* b = (char*)scratch;
-  embedRowsKernel<<<dim3((unsigned)T, (unsigned)L.colBlocks), kEmbThreads, 0, s>>>((const bf16*)dy, (const int4*)b, (float*)(b + L.partsAt),
-                                                                            (unsigned*)(b + L.countersAt), grad, T, H, vocab);
-  cocclkCountLaunches(1);
+  int4* places = (int4*)b;
+  unsigned* counters = (unsigned*)(b + L.countersAt);
+  embedOrderKernel<<<(T + 7) / 8, 256, 0, s>>>(ids, places, counters, (int)(L.windows * L.colBlocks), T);
+  embedRowsKernel<<<dim3((unsigned)T, (unsigned)L.colBlocks), kEmbThreads, 0, s>>>((const bf16*)dy, places, (float*)(b + L.partsAt), counters,
+                                                                            grad, T, H, vocab);
+  cocclkCountLaunches(2);
   return (int)cudaGetLastError();
 }
 

@@ -34,13 +34,11 @@ int cocclkRotateBwdGrid(int tokens);
 int cocclkRotateBwd(const void* dq, const void* dk, const void* dv, const void* qkv, void* dqkv, const float* cosT,
                     const float* sinT, const void* qw, const void* kw, float* dqw, float* dkw, int accumulate, float* scratch,
                     int tokens, int seq, int nh, int nkv, int D, float eps, cudaStream_t s);
-// embed_kernels.cu. Order: the tokens sorted by id, equal ids in token order (T^2 comparisons, meant for up to 16384 tokens), into
-// scratch (cocclkEmbedScratchBytes(T, H), 16-byte aligned, also read and written by Bwd). Bwd: grad (fp32 [vocab][H]) row of every
-// id += sum of its tokens' rows of dy (bf16 [T][H]), in a fixed order; once per Order.
-// PositionsBwd: grad (fp32 [seq][H]) += sum over the batch of dy [batch][seq][H]. H % 8 == 0.
+// embed_kernels.cu. Bwd: grad (fp32 [vocab][H]) row of every id += sum of its tokens' rows of dy (bf16 [T][H]), in a fixed order
+// (the tokens are sorted by id with T^2 comparisons, meant for up to 16384 of them). scratch: cocclkEmbedScratchBytes(T, H),
+// 16-byte aligned. PositionsBwd: grad (fp32 [seq][H]) += sum over the batch of dy [batch][seq][H]. H % 8 == 0.
 long cocclkEmbedScratchBytes(int T, int H);
-int cocclkEmbedOrder(const long* ids, void* scratch, int T, int H, cudaStream_t s);
-int cocclkEmbedBwd(const void* dy, void* scratch, float* grad, int T, int H, long vocab, cudaStream_t s);
+int cocclkEmbedBwd(const void* dy, const long* ids, void* scratch, float* grad, int T, int H, long vocab, cudaStream_t s);
 int cocclkEmbedPositionsBwd(const void* dy, float* grad, int batch, int seq, int H, cudaStream_t s);
 // z [M][2 F] = gate | up: y = silu(gate) * up, and its gradient. F % 8 == 0.
 int cocclkSwigluFwd(const void* z, void* y, int M, int F, cudaStream_t s);

@@ -168,9 +168,8 @@ class _Embed(torch.autograd.Function):
         lib, st = _lib.lib(), _lib.cur_stream()
         if straight[0]:
             sc = torch.empty(lib.cocclkEmbedScratchBytes(T, H), dtype=torch.uint8, device=dy.device)
-            _lib.check(lib.cocclkEmbedOrder(flat.data_ptr(), sc.data_ptr(), T, H, st), "cocclkEmbedOrder")
-            _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), sc.data_ptr(), wte.main_grad.data_ptr(), T, H, wte.shape[0], st),
-                       "cocclkEmbedBwd")
+            _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), flat.data_ptr(), sc.data_ptr(), wte.main_grad.data_ptr(), T, H,
+                                          wte.shape[0], st), "cocclkEmbedBwd")
         if straight[1]:
             g = wpe.main_grad[first:first + s]
             _lib.check(lib.cocclkEmbedPositionsBwd(dy.data_ptr(), g.data_ptr(), b, s, H, st), "cocclkEmbedPositionsBwd")
