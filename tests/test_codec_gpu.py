@@ -2,6 +2,7 @@
 import pytest
 import torch
 
+from coccl_b200 import _lib
 from coccl_b200.ops import codec as C
 
 pytestmark = pytest.mark.gpu
@@ -181,9 +182,11 @@ def test_sdp4bit_tiny_groups_decode_like_the_oracle(cuda, magnitude):
 def test_mxfp8_chunk_padding_is_zero(cuda, groups):
     """The scale bytes of a chunk end anywhere in a word; the rest of the word is part of the stream and is written."""
     n = C.MXFP8.encoded_chunk_bytes(32 * groups, torch.bfloat16)
-    keep = torch.full((2, n), 255, dtype=torch.uint8, device=cuda)
-    del keep   # the encoder's output is allocated over these bytes, or over others that were never written
-    enc = C.encode(torch.randn(64 * groups, device=cuda).to(torch.bfloat16), C.MXFP8, 2)
+    x = torch.randn(64 * groups, device=cuda).to(torch.bfloat16)
+    enc = torch.full((2, n), 255, dtype=torch.uint8, device=cuda)   # memory that held something else
+    _lib.check(_lib.lib().cocclkEncode(x.data_ptr(), enc.data_ptr(), 32 * groups, 2, 32 * groups, n, C.DTYPE_CODE[x.dtype],
+                                       C.MXFP8.to_c(x.dtype), _lib.cur_stream()), "cocclkEncode")
+    assert torch.equal(enc, C.encode(x, C.MXFP8, 2))
     assert (enc[:, 33 * groups:] == 0).all()
 
 

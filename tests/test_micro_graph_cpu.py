@@ -86,3 +86,12 @@ def test_size_rule_counts_what_the_graph_would_keep():
     assert MicroBatchGraph.worth_it(GPTConfig(vocab=1024, **small), 8192)
     assert MicroBatchGraph.worth_it(GPTConfig(vocab=50304, **small), 8192)
     assert not MicroBatchGraph.worth_it(GPTConfig(vocab=50304, **small), 16384)   # 1.6 GB of logits
+
+
+def test_size_rule():
+    from coccl_b200.models.gpt import GPTConfig
+    from coccl_b200.train import MicroBatchGraph
+    small = GPTConfig(n_layer=2, hidden=256, n_head=4, ffn=1024, seq_len=96, vocab=1024)
+    assert MicroBatchGraph.worth_it(small, 192)
+    assert not MicroBatchGraph.worth_it(small, 16385)
+    assert not MicroBatchGraph.worth_it(GPTConfig(), 4096)

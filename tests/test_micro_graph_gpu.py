@@ -180,11 +180,3 @@ def test_gradients_that_autograd_hands_over_are_not_left_to_a_capture(cuda):
         ga, gb = a.stage.wte.main_grad, b.stage.wte.main_grad
         assert gb.norm() > 0 and (ga - gb).norm() <= 3e-2 * gb.norm(), step
     assert a.micro_graph.graph is None
-
-
-def test_size_rule(cuda):
-    from coccl_b200.models.gpt import GPTConfig
-    from coccl_b200.train import MicroBatchGraph
-    assert MicroBatchGraph.worth_it(_cfg("gpt"), 192)
-    assert not MicroBatchGraph.worth_it(_cfg("gpt"), 16385)
-    assert not MicroBatchGraph.worth_it(GPTConfig(), 4096)
