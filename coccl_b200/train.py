@@ -48,8 +48,8 @@ def split_layers(n_layer: int, stages: int) -> list[tuple[int, int]]:
 
 
 def _own_code() -> list:
-    """(namespace, names, values) of the functions, classes and methods that a pass through a stage can reach by name, as this
-    package and PyTorch define them."""
+    """(namespace, look-up of names in it, what it finds) of the functions, classes and methods that a pass through a stage can
+    reach by name, as this package and PyTorch define them."""
     from torch.nn.modules import module as nnm
     from .models import gpt, llama
     from .ops import fused, gemm
@@ -59,7 +59,14 @@ def _own_code() -> list:
               for x in (gpt, llama, fused, gemm, _lib, *own)]
     spaces += [(vars(torch.nn.functional), ["scaled_dot_product_attention", "embedding", "silu"]), (vars(nnm.Module), ["__call__", "_call_impl"]),
                (vars(torch.Tensor), ["backward"]), (vars(torch.autograd), ["backward"])]
-    return [(ns, keys, [ns[k] for k in keys]) for ns, keys in spaces]
+    return [(ns, operator.itemgetter(*keys), operator.itemgetter(*keys)(ns)) for ns, keys in spaces if keys]
+
+
+def _own_code_in_place() -> bool:
+    try:
+        return all(get(ns) == was for ns, get, was in _OWN_CODE)   # of functions and classes: by identity
+    except KeyError:
+        return False
 
 
 class _Snapshot:
@@ -82,23 +89,26 @@ class _Snapshot:
         module = isinstance(obj, torch.nn.Module)
         if module or (type(obj).__module__.startswith(__package__) and hasattr(obj, "__dict__")):
             obj = obj.__dict__
-        if isinstance(obj, (dict, list, tuple)):
-            self.parts.append((obj, self._content(obj)))
-            for v in [v for k, v in obj.items() if not (module and k in self.HOOKS)] if isinstance(obj, dict) else obj:
+        if isinstance(obj, dict):
+            self.parts.append((obj.values(), [*obj.values()], obj, [*obj]))
+            for k, v in obj.items():
+                if not (module and k in self.HOOKS):
+                    self._walk(v, seen)
+        elif isinstance(obj, (list, tuple)):
+            self.parts.append((obj, [*obj], (), []))
+            for v in obj:
                 self._walk(v, seen)
-
-    @staticmethod
-    def _content(c):
-        return [*c, *c.values()] if isinstance(c, dict) else list(c)
 
     def holds(self, *roots) -> bool:
         if not all(map(operator.is_, roots, self.roots)):
             return False
-        for c, was in self.parts:
-            now = self._content(c)
-            if len(now) != len(was) or not all(map(operator.is_, now, was)):
+        for values, were, keys, named in self.parts:
+            if len(values) != len(were) or not all(map(operator.is_, values, were)) or [*keys] != named:
                 return False
         return True
+
+
+_shape_of, _type_of, _trains = map(operator.attrgetter, ("shape", "dtype", "requires_grad"))
 
 
 class MicroBatchGraph:
@@ -167,10 +177,12 @@ class MicroBatchGraph:
                     torch.get_float32_matmul_precision(), mm.allow_bf16_reduced_precision_reduction,
                     torch.get_default_dtype(), torch.is_inference_mode_enabled())
         params = [p for m in t.stage.modules() for p in m._parameters.values() if p is not None]
-        if any(p._backward_hooks or p._post_accumulate_grad_hooks or getattr(p, "main_grad", None) is None for p in params):
+        grads = [getattr(p, "main_grad", None) for p in params]
+        if any([p._backward_hooks or p._post_accumulate_grad_hooks for p in params]) or any([g is None for g in grads]):
             return None
-        params = [(p.data_ptr(), p.main_grad.data_ptr(), p.main_grad.dtype, p.shape, p.stride(), p.requires_grad) for p in params]
-        return tuple(shape), scale, G.get_variant(), torch.cuda.current_device(), t._loss_acc.data_ptr(), switches, params
+        buffers = [*map(torch.Tensor.data_ptr, params), *map(torch.Tensor.data_ptr, grads), *map(_shape_of, params),
+                   *map(_type_of, grads), *map(_trains, params)]
+        return tuple(shape), scale, G.get_variant(), torch.cuda.current_device(), t._loss_acc.data_ptr(), switches, buffers
 
     def ready(self, t: "Trainer", shape, scale) -> bool:
         """Whether trainer t's micro-batches of this step are to be replayed (captures the graph at the third equal step)."""
@@ -180,7 +192,7 @@ class MicroBatchGraph:
         if not (torch.device(t.device).type == "cuda" and t.schedule is None and t.groups is None and not t.fsdp and
                 t.cfg.n_experts == 0 and self.worth_it(t.cfg, shape[0] * (shape[1] - 1)) and
                 self._plain_context(t.stage) and "_micro_batch" not in vars(t) and type(t)._micro_batch is Trainer._micro_batch and
-                all(all(map(operator.is_, map(ns.get, keys), was)) for ns, keys, was in _OWN_CODE)):
+                _own_code_in_place()):
             return False
         key = self._key(t, shape, scale)
         if key is None:

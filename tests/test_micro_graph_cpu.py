@@ -56,9 +56,9 @@ def test_snapshot_notices_what_a_pass_would_have_looked_up(arch, change):
 @pytest.mark.parametrize("arch", ["gpt", "llama"])
 def test_only_the_package_s_own_code_is_replayed(arch, monkeypatch):
     from coccl_b200.ops import fused
-    from coccl_b200.train import MicroBatchGraph, _OWN_CODE
+    from coccl_b200.train import MicroBatchGraph
+    from coccl_b200.train import _own_code_in_place as unchanged
     own = MicroBatchGraph.own_code
-    unchanged = lambda: all(ns.get(k) is v for ns, keys, was in _OWN_CODE for k, v in zip(keys, was))   # noqa: E731
     assert own(_trainer(arch).stage) and unchanged()
     t = _trainer(arch)
     t.stage.layers[0].forward = lambda *a: a
