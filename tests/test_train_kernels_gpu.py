@@ -415,7 +415,7 @@ def test_column_sum_block_rules(cuda, M, N):
 
 
 def test_column_sum_of_wide_matrices_is_not_bound_by_its_fold(cuda):
-    """A column sum of few rows writes and folds more than it reads; it must cost about what a copy of one row's launches does."""
+    """A column sum of one row is two launches whatever its width (a fold with idle warps in a second wave took 1.5 times as long)."""
     lib = _lib.lib()
 
     def us(M, N):
@@ -426,7 +426,7 @@ def test_column_sum_of_wide_matrices_is_not_bound_by_its_fold(cuda):
             for _ in range(50):
                 lib.cocclkColSum(x.data_ptr(), out.data_ptr(), 1, sc.data_ptr(), M, N, _lib.cur_stream())
         return _device_us(g.replay, 3) / 50
-    assert us(1, 16384) <= 1.6 * us(1, 512)
+    assert us(1, 16384) <= 1.33 * us(1, 512)
 
 
 @pytest.mark.parametrize("M,V", [(1, 8), (3, 2048), (593, 8192), (1300, 512), (600, 8200)])
@@ -448,6 +448,17 @@ def test_cross_entropy_narrow_rows(cuda, M, V):
     want[torch.arange(M, device=cuda), tgt.clamp(min=0)] -= 1
     want = want * valid[:, None] * 0.25
     assert ((logits.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6).all()
+
+
+def test_cross_entropy_of_narrow_rows_costs_less(cuda):
+    """A sixteenth of the logits a row (with a whole SM for a row it took 0.84 of the time)."""
+    lib = _lib.lib()
+
+    def us(V):
+        lg, tgt = torch.zeros(4096, V, device=cuda, dtype=torch.bfloat16), torch.zeros(4096, dtype=torch.int64, device=cuda)
+        loss = torch.empty(4096, device=cuda)
+        return _device_us(lambda: lib.cocclkCrossEntropy(lg.data_ptr(), tgt.data_ptr(), loss.data_ptr(), 4096, V, V, 1e-3, _lib.cur_stream()), 50)
+    assert us(512) <= 0.66 * us(8192)
 
 
 @pytest.mark.parametrize("H", [8, 1032])
