@@ -127,7 +127,7 @@ def main():
     elif a.what == "train":
         # the trainer's own kernels on one transformer layer's shapes: LayerNorm forward + backward (with the column sums of
         # the gamma / beta gradients), bias-gradient column sums (inside the linear's backward), cross-entropy forward +
-        # backward, AdamW with fp32 master weights
+        # backward, the Llama layers' norm, rotation and gate, the embedding, AdamW with fp32 master weights
         from .ops import fused as F_
         T_, H_ = a.tokens, a.hidden
         x = torch.randn(T_, H_, device=dev, dtype=torch.bfloat16, requires_grad=True)
@@ -157,6 +157,38 @@ def main():
             loss = F_.cross_entropy(logits, tgt, 1.0 / T_)
             loss.backward()
             logits.grad = None
+        # the Llama layers' kernels at the same width: norm with a residual, rotation of 32 + 8 heads with their norm, gate
+        from .models.llama import _rope_tables
+        res = torch.randn(T_, H_, device=dev, dtype=torch.bfloat16, requires_grad=True)
+        d_ = 128
+        nh = H_ // d_
+        nkv = max(1, nh // 4)
+        qkv = torch.randn(T_, (nh + 2 * nkv) * d_, device=dev, dtype=torch.bfloat16, requires_grad=True)
+        qw, kw = (torch.ones(d_, device=dev, dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+        cos, sin = _rope_tables(min(T_, 2048), d_, 1.0e6, dev)
+        z = torch.randn(T_, 6 * H_, device=dev, dtype=torch.bfloat16, requires_grad=True)
+
+        def rms():
+            torch.autograd.backward(F_.rms_norm(x, g, 1e-5, res), (dy, dy))
+            x.grad = g.grad = res.grad = None
+
+        def rotate():
+            q, k, v = F_.rotate_qkv(qkv, cos, sin, nh, nkv, qw, kw)
+            torch.autograd.backward((q, k, v), (q.detach(), k.detach(), v.detach()))
+            qkv.grad = qw.grad = kw.grad = None
+
+        def gate():
+            y = F_.swiglu(z)
+            y.backward(y.detach())
+            z.grad = None
+        wte = torch.randn(V_, H_, device=dev, dtype=torch.bfloat16, requires_grad=True)
+        wte.main_grad = torch.zeros(V_, H_, device=dev)
+        ids = torch.randint(0, V_, (1, T_), device=dev)
+
+        def emb():
+            F_.embed(ids, wte).backward(dy)
+        t_rms, t_rot, t_gate, t_emb = (timed(f, a.iters, a.warmup) for f in (rms, rotate, gate, emb))
+        out.update(rms_norm_residual_fwd_bwd_ms=t_rms, rotate_fwd_bwd_ms=t_rot, swiglu_fwd_bwd_ms=t_gate, embedding_fwd_bwd_ms=t_emb)
         np_ = 64 << 20
         master = torch.randn(np_, device=dev)
         m1, v1 = torch.zeros_like(master), torch.zeros_like(master)

@@ -95,6 +95,8 @@ __device__ __forceinline__ void encodeTiles(const T* src, const ChunkLayout& L, 
 // waits for a whole batch, and inside a batch the warps run free. An item on its own costs about 3 us in the two (8 ranks
 // emulated, 16 Mi bf16, two-shot: one tile an item 738 us, six tiles 307 us for the same work; batched 381 and 293 us), so
 // batches grow with the items a CTA has; one with less than four keeps single items, because a batch delays the receivers.
+// That is the case of ranks that share a GPU. A rank alone on its GPU has about one item a CTA (the slices are cut so) until a
+// slice has its most tiles: batches then need some 170 million elements a rank, or a limit on the CTAs.
 constexpr int kMaxBatch = 4;
 __device__ __forceinline__ int batchOf(int items) {
   const int each = (items + (int)gridDim.x - 1) / (int)gridDim.x;

@@ -492,12 +492,12 @@ __device__ __forceinline__ void cpAsync16(uint32_t smem, const void* g) {
 // rows with target < 0 get loss 0 and a zero gradient.
 //
 // A row of 50304 logits fills the registers of a CTA that fills the SM, so load, two reductions, exponentials and store of a
-// row followed one another with the memory idle in between (4096 rows 336 us, 824 MB: 126 us to copy). The next row is now
+// row followed one another with the memory idle in between (4096 rows 324 us, 824 MB: 126 us to copy). The next row is now
 // on its way into shared memory while this one is worked on; a thread copies exactly the vectors it reads back, so the copy
-// needs no barrier, only the thread's own wait; and only the one vector that holds the target looks at it. 254 us, bound by
+// needs no barrier, only the thread's own wait; and only the one vector that holds the target looks at it. 217 us, bound by
 // the exponentials and the two block reductions of the one CTA an SM has room for. Rows of up to 8192 logits leave most of 1024
-// threads without one and take 256, four CTAs an SM, so that one row's
-// reductions run beside another's arithmetic: 4096 x 512 71 us with 1024 threads, 12.5 with 256, 4096 x 8192 85 and 26 us.
+// threads without one and take 256, four CTAs an SM, so that one row's reductions run beside another's arithmetic: 4096 x 512
+// 71 us with 1024 threads, 12.5 with 256, 4096 x 8192 85 and 26 us.
 template <int THREADS, int VECS>
 __global__ void __launch_bounds__(THREADS) crossEntropyKernel(bf16* logits, const long* targets, float* loss,
                                                                  int M, int V, long ld, float gscale) {
