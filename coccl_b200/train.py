@@ -15,7 +15,7 @@ from dataclasses import dataclass
 import torch
 
 from . import _lib
-from .models.gpt import GPTConfig, GPTStage, ParamStore, TransformerLayer
+from .models.gpt import GPTConfig, GPTStage, NoTP, ParamStore, TransformerLayer
 from .parallel.dp import DistributedOptimizer
 
 
@@ -149,11 +149,12 @@ class MicroBatchGraph:
 
     @staticmethod
     def own_code(stage) -> bool:
-        """Whether `stage` is built of this package's own dense modules, with none of their methods replaced."""
+        """Whether `stage` is built of this package's own dense modules and single-GPU context, none of their methods replaced."""
         from .models.llama import LlamaLayer
+        parts = [*stage.modules(), *(m.tp for m in stage.modules() if hasattr(m, "tp"))]
         return type(stage) is GPTStage and all(
-            type(m) in (GPTStage, TransformerLayer, LlamaLayer, torch.nn.ModuleList) and
-            not any(callable(getattr(type(m), k, None)) for k in vars(m)) for m in stage.modules())
+            type(m) in (GPTStage, TransformerLayer, LlamaLayer, torch.nn.ModuleList, NoTP) and
+            not any(callable(getattr(type(m), k, None)) for k in vars(m)) for m in parts)
 
     @staticmethod
     def _plain_context(stage) -> bool:

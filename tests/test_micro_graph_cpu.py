@@ -70,6 +70,12 @@ def test_only_the_package_s_own_code_is_replayed(arch, monkeypatch):
     t.stage.layers[1].__class__ = type("Other", (type(t.stage.layers[1]),), {})
     assert not own(t.stage)
     t = _trainer(arch)
+    t.stage.layers[0].tp.linear_scatter = lambda x, w, bias=None: x
+    assert not own(t.stage)
+    t = _trainer(arch)
+    t.stage.layers[0].tp = type("Other", (type(t.stage.tp),), {})()
+    assert not own(t.stage)
+    t = _trainer(arch)
     t.stage.extra = torch.nn.Linear(2, 2)
     assert not own(t.stage)
     for space, name in ((fused, "layer_norm"), (fused, "swiglu"), (type(t.stage), "embed"), (torch.nn.functional, "embedding")):
