@@ -113,7 +113,7 @@ def build(verbose: bool = False, jobs: int | None = None) -> Path:
 
     # bounds-checked twin (COCCL_CHECKED_KERNELS=1 makes the Python layer load it): the same objects, except that the
     # translation units with the codec accesses are compiled with -DCOCCL_BOUNDS_CHECK
-    checked_units = {CSRC / "kernels" / "collective_kernels.cu", CSRC / "kernels" / "codec_kernels.cu"}
+    checked_units = {*(CSRC / "kernels").glob("collective_*.cu"), CSRC / "kernels" / "codec_kernels.cu"}
     with cf.ThreadPoolExecutor(jobs) as ex:
         cobjs = list(ex.map(lambda s: _compile(s, verbose, hdr, ("-DCOCCL_BOUNDS_CHECK",), ".checked"), sorted(checked_units)))
     cso = LIB / "libcoccl_checked.so"

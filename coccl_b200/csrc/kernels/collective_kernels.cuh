@@ -69,19 +69,44 @@ __device__ __forceinline__ unsigned int* flagPtr(unsigned int* base, int region,
   return base + ((long)region * kMaxRanks + src) * kMaxSlices + slice;
 }
 
-// Encode the tiles [t0, t1) of one source chunk and store the result into the nDst chunk buffers dst(0), dst(1), ...
-template <typename T, class Codec, class Dst>
+// Stages of raw values: for codecs that are bound by instructions the next tile's are on their way to shared memory while this one
+// is encoded, except for fp32, where the loads alone take 0.95 of the copy rate with four CTAs an SM and a second stage leaves
+// room for three (4 bits, groups of 128, 8 x 8 Mi: fp32 48.1 us with one stage, 52.9 with two; bf16 38.5 and 35.6; 8 bits in
+// groups of 8, bound by stores: bf16 63.7 and 84.3).
+template <typename T, class Codec>
+constexpr int kEncodeStages = sizeof(T) == 2 && Codec::kEncodeAhead ? 2 : 1;
+
+// Encode the tiles [t0, t1) of one source chunk and store the result into the nDst chunk buffers dst(0), dst(1), ... With DELTA
+// what is sent is the change since the previous result, `prev`.
+template <typename T, class Codec, bool DELTA, class Dst>
 __device__ __forceinline__ void encodeTiles(const T* src, const ChunkLayout& L, const CodecCfg& c, long t0, long t1,
-                                            int nDst, Dst dst, TileStage<T>& stage, float* sm,
-                                            uint64_t rngBase, const T* prev = nullptr) {
-  for (long t = t0; t < t1; ++t) {
-    const long e0 = t * kTileElems;
-    const long e = e0 + (long)threadIdx.x * kElemsPerThread;
+                                            int nDst, Dst dst, TileStage<T>* stage, float* sm,
+                                            uint64_t rngBase, const T* prev) {
+  constexpr int S = DELTA ? 1 : kEncodeStages<T, Codec>;
+  auto start = [&](const T* chunk, long t, int s) {
+    const long e0 = t * kTileElems, left = L.count - e0;
+    if (t < t1) TileIO<T, false>::template bring<S == 2>(chunk + e0, left, e0 == 0, TileIO<T, false>::fast(chunk + e0, left), stage[s]);
+    if (S == 2) commitCopies();
+  };
+  auto take = [&](const T* chunk, long t, int s, float (&v)[32]) {
+    const long e0 = t * kTileElems, left = L.count - e0;
+    TileIO<T, false>::take(chunk + e0, left, e0 == 0, TileIO<T, false>::fast(chunk + e0, left), stage[s], v);
+  };
+  int s = 0;
+  __syncwarp();   // the stages are not in use any more
+  if (S == 2) start(src, t0, 0);
+  for (long t = t0; t < t1; ++t, s ^= S - 1) {
+    const long e = t * kTileElems + (long)threadIdx.x * kElemsPerThread;
     float v[32];
-    TileIO<T>::load(src, L.count, e0, TileIO<T>::fastTile(src, L.count, e0), stage, v);
-    if (prev != nullptr) {  // delta coding: what is sent is the change since the previous result
+    __syncwarp();
+    start(src, S == 2 ? t + 1 : t, S == 2 ? s ^ 1 : 0);
+    if (S == 2) waitCopies<1>();
+    take(src, t, s, v);
+    if constexpr (DELTA) {
       float pv[32];
-      TileIO<T>::load(prev, L.count, e0, TileIO<T>::fastTile(prev, L.count, e0), stage, pv);
+      __syncwarp();
+      start(prev, t, 0);
+      take(prev, t, 0, pv);
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] -= pv[i];
     }
@@ -126,9 +151,58 @@ __device__ __forceinline__ bool waitAll(int n, Addr addr, Item item, unsigned in
 }
 static_assert(kMaxBatch * kMaxRanks <= 32, "a batch's flags are handled by one warp");
 
-template <typename T, class Codec>
+// Decode the tiles [t0, t1) of one encoded chunk into dst. With ADD they are added to what dst holds.
+template <typename T, class Codec, bool ADD>
+__device__ __forceinline__ void decodeTiles(const uint8_t* enc, T* dst, const ChunkLayout& L, const CodecCfg& c, long t0, long t1,
+                                            bool aligned, TileStage<T>& stage, float* sm) {
+  auto put = [&](long t, float (&acc)[32]) {
+    const long e0 = t * kTileElems, left = L.count - e0;
+    const bool fast = TileIO<T, false>::fast(dst + e0, left);
+    Codec::finish(acc, c);
+    if constexpr (ADD) {
+      float pv[32];
+      TileIO<T, false>::load(dst, L.count, e0, fast, stage, pv);
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] += pv[i];
+    }
+    TileIO<T, false>::storeTile(dst + e0, left, fast, stage, acc);
+  };
+  const long lane = (long)threadIdx.x * kElemsPerThread;
+  if constexpr (HasDirectSums<Codec>::value) {
+    typename Codec::Ahead r = Codec::ahead(enc, L, c, t0 * kTileElems + lane);
+    for (long t = t0; t < t1; ++t) {
+      float acc[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+      Codec::addAhead(r, c, Codec::finishScale(c), acc);
+      if (t + 1 < t1) r = Codec::ahead(enc, L, c, (t + 1) * kTileElems + lane);
+      put(t, acc);
+    }
+  } else {
+    for (long t = t0; t < t1; ++t) {
+      float acc[32];
+#pragma unroll
+      for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+      decodeSum<Codec>(enc, 0, 1, L, c, t * kTileElems + lane, Codec::finishScale(c), acc, sm, aligned);
+      put(t, acc);
+    }
+  }
+}
+
+// What a collective does after its encoded chunks have arrived; one kernel each, so that none carries another's code and registers.
+enum CollForm : int { kFormGather = 0, kFormGatherDelta = 1, kFormReduce = 2, kFormTwoShot = 3 };
+inline CollForm collForm(int op) {
+  switch (op) {
+    case kOpReduceScatter: case kOpAllReduceOneShot: return kFormReduce;
+    case kOpAllReduceTwoShot: return kFormTwoShot;
+    case kOpAllGatherDelta: return kFormGatherDelta;
+    default: return kFormGather;
+  }
+}
+
+template <typename T, class Codec, int FORM>
 __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollectiveKernel(const __grid_constant__ CollArgs a) {
-  __shared__ TileStage<T> stage;
+  __shared__ TileStage<T> stage[FORM == kFormGatherDelta ? 1 : kEncodeStages<T, Codec>];
   __shared__ float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
   __syncthreads();
@@ -170,10 +244,10 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollecti
         const int p = peer(it);   // perPeer only
         const long t0 = (long)s * a.sliceTiles;
         const long t1 = min(tiles, t0 + (long)a.sliceTiles);
-        encodeTiles<T, Codec>(perPeer ? in + (long)p * a.count : in, L, c, t0, t1, nDst,
+        encodeTiles<T, Codec, FORM == kFormGatherDelta>(perPeer ? in + (long)p * a.count : in, L, c, t0, t1, nDst,
                               [&](int d) { return a.ws[perPeer ? p : peerAt(d)] + (long)rank * a.slotBytes; }, stage, sm,
                               (uint64_t)(perPeer ? rank * N + p : rank) << 40,
-                              a.op == kOpAllGatherDelta ? out + (long)rank * a.count : nullptr);
+                              out + (long)rank * a.count);
       }
       publish(nb * nDst, [&](int i) {
         const int it = it0 + i / nDst * (int)gridDim.x;
@@ -184,7 +258,9 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollecti
 
   tracePhase(tr, 1);
   // ---------------- phase 2: wait + decode ----------------
-  const bool reduce = (a.op == kOpReduceScatter || a.op == kOpAllReduceOneShot || a.op == kOpAllReduceTwoShot);
+  constexpr bool reduce = FORM == kFormReduce || FORM == kFormTwoShot;
+  // the slots are laid out on 16 bytes unless a caller's geometry says otherwise
+  const bool aligned = ((reinterpret_cast<uintptr_t>(myWs) | (uintptr_t)a.slotBytes | (uintptr_t)a.regionBOffset) & 15u) == 0;
   {
     const int items = reduce ? slices : slices * N;
     const int nq = reduce ? N : 1, B = batchOf(items);
@@ -203,41 +279,37 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollecti
         const int q0 = qs.x;
         const long t0 = (long)qs.y * a.sliceTiles;
         const long t1 = min(tiles, t0 + (long)a.sliceTiles);
-        T* dstChunk = reduce ? out : out + (long)q0 * a.count;
+        if constexpr (!reduce) {
+          decodeTiles<T, Codec, FORM == kFormGatherDelta>(myWs + (long)q0 * a.slotBytes, out + (long)q0 * a.count, L, c, t0, t1, aligned,
+                                                          stage[0], sm);
+          continue;
+        }
         for (long t = t0; t < t1; ++t) {
-          const long e0 = t * kTileElems;
+          const long e0 = t * kTileElems, left = L.count - e0;
           const long e = e0 + (long)threadIdx.x * kElemsPerThread;
           float acc[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-          decodeSum<Codec>(myWs + (long)q0 * a.slotBytes, a.slotBytes, nq, L, c, e,
-                           a.op == kOpAllReduceTwoShot ? 1.f : Codec::finishScale(c), acc, sm);
-          if (a.op == kOpAllReduceTwoShot) {
+          decodeSum<Codec>(myWs, a.slotBytes, N, L, c, e, FORM == kFormTwoShot ? 1.f : Codec::finishScale(c), acc, sm, aligned);
+          if constexpr (FORM == kFormTwoShot) {
             // stay in the rotated domain: the sum of rotated values is the rotation of the sum
             const typename Codec::Enc enc = Codec::encode(acc, c, false, sm, ((uint64_t)(0x80 + rank) << 40) + (uint64_t)e);
             if (COCCL_CHUNK_RANGE_OK(Codec, L, c, e, 3))
               for (int d = 0; d < N; ++d) Codec::store(enc, a.ws[peerAt(d)] + a.regionBOffset + (long)rank * a.slotBytes, L, c, e);
           } else {
             Codec::finish(acc, c);
-            const bool fast = TileIO<T>::fastTile(dstChunk, L.count, e0);
-            if (a.op == kOpAllGatherDelta) {
-              float pv[32];
-              TileIO<T>::load(dstChunk, L.count, e0, fast, stage, pv);
-#pragma unroll
-              for (int i = 0; i < 32; ++i) acc[i] += pv[i];
-            }
-            TileIO<T>::store(dstChunk, L.count, e0, fast, stage, acc);
+            TileIO<T, false>::storeTile(out + e0, left, TileIO<T, false>::fast(out + e0, left), stage[0], acc);
           }
         }
       }
-      if (a.op == kOpAllReduceTwoShot)
+      if (FORM == kFormTwoShot)
         publish(nb * N, [&](int i) { return flagPtr(a.flags[peerAt(i % N)], 1, rank, it0 + i / N * (int)gridDim.x); }, a.epoch);
     }
   }
 
   tracePhase(tr, 2);
   // ---------------- phase 3 (two-shot all-reduce): gather reduced chunks ----------------
-  if (a.op == kOpAllReduceTwoShot) {
+  if constexpr (FORM == kFormTwoShot) {
     const int items = slices * N;
     const int B = batchOf(items);
     for (int it0 = blockIdx.x; it0 < items; it0 += B * (int)gridDim.x) {
@@ -253,17 +325,8 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollecti
         const int2 qs = from(j);
         const long t0 = (long)qs.y * a.sliceTiles;
         const long t1 = min(tiles, t0 + (long)a.sliceTiles);
-        T* dstChunk = out + (long)qs.x * a.count;
-        for (long t = t0; t < t1; ++t) {
-          const long e0 = t * kTileElems;
-          const long e = e0 + (long)threadIdx.x * kElemsPerThread;
-          float acc[32];
-#pragma unroll
-          for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-          decodeSum<Codec>(myWs + a.regionBOffset + (long)qs.x * a.slotBytes, 0, 1, L, c, e, Codec::finishScale(c), acc, sm);
-          Codec::finish(acc, c);
-          TileIO<T>::store(dstChunk, L.count, e0, TileIO<T>::fastTile(dstChunk, L.count, e0), stage, acc);
-        }
+        decodeTiles<T, Codec, false>(myWs + a.regionBOffset + (long)qs.x * a.slotBytes, out + (long)qs.x * a.count, L, c, t0, t1, aligned,
+                                     stage[0], sm);
       }
     }
   }
@@ -292,34 +355,72 @@ struct CodecArgs {
 // with stochastic rounding 68.6 -> 54.6 us (290 MB: 44 us to copy), decode + sum 30.6 -> 26.4 us; chunks of 5,000,003 bf16
 // elements (misaligned: see tile_io.cuh) 74.4 -> 30.0 us.
 //
-// The tiles of all chunks in order, `gridDim.x` apart: (chunk, tile) advances by a fixed step with one carry, because a 64-bit
-// division per tile and thread was a fifth of the instructions of these kernels.
+// whether every encoded input chunk starts on 16 bytes
+__device__ __forceinline__ bool encodedAligned(const CodecArgs& a) {
+  return ((reinterpret_cast<uintptr_t>(a.in) | (uintptr_t)a.encStrideIn) & 15u) == 0;
+}
+
+// The tiles of all chunks in order, `gridDim.x` apart: (chunk, tile) and every address that belongs to it advance by fixed
+// steps with one carry, because a 64-bit division per tile and thread was a fifth of the instructions of these kernels.
 struct TileWalk {
-  long tiles, chunks, ch, t, stepCh, stepT;
-  __device__ __forceinline__ TileWalk(long count, long chunks_) : chunks(chunks_) {
-    tiles = (count + kTileElems - 1) / kTileElems;
-    const unsigned n = (unsigned)tiles;   // 2^32 tiles would be 2^45 elements
-    ch = blockIdx.x / n; t = blockIdx.x % n; stepCh = gridDim.x / n; stepT = gridDim.x % n;
+  unsigned tiles, t, stepT;   // 2^32 tiles would be 2^45 elements
+  long chunks, ch, stepCh;
+  bool carried;               // whether the last step began another chunk
+  __device__ __forceinline__ TileWalk(long count, long chunks_) : chunks(chunks_), carried(false) {
+    tiles = (unsigned)((count + kTileElems - 1) / kTileElems);
+    ch = blockIdx.x / tiles; t = blockIdx.x % tiles; stepCh = gridDim.x / tiles; stepT = gridDim.x % tiles;
   }
   __device__ __forceinline__ bool more() const { return ch < chunks; }
   __device__ __forceinline__ void next() {
-    ch += stepCh;
-    t += stepT;
-    if (t >= tiles) { t -= tiles; ++ch; }
+    const unsigned rest = tiles - t;   // the sum itself may pass 2^32
+    carried = stepT >= rest;
+    ch += stepCh + (carried ? 1 : 0);
+    t = carried ? stepT - rest : t + stepT;
   }
+};
+// An address that grows by `pitch` with the chunk and by `tileElems` with the tile.
+template <class P>
+struct Along {
+  P* p;
+  long step, carry;
+  __device__ __forceinline__ Along(P* base, long pitch, long tileElems, const TileWalk& w)
+      : p(base + w.ch * pitch + w.t * tileElems), step(w.stepCh * pitch + w.stepT * tileElems), carry(pitch - (long)w.tiles * tileElems) {}
+  __device__ __forceinline__ void next(const TileWalk& w) { p += w.carried ? step + carry : step; }
 };
 
 template <typename T, class Codec>
 __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKernel(const CodecArgs a) {
-  __shared__ TileStage<T> stage;
+  constexpr int S = kEncodeStages<T, Codec>;
+  __shared__ TileStage<T> stage[S];
   __shared__ float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
   __syncthreads();
   const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);
-  for (TileWalk w(a.count, a.chunks); w.more(); w.next()) {
-    encodeTiles<T, Codec>(reinterpret_cast<const T*>(a.in) + w.ch * a.rawPitch, L, a.codec, w.t, w.t + 1, 1,
-                          [&](int) { return reinterpret_cast<uint8_t*>(a.out) + w.ch * a.encStrideOut; }, stage, sm,
-                          (uint64_t)w.ch << 40);
+  TileWalk w(a.count, a.chunks);
+  Along<const T> src(reinterpret_cast<const T*>(a.in), a.rawPitch, kTileElems, w);
+  Along<uint8_t> dst(reinterpret_cast<uint8_t*>(a.out), a.encStrideOut, 0, w);
+  auto start = [&](int s) {
+    const long left = L.count - (long)w.t * kTileElems;
+    if (w.more()) TileIO<T>::template bring<S == 2>(src.p, left, w.t == 0, TileIO<T>::fast(src.p, left), stage[s]);
+    if (S == 2) commitCopies();
+  };
+  if (S == 2) start(0);
+  for (int s = 0; w.more(); s ^= S - 1) {
+    const T* tile = src.p;
+    uint8_t* out = dst.p;
+    const long e0 = (long)w.t * kTileElems, left = L.count - e0, ch = w.ch;
+    __syncwarp();   // the stage that is filled next has been read
+    if (S == 1) start(0);
+    w.next();
+    src.next(w);
+    dst.next(w);
+    if (S == 2) start(s ^ 1);
+    if (S == 2) waitCopies<1>();
+    float v[32];
+    TileIO<T>::take(tile, left, e0 == 0, TileIO<T>::fast(tile, left), stage[s], v);
+    const long e = e0 + (long)threadIdx.x * kElemsPerThread;
+    const typename Codec::Enc enc = Codec::encode(v, a.codec, true, sm, ((uint64_t)ch << 40) + (uint64_t)e);
+    if (COCCL_CHUNK_RANGE_OK(Codec, L, a.codec, e, 1)) Codec::store(enc, out, L, a.codec, e);
   }
 }
 
@@ -331,18 +432,42 @@ __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const
   Codec::initShared(sm);
   __syncthreads();
   const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);
-  const uint8_t* enc = reinterpret_cast<const uint8_t*>(a.in);
-  for (TileWalk w(a.count, a.chunks); w.more(); w.next()) {
-    T* dst = reinterpret_cast<T*>(a.out) + w.ch * a.rawPitch;
-    const long e0 = w.t * kTileElems;
+  TileWalk w(a.count, a.chunks);
+  Along<const uint8_t> src(reinterpret_cast<const uint8_t*>(a.in), a.encStrideIn, 0, w);
+  Along<T> dst(reinterpret_cast<T*>(a.out), a.rawPitch, kTileElems, w);
+  if constexpr (HasDirectSums<Codec>::value) {
+    // One copy (all-gather, all-to-all): the next tile's words are loaded before this one is transformed and stored (4 bits,
+    // groups of 128, rotated: 8 x 8 Mi bf16 40.3 -> 33.0 us, 8 x 5,000,003 29.4 -> 23.9 us).
+    if (a.reduce == 1) {
+      auto fetch = [&] { return Codec::ahead(src.p, L, a.codec, (long)w.t * kTileElems + (long)threadIdx.x * kElemsPerThread); };
+      typename Codec::Ahead r;
+      if (w.more()) r = fetch();
+      while (w.more()) {
+        T* tile = dst.p;
+        const long left = L.count - (long)w.t * kTileElems;
+        float acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+        Codec::addAhead(r, a.codec, Codec::finishScale(a.codec), acc);
+        w.next();
+        src.next(w);
+        dst.next(w);
+        if (w.more()) r = fetch();
+        Codec::finish(acc, a.codec);
+        TileIO<T>::storeTile(tile, left, TileIO<T>::fast(tile, left), stage, acc);
+      }
+      return;
+    }
+  }
+  for (; w.more(); w.next(), src.next(w), dst.next(w)) {
+    const long e0 = (long)w.t * kTileElems, left = L.count - e0;
     const long e = e0 + (long)threadIdx.x * kElemsPerThread;
     float acc[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-    decodeSum<Codec>(enc + w.ch * a.encStrideIn, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e,
-                     Codec::finishScale(a.codec), acc, sm);
+    decodeSum<Codec>(src.p, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, Codec::finishScale(a.codec), acc, sm, encodedAligned(a));
     Codec::finish(acc, a.codec);
-    TileIO<T>::store(dst, L.count, e0, TileIO<T>::fastTile(dst, L.count, e0), stage, acc);
+    TileIO<T>::storeTile(dst.p, left, TileIO<T>::fast(dst.p, left), stage, acc);
   }
 }
 
@@ -354,15 +479,17 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) decodeReduceE
   Codec::initShared(sm);
   __syncthreads();
   const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);
-  const uint8_t* enc = reinterpret_cast<const uint8_t*>(a.in);
-  for (TileWalk w(a.count, a.chunks); w.more(); w.next()) {
-    const long e = w.t * kTileElems + (long)threadIdx.x * kElemsPerThread;
+  TileWalk w(a.count, a.chunks);
+  Along<const uint8_t> src(reinterpret_cast<const uint8_t*>(a.in), a.encStrideIn, 0, w);
+  Along<uint8_t> dst(reinterpret_cast<uint8_t*>(a.out), a.encStrideOut, 0, w);
+  for (; w.more(); w.next(), src.next(w), dst.next(w)) {
+    const long e = (long)w.t * kTileElems + (long)threadIdx.x * kElemsPerThread;
     float acc[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-    decodeSum<Codec>(enc + w.ch * a.encStrideIn, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, 1.f, acc, sm);
+    decodeSum<Codec>(src.p, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, 1.f, acc, sm, encodedAligned(a));
     const typename Codec::Enc o = Codec::encode(acc, a.codec, false, sm, ((uint64_t)(0x40 + w.ch) << 40) + (uint64_t)e);
-    Codec::store(o, reinterpret_cast<uint8_t*>(a.out) + w.ch * a.encStrideOut, L, a.codec, e);
+    Codec::store(o, dst.p, L, a.codec, e);
   }
 }
 

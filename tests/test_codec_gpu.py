@@ -206,3 +206,69 @@ def test_sums_on_both_sides_of_the_rounds_of_tiles(cuda, cfg, tiles):
     got = C.decode_reduce(enc, cfg, count, torch.float32, 1, 3)[0].double()
     size = one.abs().sum(0).amax()
     assert ((got - one.sum(0)).abs() <= 64 * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("offset", [0, 4, 8])
+@pytest.mark.parametrize("cfg,dtype", [(C.SDP4BIT_G128, torch.float32), (C.SDP4BIT_G128, torch.bfloat16),
+                                       (C.CodecConfig("sdp4bit", 4, 32, True, False), torch.float16),
+                                       (C.CodecConfig("sdp4bit", 8, 128, False, True), torch.bfloat16),
+                                       (C.CodecConfig("sdp4bit", 8, 64, True, True), torch.float32)],
+                         ids=lambda v: f"{v.kind}{v.bits}g{v.group}{'a' if v.asym else 's'}" if isinstance(v, C.CodecConfig) else str(v)[6:])
+@pytest.mark.parametrize("groups", [1, 3, 66])
+def test_sums_at_every_alignment_and_number_of_copies(cuda, cfg, dtype, groups, offset):
+    """Encoded copies that start on any word (the distance between them a multiple of 4, 8 or 16 bytes by the number of
+    groups), 1 to 9 of them: the sum of what each decodes to on its own, to the rounding of fp32 sums (and of the output)."""
+    torch.manual_seed(groups)
+    count = groups * cfg.group - 5
+    x = (torch.randn(9 * count, device=cuda)).to(dtype)
+    enc = C.encode(x, cfg, 9)
+    nb = enc.shape[1]
+    room = torch.empty(9 * nb + 16, dtype=torch.uint8, device=cuda)
+    room[offset:offset + 9 * nb] = enc.reshape(-1)
+    one = C.decode(enc, cfg, count, torch.float32, 9) if cfg.param_bytes(dtype) == cfg.param_bytes(torch.float32) else None
+    for n in range(1, 10):
+        got = torch.full((count,), float("nan"), dtype=dtype, device=cuda)
+        _lib.check(_lib.lib().cocclkDecodeReduce(room.data_ptr() + offset, got.data_ptr(), count, 1, n, count, nb, C.DTYPE_CODE[dtype],
+                                                 cfg.to_c(dtype), _lib.cur_stream()), "cocclkDecodeReduce")
+        each = [C.decode(enc[i:i + 1].clone(), cfg, count, dtype, 1)[0].double() for i in range(n)]
+        want, size = sum(each), sum(e.abs() for e in each).amax()
+        ulp = torch.finfo(dtype).eps
+        assert ((got.double() - want).abs() <= (n + 1) * max(ulp, 64 * 2.0 ** -24) * size).all()
+        if one is not None:
+            assert ((got.double() - one[:n].double().sum(0)).abs() <= max(ulp, 64 * 2.0 ** -24) * size).all()
+
+
+@pytest.mark.parametrize("cfg", [C.SDP4BIT_G128, C.CodecConfig("sdp4bit", 4, 128, False, True, True), C.CodecConfig("sdp4bit", 4, 16, False, False),
+                                 C.MXFP8, C.TACO_G128, C.ZFP_RATE8], ids=lambda c: f"{c.kind}g{c.group}{'r' if c.stochastic else ''}")
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("count", [8192 * 7 + 3, 8192 * 7, 41])
+def test_several_tiles_a_cta_equal_one(cuda, cfg, dtype, count):
+    """More tiles than the GPU has places, so that a CTA's tiles follow one another through its stages and over the ends of chunks
+    (chunks of one tile: the walk steps over many chunks at once): the same bytes and values as a chunk on its own."""
+    torch.manual_seed(2)
+    chunks = 1900 if count < 8192 else 240
+    x = (torch.randn(chunks * count, device=cuda) * 0.01).to(dtype)
+    enc = C.encode(x, cfg, chunks)
+    dec = C.decode(enc, cfg, count, dtype, chunks)
+    for j in (0, 1, 83, 84, chunks // 2, chunks - 2, chunks - 1):
+        if cfg.stochastic and j:
+            continue   # the rounding stream is keyed by the chunk
+        one = C.encode(x[j * count:(j + 1) * count].clone(), cfg, 1)
+        assert torch.equal(enc[j], one[0]), j
+    for j in (0, 1, 83, 84, chunks // 2, chunks - 2, chunks - 1):
+        assert torch.equal(dec[j], C.decode(enc[j:j + 1].clone(), cfg, count, dtype, 1)[0]), j
+
+
+@pytest.mark.parametrize("asym", [False, True])
+def test_not_a_number_counts_in_no_maximum(cuda, asym):
+    """A group's largest (and smallest) value is that of its numbers: groups with a NaN at any place keep the parameters they have
+    with a zero there."""
+    cfg = C.CodecConfig("sdp4bit", 4, 32, asym, False)
+    x = torch.randn(32, 32, device=cuda)
+    at = torch.arange(32, device=cuda)
+    zero, nan = x.clone(), x.clone()
+    zero[at, at] = 0.0
+    nan[at, at] = float("nan")
+    a, b = (C.encode(v.reshape(-1), cfg, 1)[0] for v in (zero, nan))
+    payload = 32 * 16
+    assert torch.equal(a[payload:], b[payload:])
