@@ -97,6 +97,7 @@ _PROTOS = {
     # moe_api.h
     "cocclkMoeWorkspaceBytes": (c_long, [c_int, c_int, c_int, c_int]),
     "cocclkMoeLayout": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "cocclkMoeLayoutRanks": (c_int, [C.POINTER(MoeArgs), c_void_p]),
     "cocclkMoeDispatch": (c_int, [C.POINTER(MoeArgs), c_int, c_int, c_void_p]),
     "cocclkMoeCombine": (c_int, [C.POINTER(MoeArgs), c_int, c_int, c_void_p]),
     # launch_count.h

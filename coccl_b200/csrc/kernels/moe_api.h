@@ -51,6 +51,8 @@ long cocclkMoeWorkspaceBytes(int nRanks, int capacity, int hidden, int localExpe
 // expertIds [entries] -> pos [entries], counts [experts]; one CTA, deterministic. entries = tokens * topk.
 int cocclkMoeLayout(const int* expertIds, int entries, int experts, int expertsPerRank, int* pos, int* counts,
                     cudaStream_t stream);
+// The same for the ranks 0 .. nRanks - 1 of `args` (expertIds -> pos, sendCounts, both written), side by side in one launch.
+int cocclkMoeLayoutRanks(const cocclkMoeArgs* args, cudaStream_t stream);
 int cocclkMoeDispatch(const cocclkMoeArgs* args, int emulatedRanks, int maxCtas, cudaStream_t stream);
 int cocclkMoeCombine(const cocclkMoeArgs* args, int emulatedRanks, int maxCtas, cudaStream_t stream);
 

@@ -41,8 +41,15 @@ __host__ __device__ inline Layout makeLayout(int nRanks, int capacity, int hidde
 // ------------------------------------------------------------------ routing layout
 // Stable counting sort of the entries by expert: warp w owns a contiguous segment of entries; a first walk
 // builds per-warp histograms, a scan turns them into bases, a second walk hands out the positions.
-__global__ void __launch_bounds__(1024) moeLayoutKernel(const int* __restrict__ ids, int entries, int experts,
-                                                        int expertsPerRank, int* __restrict__ pos, int* __restrict__ counts) {
+struct LayoutArgs {   // one CTA for each of the ranks that play on this GPU
+  const int* ids[COCCLK_MOE_MAX_RANKS];
+  int* pos[COCCLK_MOE_MAX_RANKS];
+  int* counts[COCCLK_MOE_MAX_RANKS];
+};
+__global__ void __launch_bounds__(1024) moeLayoutKernel(const __grid_constant__ LayoutArgs a, int entries, int experts, int expertsPerRank) {
+  const int* __restrict__ ids = a.ids[blockIdx.x];
+  int* __restrict__ pos = a.pos[blockIdx.x];
+  int* __restrict__ counts = a.counts[blockIdx.x];
   __shared__ int hist[32][COCCLK_MOE_MAX_EXPERTS];  // becomes the running base of (warp, expert)
   __shared__ int expertBase[COCCLK_MOE_MAX_EXPERTS];
   // One CTA, so latency is all that counts: the first kCached strips of a warp's segment (8192 entries in all) are loaded
@@ -466,7 +473,28 @@ extern "C" long cocclkMoeWorkspaceBytes(int nRanks, int capacity, int hidden, in
 extern "C" int cocclkMoeLayout(const int* expertIds, int entries, int experts, int expertsPerRank, int* pos, int* counts,
                                cudaStream_t stream) {
   if (entries <= 0 || experts <= 0 || experts > COCCLK_MOE_MAX_EXPERTS || expertsPerRank <= 0 || experts % expertsPerRank) return -1;
-  moeLayoutKernel<<<1, 1024, 0, stream>>>(expertIds, entries, experts, expertsPerRank, pos, counts);
+  LayoutArgs l = {};
+  l.ids[0] = expertIds; l.pos[0] = pos; l.counts[0] = counts;
+  moeLayoutKernel<<<1, 1024, 0, stream>>>(l, entries, experts, expertsPerRank);
+  cocclkCountLaunches(1);
+  return (int)cudaGetLastError();
+}
+
+// The layouts of all emulated ranks side by side (four ranks of 4096 entries: one after the other 24 us of one-CTA kernels, 6 us in one
+// launch).
+extern "C" int cocclkMoeLayoutRanks(const cocclkMoeArgs* args, cudaStream_t stream) {
+  const cocclkMoeArgs& a = *args;
+  const long entries = (long)a.tokens * a.topk;
+  if (a.nRanks < 1 || a.nRanks > COCCLK_MOE_MAX_RANKS || entries <= 0 || entries > 0x7fffffffL || a.experts <= 0 ||
+      a.experts > COCCLK_MOE_MAX_EXPERTS || a.experts % a.nRanks)
+    return -1;
+  LayoutArgs l = {};
+  for (int r = 0; r < a.nRanks; ++r) {
+    l.ids[r] = a.expertIds[r];
+    l.pos[r] = const_cast<int*>(a.pos[r]);
+    l.counts[r] = const_cast<int*>(a.sendCounts[r]);
+  }
+  moeLayoutKernel<<<a.nRanks, 1024, 0, stream>>>(l, (int)entries, a.experts, a.experts / a.nRanks);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }

@@ -99,15 +99,18 @@ def emulate_dispatch(xs, ids, n_experts, *, capacity=None, state=None, max_ctas=
     a = _base_args(n, tokens, hidden, topk, n_experts, capacity, state, timeout_ms)
     keep, handles, recvs = [], [], []
     for r in range(n):
-        pos, counts = route_layout(ids[r], n_experts, n)
+        assert ids[r].dtype == torch.int32 and n_experts % n == 0
+        routed = ids[r].contiguous()
+        pos, counts = torch.empty_like(routed), torch.empty(n_experts, dtype=torch.int32, device=dev)
         recv = torch.empty(n * capacity, hidden, dtype=torch.bfloat16, device=dev)
         roff = torch.empty(le + 1, dtype=torch.int32, device=dev)   # both written in full by the kernel
         rcnt = torch.empty(n, le, dtype=torch.int32, device=dev)
-        a.x[r], a.expertIds[r], a.pos[r], a.sendCounts[r] = xs[r].data_ptr(), ids[r].data_ptr(), pos.data_ptr(), counts.data_ptr()
+        a.x[r], a.expertIds[r], a.pos[r], a.sendCounts[r] = xs[r].data_ptr(), routed.data_ptr(), pos.data_ptr(), counts.data_ptr()
         a.recv[r], a.recvOffsets[r], a.recvCounts[r] = recv.data_ptr(), roff.data_ptr(), rcnt.data_ptr()
-        keep.append((pos, counts))
+        keep.append((routed, pos, counts))
         recvs.append(recv)
-        handles.append(Handle(ids[r], pos, rcnt, roff, capacity, n_experts))
+        handles.append(Handle(routed, pos, rcnt, roff, capacity, n_experts))
+    _lib.check(_lib.lib().cocclkMoeLayoutRanks(a, _lib.cur_stream()), "cocclkMoeLayoutRanks")
     _lib.check(_lib.lib().cocclkMoeDispatch(a, n, max_ctas, _lib.cur_stream()), "cocclkMoeDispatch")
     return recvs, handles, state
 

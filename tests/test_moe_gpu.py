@@ -85,3 +85,17 @@ def test_route_layout_equals_the_host_restatement(cuda, tokens, topk, experts, r
     pos, counts = M.route_layout(ids.to(cuda), experts, ranks)
     want_pos, want_counts = M.route_layout(ids, experts, ranks)
     assert torch.equal(pos.cpu(), want_pos) and torch.equal(counts.cpu(), want_counts)
+
+
+@pytest.mark.parametrize("n,tokens,topk,experts", [(2, 1, 1, 8), (4, 33, 2, 16), (3, 5000, 2, 48), (8, 257, 8, 256)])
+def test_layouts_of_all_ranks_in_one_launch_equal_one_by_one(cuda, n, tokens, topk, experts):
+    torch.manual_seed(n)
+    xs = [torch.randn(tokens, 256, device=cuda).bfloat16() for _ in range(n)]
+    ids = [torch.rand(tokens, experts, device=cuda).topk(topk, 1).indices.int() for _ in range(n)]
+    _, handles, _ = M.emulate_dispatch(xs, ids, experts)
+    for r in range(n):
+        pos, counts = M.route_layout(ids[r], experts, n)
+        assert torch.equal(handles[r].pos, pos), r
+        le = experts // n
+        for d in range(n):   # what rank d received from r, by local expert
+            assert torch.equal(handles[d].recv_counts[r], counts[d * le:(d + 1) * le])
