@@ -4,7 +4,8 @@
 // A CTA of 256 threads owns a tile of 8192 consecutive elements of one chunk; every thread owns one
 // aligned run of 32 elements in registers (tile_io.cuh). A codec turns a run into an `Enc` (packed payload
 // words + the parameters of the groups that start in the run) that can be stored to any number of
-// destinations (local scratch or a peer's receive slot), and back.
+// destinations (local scratch or a peer's receive slot), and back. encode and finish get a 2 KiB window of shared memory for
+// each warp, which TACO needs; the caller has not used it since the last __syncwarp().
 //
 // Numerics follow the reference codecs:
 //  * SDP4Bit group quantisation: symmetric scale=(2^(b-1)-1)/absmax, stored parameter 1/scale, clamp to
@@ -125,10 +126,7 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 
 // Unnormalised 32-point Walsh-Hadamard transform of one run, entirely in registers: the first stage inside the pairs, the
 // other four on pairs.
-__device__ __forceinline__ void hadamard32(float (&v)[32]) {
-  uint64_t p[16];
-#pragma unroll
-  for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i] + v[2 * i + 1], v[2 * i] - v[2 * i + 1]);
+__device__ __forceinline__ void hadamardPairs(uint64_t (&p)[16]) {   // the four stages on pairs
 #pragma unroll
   for (int s = 1; s < 16; s <<= 1) {
 #pragma unroll
@@ -140,6 +138,12 @@ __device__ __forceinline__ void hadamard32(float (&v)[32]) {
       }
     }
   }
+}
+__device__ __forceinline__ void hadamard32(float (&v)[32]) {
+  uint64_t p[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) p[i] = pack2(v[2 * i] + v[2 * i + 1], v[2 * i] - v[2 * i + 1]);
+  hadamardPairs(p);
 #pragma unroll
   for (int i = 0; i < 16; ++i) unpack2(p[i], v[2 * i], v[2 * i + 1]);
 }
@@ -205,7 +209,7 @@ __device__ __forceinline__ uint64_t rngCentered2(uint32_t word, int k) {
 // number of groups), else words.
 template <int N>
 __device__ __forceinline__ void storeWords(uint8_t* p, const uint32_t (&w)[N]) {
-  if (aligned16(p)) {
+  if (N >= 4 && aligned16(p)) {
 #pragma unroll
     for (int q = 0; q < N / 4; ++q) reinterpret_cast<uint4*>(p)[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
   } else if ((reinterpret_cast<uintptr_t>(p) & 7u) == 0) {
@@ -219,7 +223,7 @@ __device__ __forceinline__ void storeWords(uint8_t* p, const uint32_t (&w)[N]) {
 // __ldcg: the bytes may have been written by a peer GPU during this launch
 template <int N>
 __device__ __forceinline__ void loadWords(const uint8_t* p, uint32_t (&w)[N]) {
-  if (aligned16(p)) {
+  if (N >= 4 && aligned16(p)) {
 #pragma unroll
     for (int q = 0; q < N / 4; ++q) {
       const uint4 t = __ldcg(reinterpret_cast<const uint4*>(p) + q);
@@ -252,10 +256,22 @@ __device__ __forceinline__ void loadWordsBy(const uint8_t* p, uint32_t (&w)[N]) 
       const uint2 t = __ldcg(reinterpret_cast<const uint2*>(p) + q);
       w[2 * q] = t.x; w[2 * q + 1] = t.y;
     }
+  } else if constexpr (N > 4) {
+    loadWords(p, w);   // copies at different distances: some are better aligned
   } else {
-    loadWords(p, w);
+#pragma unroll
+    for (int k = 0; k < N; ++k) w[k] = __ldcg(reinterpret_cast<const uint32_t*>(p) + k);
   }
 }
+
+// Where a thread's run lies in an encoded chunk: the tile's addresses, the same in all threads, and the thread's distances from them.
+struct RunAddress {
+  const uint8_t *tileWords, *tileParams;
+  unsigned word, param;
+  __device__ __forceinline__ const uint8_t* words() const { return tileWords + word; }
+  __device__ __forceinline__ const uint8_t* params() const { return tileParams + param; }
+  __device__ __forceinline__ void next(long stride) { tileWords += stride; tileParams += stride; }   // the next copy
+};
 
 // ------------------------------------------------------------------ SDP4Bit
 // SMALLG: groups of 8 or 16 elements (several per run, no rotation); otherwise group >= 32.
@@ -273,6 +289,7 @@ struct SdpCodec {
   // against 20.3; 4 bits, groups of 8: 29.5 (three) and 31.2 (four), 26.1 and 23.1; 8 bits, asymmetric groups of 8, whose
   // parameters do not fit 80 registers beside a run: 35.6 (three) and 39.8 (four), 28.9 (two) and 32.8 (three).
   static constexpr int kEncodeBlocks = SMALLG ? 3 : 4, kDecodeBlocks = BITS == 8 && SMALLG && ASYM ? 2 : 3, kSumBlocks = 2;
+  static constexpr bool kExchanges = false;   // runs of neighbouring lanes through the window
   static constexpr bool kEncodeAhead = !(SMALLG && BITS == 8);   // collective_kernels.cuh
   static constexpr int kSmemFloats = 8; // shared scratch every kernel passes as `sm` (group reductions wider than a warp)
   static __device__ __forceinline__ void initShared(float*) {}
@@ -345,7 +362,7 @@ struct SdpCodec {
   // v: the run of this thread (zero beyond the chunk). `rotate=false` when v is already in the rotated
   // domain. rngElem = message-wide element index of v[0] (keys the rounding RNG).
   static __device__ __forceinline__ Enc encode(float (&v)[32], const CodecCfg& c, bool rotate, float* sm,
-                                               uint64_t rngElem) {
+                                               uint64_t rngElem, uint4* /*win*/ = nullptr) {
     if (HAD && rotate) hadamard32(v);
     Enc e;
     float scale[kParams], offset[kParams];
@@ -590,7 +607,7 @@ struct SdpCodec {
     return elem < (L.groups << gs);
   }
   static __device__ __forceinline__ void sum(const uint8_t* base, long stride, int n, const ChunkLayout& L, const CodecCfg& c, long elem,
-                                             float mul, bool aligned, float (&acc)[32]) {
+                                             float mul, bool aligned, bool /*spread*/, float (&acc)[32]) {
     const uint8_t *pw, *pp;
     if (!runAt(base, L, c, elem, pw, pp)) return;
     const uint32_t magic = opaqueMagic(c);
@@ -620,7 +637,7 @@ struct SdpCodec {
   // Leave the rotated domain (after any reduction: the transform is linear). The 1/32 of the inverse
   // transform was applied by fetch (kFinishScale).
   static __device__ __forceinline__ float finishScale(const CodecCfg&) { return HAD ? 1.f / 32.f : 1.f; }
-  static __device__ __forceinline__ void finish(float (&v)[32], const CodecCfg&) {
+  static __device__ __forceinline__ void finish(float (&v)[32], const CodecCfg&, uint4* /*win*/ = nullptr) {
     if (HAD) hadamard32(v);
   }
 };
@@ -634,6 +651,7 @@ struct MxFp8Codec {
   static constexpr int kMinBlocks = 3;
   // 4 x 16 Mi bf16: decode 42.8 us with four, 35.7 with three; 8 x 4 Mi encode 15.7 us with three, 14.6 with four
   static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3, kSumBlocks = 2;
+  static constexpr bool kExchanges = false;
   static constexpr bool kEncodeAhead = false;
   static constexpr int kSmemFloats = 8;
   static __device__ __forceinline__ void initShared(float*) {}
@@ -644,7 +662,7 @@ struct MxFp8Codec {
   };
 
   static __device__ __forceinline__ Enc encode(float (&v)[32], const CodecCfg& /*c*/, bool /*rotate*/, float* /*sm*/,
-                                               uint64_t /*rngElem*/) {
+                                               uint64_t /*rngElem*/, uint4* /*win*/ = nullptr) {
     float m = 0.f;
 #pragma unroll
     for (int i = 0; i < 32; ++i) m = fmaxf(m, fabsf(v[i]));
@@ -722,16 +740,15 @@ struct MxFp8Codec {
 
   static constexpr bool kDirectSums = true;
   template <int ALIGN, int B>
-  static __device__ __forceinline__ void sumBatches(const uint8_t*& pw, const uint8_t*& ps, long stride, int& n, float (&acc)[32]) {
+  static __device__ __forceinline__ void sumBatches(RunAddress& r, long stride, int& n, float (&acc)[32]) {
 #pragma unroll 1
     while (n >= B) {
       uint32_t w[B][8], biased[B];
 #pragma unroll
       for (int j = 0; j < B; ++j) {
-        loadWordsBy<ALIGN>(pw, w[j]);
-        biased[j] = __ldcg(ps);
-        pw += stride;
-        ps += stride;
+        loadWordsBy<ALIGN>(r.words(), w[j]);
+        biased[j] = __ldcg(r.params());
+        r.next(stride);
       }
 #pragma unroll
       for (int j = 0; j < B; ++j) addRun(w[j], biased[j], acc);
@@ -739,15 +756,16 @@ struct MxFp8Codec {
     }
   }
   static __device__ __forceinline__ void sum(const uint8_t* base, long stride, int n, const ChunkLayout& L, const CodecCfg& /*c*/, long elem,
-                                             float /*mul*/, bool aligned, float (&acc)[32]) {
+                                             float /*mul*/, bool aligned, bool /*spread*/, float (&acc)[32]) {
     if (elem >= L.groups * 32) return;
-    const uint8_t *pw = base + elem, *ps = base + L.payloadBytes + elem / 32;
+    const long e0 = elem - (long)threadIdx.x * kElemsPerThread;
+    RunAddress r = {base + e0, base + L.payloadBytes + e0 / 32, threadIdx.x * 32u, threadIdx.x};
     if (aligned) {
-      sumBatches<16, 2>(pw, ps, stride, n, acc);
-      sumBatches<16, 1>(pw, ps, stride, n, acc);
+      sumBatches<16, 2>(r, stride, n, acc);
+      sumBatches<16, 1>(r, stride, n, acc);
     } else {
-      sumBatches<4, 2>(pw, ps, stride, n, acc);
-      sumBatches<4, 1>(pw, ps, stride, n, acc);
+      sumBatches<4, 2>(r, stride, n, acc);
+      sumBatches<4, 1>(r, stride, n, acc);
     }
   }
   // One copy, its loads apart from its use (behind the chunk: zeros).
@@ -764,7 +782,7 @@ struct MxFp8Codec {
   static __device__ __forceinline__ void addAhead(const Ahead& r, const CodecCfg& /*c*/, float /*mul*/, float (&acc)[32]) { addRun(r.w, r.biased, acc); }
 
   static __device__ __forceinline__ float finishScale(const CodecCfg&) { return 1.f; }
-  static __device__ __forceinline__ void finish(float (&)[32], const CodecCfg&) {}
+  static __device__ __forceinline__ void finish(float (&)[32], const CodecCfg&, uint4* /*win*/ = nullptr) {}
 };
 
 // ------------------------------------------------------------------ TACO
@@ -772,33 +790,89 @@ struct MxFp8Codec {
 //   ada = clamp(fp8max * rsqrt(mean(x^2) + lambda), 1e-3, 1e3);  y = H_G(x * ada) / sqrt(G);
 //   qs = clamp(max|y| / targetRange, 1e-12, 1e6);  code = fp8(clamp(y / qs, +-448));  x^ = H_G(code * qs) / sqrt(G) / ada
 // Chunk layout as the reference's: [one fp8 byte per value of every (padded) group][groups x f32 qs][groups x f32 ada].
-// A group is G/32 consecutive runs, i.e. G/32 adjacent lanes of one warp: the first five butterfly stages are
-// register work, the rest and the group statistics are warp shuffles, so every lane of the warp must call
-// encode() and finish() together. "Rotated domain" here is y / ada = H_G(x) / sqrt(G): independent of the
-// sender's ada, so copies from different ranks add up there and one inverse transform serves the sum; the
-// transform is orthonormal, so mean(x^2) for a re-encode is available without leaving the domain.
+// A group is G/32 consecutive runs, i.e. G/32 adjacent lanes of one warp: the first five butterfly stages are register work.
+// For the next two, E = min(4, G/32) lanes exchange their runs through shared memory, so that each holds the same 32/E places
+// of E runs (the "spread" ownership) and finds its partners in its own registers: 16 vector accesses instead of 64 shuffles
+// and as many multiply-adds, and what follows (maxima, FP8, stores) is as easy there. Wider groups use shuffles for the rest.
+// Groups of 128, 8 x 8 Mi fp16: encode 65.3 -> 51.3 us, sum 21.8 -> 19.4 us, re-encoding sum 24.3 -> 15.7 us; 8 x 3,000,008:
+// encode 26.0 -> 21.4 us. (Groups of 64 with their one stage by shuffles: sum of 8 x 3,000,008 12.3 us, 9.2 with the exchange.)
+// The group statistics are warp shuffles, so every lane of the warp must call encode() and finish() together. "Rotated domain"
+// here is y / ada = H_G(x) / sqrt(G): independent of the sender's ada, so copies from different ranks add up there and one
+// inverse transform serves the sum; the transform is orthonormal, so mean(x^2) for a re-encode is available without leaving the
+// domain (in the order of the run ownership, in which a re-encoding sum is therefore formed).
 struct TacoCodec {
   static constexpr int kBits = 8;
   static constexpr int kWords = 8;
   static constexpr bool kRotated = true;
-  // stand-alone kernels: 61 and 79 registers, 8 x 3,000,008 fp16 encode 28.3 -> 25.5 us, decode + sum 13.2 -> 10.5 us against
-  // one CTA fewer (367 tiles then fit the GPU at once)
   static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3, kSumBlocks = 2;
-  static constexpr int kMinBlocks = 2;  // the lane butterflies keep two copies of a run live: 128 registers, no spills
-  static constexpr bool kEncodeAhead = false;
+  static constexpr int kMinBlocks = 3;
+  static constexpr bool kExchanges = true;
+  static constexpr bool kEncodeAhead = true;
   static constexpr int kSmemFloats = 8;
   static __device__ __forceinline__ void initShared(float*) {}
 
   struct Enc {
     uint32_t w[8];
     float qs, ada;
+    bool spread;
   };
   static __device__ __forceinline__ int groupShift(const CodecCfg& c) { return 31 - __clz(c.group); }  // a power of two
+  template <class F>
+  static __device__ __forceinline__ void byLanes(const CodecCfg& c, F&& f) {   // f(integral_constant<E>)
+    if (c.group >= 128) f(std::integral_constant<int, 4>{});
+    else if (c.group == 64) f(std::integral_constant<int, 2>{});
+    else f(std::integral_constant<int, 1>{});
+  }
 
+  // Vector a (of four) of run r in the warp's 2 KiB window: neither the lanes that write their runs nor those that read one
+  // place of several runs meet in a bank.
+  static __device__ __forceinline__ int at(int r, int a) { return ((r ^ ((r >> 2) & 1)) << 2) + (a ^ ((r >> 1) & 3)); }
+  // Run ownership -> spread (SPREAD) or back. Vector q of a run goes with pass q & 1; lane j of E owns the vectors j * 8 / E on.
+  template <int E, bool SPREAD>
+  static __device__ __forceinline__ void exchange(float (&v)[32], uint4* win) {
+    const int lane = threadIdx.x & 31, j = lane & (E - 1);
+    float o[32];
+    auto own = [](int p, int i) { return 4 * (2 * i + p); };
+    auto theirs = [](int p, int i) { return (i / (4 / E)) * (32 / E) + 4 * (2 * (i % (4 / E)) + p); };
+    auto slotOf = [&](bool spread, int i) { return spread ? at(lane - j + i / (4 / E), j * (4 / E) + i % (4 / E)) : at(lane, i); };
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = SPREAD ? own(p, i) : theirs(p, i);
+        win[slotOf(!SPREAD, i)] = make_uint4(__float_as_uint(v[k]), __float_as_uint(v[k + 1]), __float_as_uint(v[k + 2]), __float_as_uint(v[k + 3]));
+      }
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = SPREAD ? theirs(p, i) : own(p, i);
+        const uint4 y = win[slotOf(SPREAD, i)];
+        o[k] = __uint_as_float(y.x); o[k + 1] = __uint_as_float(y.y); o[k + 2] = __uint_as_float(y.z); o[k + 3] = __uint_as_float(y.w);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = o[i];
+  }
+  // The butterfly stages across lanes, in the spread ownership.
+  template <int E>
   static __device__ __forceinline__ void lanes(float (&v)[32], int lpg) {
-    const int lane = threadIdx.x & 31;
-    for (int s = 1; s < lpg; s <<= 1) {
-      const float sign = (lane & s) != 0 ? -1.f : 1.f;
+#pragma unroll
+    for (int s = 1; s < E; s <<= 1) {
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        if (r & s) continue;
+#pragma unroll
+        for (int k = 0; k < 32 / E; k += 2) {
+          const int lo = r * (32 / E) + k, hi = (r | s) * (32 / E) + k;
+          const uint64_t a = pack2(v[lo], v[lo + 1]), b = pack2(v[hi], v[hi + 1]);
+          unpack2(add2(a, b), v[lo], v[lo + 1]);
+          unpack2(sub2(a, b), v[hi], v[hi + 1]);
+        }
+      }
+    }
+    for (int s = E; s < lpg; s <<= 1) {
+      const float sign = (threadIdx.x & s) != 0 ? -1.f : 1.f;
 #pragma unroll
       for (int i = 0; i < 32; ++i) {
         const float o = __shfl_xor_sync(0xffffffffu, v[i], s);
@@ -806,9 +880,14 @@ struct TacoCodec {
       }
     }
   }
+  static __device__ __forceinline__ void scaleAll(float (&v)[32], float f) {   // a packed multiply; -0 leaves the sign of zeros
+    const uint64_t f2 = pack2(f, f), z2 = 0x8000000080000000ull;
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) unpack2(fma2(pack2(v[i], v[i + 1]), f2, z2), v[i], v[i + 1]);
+  }
 
   static __device__ __forceinline__ Enc encode(float (&v)[32], const CodecCfg& c, bool rotate, float* /*sm*/,
-                                               uint64_t /*rngElem*/) {
+                                               uint64_t /*rngElem*/, uint4* win = nullptr) {
     const int lpg = c.group >> 5;
     float ss = 0.f;
 #pragma unroll
@@ -816,46 +895,83 @@ struct TacoCodec {
     for (int o = 1; o < lpg; o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     Enc e;
     e.ada = fminf(fmaxf(c.f2 * rsqrtf(ss / (float)c.group + c.f1), 1e-3f), 1e3f);
-#pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] *= e.ada;
+    e.spread = rotate;
     if (rotate) {
-      hadamard32(v);
-      lanes(v, lpg);
-      const float rsG = rsqrtf((float)c.group);
+      // the first stage takes the product with ada along in a multiply-add
+      uint64_t p[16];
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] *= rsG;
+      for (int i = 0; i < 16; ++i) {
+        const float b = v[2 * i + 1] * e.ada;
+        p[i] = pack2(fmaf(v[2 * i], e.ada, b), fmaf(v[2 * i], e.ada, -b));
+      }
+      hadamardPairs(p);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) unpack2(p[i], v[2 * i], v[2 * i + 1]);
+      byLanes(c, [&](auto n) {
+        constexpr int E = decltype(n)::value;
+        if constexpr (E > 1) exchange<E, true>(v, win);
+        lanes<E>(v, lpg);
+      });
+      scaleAll(v, rsqrtf((float)c.group));
+    } else {
+      scaleAll(v, e.ada);
     }
-    float m = 0.f;
-#pragma unroll
-    for (int i = 0; i < 32; ++i) m = fmaxf(m, fabsf(v[i]));
+    float m = maxAbs(v);
     for (int o = 1; o < lpg; o <<= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     e.qs = fminf(fmaxf(m / c.f0, 1e-12f), 1e6f);
     const float inv = 1.f / e.qs;
-    const __nv_fp8_interpretation_t fmt = (c.aux & 1) ? __NV_E5M2 : __NV_E4M3;
-    const __nv_saturation_t sat = (c.aux & 2) ? __NV_SATFINITE : __NV_NOSAT;
+    scaleAll(v, inv);
+    // Values within a rounding of +-448 are what the clamp and either conversion make 448 of; infinities, NaN (the sum of squares has
+    // them too) and a range beyond +-448 take the clamp and the conversion that was asked for.
+    auto convert = [&](__nv_saturation_t sat, __nv_fp8_interpretation_t fmt) {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      float q[4];
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * k], v[4 * k + 1]), sat, fmt);
+        const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v[4 * k + 2], v[4 * k + 3]), sat, fmt);
+        e.w[k] = lo | (hi << 16);
+      }
+    };
+    const bool plain = m * inv <= 449.f && ss < INFINITY;
+    if (!plain) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) q[i] = fminf(fmaxf(v[4 * k + i] * inv, -448.f), 448.f);
-      const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(q[0], q[1]), sat, fmt);
-      const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(q[2], q[3]), sat, fmt);
-      e.w[k] = lo | (hi << 16);
+      for (int i = 0; i < 32; ++i) v[i] = fminf(fmaxf(v[i], -448.f), 448.f);
     }
+    if (plain && (c.aux & 1) == 0) convert(__NV_SATFINITE, __NV_E4M3);
+    else if (plain) convert(__NV_SATFINITE, __NV_E5M2);
+    else convert((c.aux & 2) ? __NV_SATFINITE : __NV_NOSAT, (c.aux & 1) ? __NV_E5M2 : __NV_E4M3);
     return e;
   }
 
   static __device__ __forceinline__ void touched(const ChunkLayout& L, const CodecCfg& c, long elem, long* payloadEnd, long* totalEnd) {
     if (elem >= L.payloadBytes) { *payloadEnd = 0; *totalEnd = 0; return; }
-    *payloadEnd = elem + 32;
+    const int lpg = c.group >> 5, E = lpg < 4 ? lpg : 4;
+    *payloadEnd = (elem | (32L * E - 1)) + 1;                                   // the runs of the lanes that exchange theirs
     *totalEnd = L.payloadBytes + (L.groups + (elem >> groupShift(c)) + 1) * 4;   // the group's scale, then its adaptive factor
+  }
+
+  // First byte of this lane's 32 / E places in the first of its E runs; the others follow 32 bytes apart.
+  template <int E>
+  static __device__ __forceinline__ long placesAt(long elem) {
+    const int j = threadIdx.x & (E - 1);
+    return elem - 32 * j + j * (32 / E);
   }
 
   static __device__ __forceinline__ void store(const Enc& e, uint8_t* chunk, const ChunkLayout& L, const CodecCfg& c,
                                                long elem) {
     if (elem >= L.payloadBytes) return;  // runs of the padded last group are part of the stream
-    uint8_t* pw = chunk + elem;
-    storeWords(pw, e.w);
+    auto put = [&](auto n) {
+      constexpr int E = decltype(n)::value, W = 8 / E;
+      uint8_t* p = chunk + placesAt<E>(elem);
+#pragma unroll
+      for (int r = 0; r < E; ++r) {
+        uint32_t part[W];
+#pragma unroll
+        for (int i = 0; i < W; ++i) part[i] = e.w[r * W + i];
+        storeWords(p + 32 * r, part);
+      }
+    };
+    if (e.spread) byLanes(c, put);
+    else put(std::integral_constant<int, 1>{});
     if ((elem & (c.group - 1)) == 0) {
       float* ps = reinterpret_cast<float*>(chunk + L.payloadBytes);
       const long g = elem >> groupShift(c);
@@ -864,47 +980,103 @@ struct TacoCodec {
     }
   }
 
-  struct Raw {
-    uint32_t w[8];
-    float scale;  // qs / ada (* mul)
-    int e5m2;
-    bool valid;
-  };
-  static constexpr int kBatch = 2;
-
-  static __device__ __forceinline__ Raw fetch(const uint8_t* chunk, const ChunkLayout& L, const CodecCfg& c, long elem,
-                                              float mul, const float* /*sm*/ = nullptr) {
-    Raw r;
-    r.valid = elem < L.payloadBytes;
-    r.e5m2 = c.aux & 1;
-    if (!r.valid) return r;
-    const uint8_t* pw = chunk + elem;
-    loadWords(pw, r.w);
-    const float* ps = reinterpret_cast<const float*>(chunk + L.payloadBytes);
-    const long g = elem >> groupShift(c);
-    r.scale = __ldcg(ps + g) / __ldcg(ps + L.groups + g) * mul;
-    return r;
+  // acc += scale * values of the eight words
+  static __device__ __forceinline__ void addRun(const uint32_t (&w)[8], float scale, bool e5m2, float (&acc)[32]) {
+    const uint64_t s2 = pack2(scale, scale);
+    auto add = [&](int i, __half2_raw hr) {
+      const float2 f = __half22float2(*reinterpret_cast<__half2*>(&hr));
+      unpack2(fma2(pack2(f.x, f.y), s2, pack2(acc[i], acc[i + 1])), acc[i], acc[i + 1]);
+    };
+    if (e5m2) {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) add(2 * k, __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[k >> 1] >> (16 * (k & 1))), __NV_E5M2));
+    } else {
+#pragma unroll
+      for (int k = 0; k < 16; ++k) add(2 * k, __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(w[k >> 1] >> (16 * (k & 1))), __NV_E4M3));
+    }
   }
-
-  static __device__ __forceinline__ void accumulate(const Raw& r, float (&acc)[32]) {
-    if (!r.valid) return;
-    const __nv_fp8_interpretation_t fmt = r.e5m2 ? __NV_E5M2 : __NV_E4M3;
+  template <int E, int ALIGN>
+  static __device__ __forceinline__ void loadPlaces(const uint8_t* p, uint32_t (&w)[8]) {
+    constexpr int W = 8 / E;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int r = 0; r < E; ++r) {
+      uint32_t part[W];
+      loadWordsBy<(W >= 4 ? ALIGN : (ALIGN < 8 ? ALIGN : 8))>(p + 32 * r, part);
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        __half2_raw hr = __nv_cvt_fp8x2_to_halfraw2((__nv_fp8x2_storage_t)(r.w[k] >> (16 * h)), fmt);
-        const float2 f = __half22float2(*reinterpret_cast<__half2*>(&hr));
-        acc[4 * k + 2 * h] = fmaf(f.x, r.scale, acc[4 * k + 2 * h]);
-        acc[4 * k + 2 * h + 1] = fmaf(f.y, r.scale, acc[4 * k + 2 * h + 1]);
-      }
+      for (int i = 0; i < W; ++i) w[r * W + i] = part[i];
     }
   }
 
+  static constexpr bool kDirectSums = true;
+  template <int E, int ALIGN, int B>
+  static __device__ __forceinline__ void sumBatches(RunAddress& r, long groups, long stride, int& n, float mul, bool e5m2, float (&acc)[32]) {
+#pragma unroll 1
+    while (n >= B) {
+      uint32_t w[B][8];
+      float qs[B], ada[B];
+#pragma unroll
+      for (int j = 0; j < B; ++j) {
+        loadPlaces<E, ALIGN>(r.words(), w[j]);
+        qs[j] = __ldcg(reinterpret_cast<const float*>(r.params()));
+        ada[j] = __ldcg(reinterpret_cast<const float*>(r.params() + 4 * groups));
+        r.next(stride);
+      }
+#pragma unroll
+      for (int j = 0; j < B; ++j) addRun(w[j], qs[j] / ada[j] * mul, e5m2, acc);
+      n -= B;
+    }
+  }
+  static __device__ __forceinline__ void sum(const uint8_t* base, long stride, int n, const ChunkLayout& L, const CodecCfg& c, long elem,
+                                             float mul, bool aligned, bool spread, float (&acc)[32]) {
+    if (elem >= L.payloadBytes) return;
+    const long e0 = elem - (long)threadIdx.x * kElemsPerThread;
+    const int gs = groupShift(c);
+    auto go = [&](auto lanesTag, auto alignTag) {
+      constexpr int E = decltype(lanesTag)::value, ALIGN = decltype(alignTag)::value;
+      RunAddress r = {base + e0, base + L.payloadBytes + (e0 >> gs) * 4, (unsigned)placesAt<E>((long)threadIdx.x * kElemsPerThread),
+                      ((threadIdx.x * kElemsPerThread) >> gs) * 4u};
+      sumBatches<E, ALIGN, 2>(r, L.groups, stride, n, mul, (c.aux & 1) != 0, acc);
+      sumBatches<E, ALIGN, 1>(r, L.groups, stride, n, mul, (c.aux & 1) != 0, acc);
+    };
+    auto byAlign = [&](auto lanesTag) {
+      if (aligned) go(lanesTag, std::integral_constant<int, 16>{});
+      else go(lanesTag, std::integral_constant<int, 4>{});
+    };
+    if (spread) byLanes(c, byAlign);
+    else byAlign(std::integral_constant<int, 1>{});
+  }
+  // One copy in the spread ownership, its loads apart from its use (behind the chunk: zeros).
+  struct Ahead {
+    uint32_t w[8];
+    float qs, ada;
+  };
+  static __device__ __forceinline__ Ahead ahead(const uint8_t* base, const ChunkLayout& L, const CodecCfg& c, long elem) {
+    Ahead r = {};
+    r.ada = 1.f;
+    if (elem >= L.payloadBytes || !COCCL_CHUNK_RANGE_OK(TacoCodec, L, c, elem, 2)) return r;
+    byLanes(c, [&](auto n) {
+      constexpr int E = decltype(n)::value;
+      const uint8_t* p = base + placesAt<E>(elem);
+      if ((reinterpret_cast<uintptr_t>(base) & 15u) == 0) loadPlaces<E, 16>(p, r.w);
+      else loadPlaces<E, 4>(p, r.w);
+    });
+    const float* ps = reinterpret_cast<const float*>(base + L.payloadBytes) + (elem >> groupShift(c));
+    r.qs = __ldcg(ps);
+    r.ada = __ldcg(ps + L.groups);
+    return r;
+  }
+  static __device__ __forceinline__ void addAhead(const Ahead& r, const CodecCfg& c, float mul, float (&acc)[32]) {
+    addRun(r.w, r.qs / r.ada * mul, (c.aux & 1) != 0, acc);
+  }
+
   static __device__ __forceinline__ float finishScale(const CodecCfg& c) { return rsqrtf((float)c.group); }
-  static __device__ __forceinline__ void finish(float (&v)[32], const CodecCfg& c) {
+  static __device__ __forceinline__ void finish(float (&v)[32], const CodecCfg& c, uint4* win = nullptr) {
+    byLanes(c, [&](auto n) {
+      constexpr int E = decltype(n)::value;
+      lanes<E>(v, c.group >> 5);
+      if constexpr (E > 1) exchange<E, false>(v, win);
+    });
     hadamard32(v);
-    lanes(v, c.group >> 5);
   }
 };
 
@@ -929,6 +1101,7 @@ struct ZfpCodec {
   static constexpr int kEncodeBlocks = 4, kDecodeBlocks = RATE == 16 ? 3 : 4, kSumBlocks = 3;
   static constexpr int kMaxBits = 4 * RATE;
   // the plane tables of oracle/zfp1d_planes.h live in the kernel's shared scratch, behind its first 8 floats
+  static constexpr bool kExchanges = false;
   static constexpr bool kEncodeAhead = false;
   static constexpr int kSmemFloats = 8 + (int)sizeof(zfp1d::PlaneTables) / 4;
   static __device__ __forceinline__ const zfp1d::PlaneTables& tables(const float* sm) {
@@ -943,7 +1116,7 @@ struct ZfpCodec {
   struct Enc { uint32_t w[RATE]; };
 
   static __device__ __forceinline__ Enc encode(float (&v)[32], const CodecCfg& /*c*/, bool /*rotate*/, float* sm,
-                                               uint64_t /*rngElem*/) {
+                                               uint64_t /*rngElem*/, uint4* /*win*/ = nullptr) {
     Enc e;
     const zfp1d::PlaneTables& tab = tables(sm);
     if (RATE == 4) {
@@ -1034,7 +1207,7 @@ struct ZfpCodec {
   }
 
   static __device__ __forceinline__ float finishScale(const CodecCfg&) { return 1.f; }
-  static __device__ __forceinline__ void finish(float (&)[32], const CodecCfg&) {}
+  static __device__ __forceinline__ void finish(float (&)[32], const CodecCfg&, uint4* /*win*/ = nullptr) {}
 };
 
 template <class Codec, class = void> struct HasDirectSums : std::false_type {};
@@ -1044,7 +1217,7 @@ template <class Codec> struct HasDirectSums<Codec, std::enable_if_t<Codec::kDire
 // are issued before any of them is unpacked; what is left over after whole batches goes through the smaller batch sizes, so
 // that a single copy (all-gather, all-to-all) carries no code for absent ones.
 // `sm`: the kernel's shared scratch (Codec::kSmemFloats floats, Codec::initShared called); `aligned`: base and stride are
-// multiples of 16 bytes.
+// multiples of 16 bytes; `spread`: finish() follows (a re-encoding sum stays in the run ownership, see TacoCodec).
 template <class Codec, int B>
 __device__ __forceinline__ void decodeBatches(const uint8_t*& src, long stride, int& n, const ChunkLayout& L, const CodecCfg& c,
                                               long elem, float mul, float (&acc)[32], const float* sm) {
@@ -1061,12 +1234,16 @@ __device__ __forceinline__ void decodeBatches(const uint8_t*& src, long stride, 
 }
 template <class Codec>
 __device__ __forceinline__ void decodeSum(const uint8_t* base, long stride, int n, const ChunkLayout& L,
-                                          const CodecCfg& c, long elem, float mul, float (&acc)[32], const float* sm, bool aligned) {
+                                          const CodecCfg& c, long elem, float mul, float (&acc)[32], const float* sm, bool aligned,
+                                          bool spread) {
   if (!COCCL_CHUNK_RANGE_OK(Codec, L, c, elem, 2)) return;   // the same range of every copy
-  if constexpr (HasDirectSums<Codec>::value) { Codec::sum(base, stride, n, L, c, elem, mul, aligned, acc); return; }
-  if constexpr (Codec::kBatch >= 4) decodeBatches<Codec, 4>(base, stride, n, L, c, elem, mul, acc, sm);
-  if constexpr (Codec::kBatch >= 2) decodeBatches<Codec, 2>(base, stride, n, L, c, elem, mul, acc, sm);
-  decodeBatches<Codec, 1>(base, stride, n, L, c, elem, mul, acc, sm);
+  if constexpr (HasDirectSums<Codec>::value) {
+    Codec::sum(base, stride, n, L, c, elem, mul, aligned, spread, acc);
+  } else {
+    if constexpr (Codec::kBatch >= 4) decodeBatches<Codec, 4>(base, stride, n, L, c, elem, mul, acc, sm);
+    if constexpr (Codec::kBatch >= 2) decodeBatches<Codec, 2>(base, stride, n, L, c, elem, mul, acc, sm);
+    decodeBatches<Codec, 1>(base, stride, n, L, c, elem, mul, acc, sm);
+  }
 }
 
 // Dispatch a generic lambda on the runtime codec configuration. The functor receives a codec type tag;

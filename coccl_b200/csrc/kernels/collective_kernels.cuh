@@ -110,7 +110,7 @@ __device__ __forceinline__ void encodeTiles(const T* src, const ChunkLayout& L, 
 #pragma unroll
       for (int i = 0; i < 32; ++i) v[i] -= pv[i];
     }
-    const typename Codec::Enc enc = Codec::encode(v, c, true, sm, rngBase + (uint64_t)e);
+    const typename Codec::Enc enc = Codec::encode(v, c, true, sm, rngBase + (uint64_t)e, TileIO<T, false>::window(stage[s]));
     if (!COCCL_CHUNK_RANGE_OK(Codec, L, c, e, 1)) continue;
     for (int d = 0; d < nDst; ++d) Codec::store(enc, dst(d), L, c, e);
   }
@@ -158,7 +158,7 @@ __device__ __forceinline__ void decodeTiles(const uint8_t* enc, T* dst, const Ch
   auto put = [&](long t, float (&acc)[32]) {
     const long e0 = t * kTileElems, left = L.count - e0;
     const bool fast = TileIO<T, false>::fast(dst + e0, left);
-    Codec::finish(acc, c);
+    Codec::finish(acc, c, TileIO<T, false>::window(stage));
     if constexpr (ADD) {
       float pv[32];
       TileIO<T, false>::load(dst, L.count, e0, fast, stage, pv);
@@ -183,7 +183,7 @@ __device__ __forceinline__ void decodeTiles(const uint8_t* enc, T* dst, const Ch
       float acc[32];
 #pragma unroll
       for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-      decodeSum<Codec>(enc, 0, 1, L, c, t * kTileElems + lane, Codec::finishScale(c), acc, sm, aligned);
+      decodeSum<Codec>(enc, 0, 1, L, c, t * kTileElems + lane, Codec::finishScale(c), acc, sm, aligned, true);
       put(t, acc);
     }
   }
@@ -200,8 +200,12 @@ inline CollForm collForm(int op) {
   }
 }
 
+// The delta form holds a second run of values: with a codec that needs most of the registers itself, one CTA an SM fewer (TACO, 8 x 1 Mi
+// fp32: 215 us with three, 164 with two).
+template <class Codec, int FORM>
+constexpr int kFusedBlocks = FORM == kFormGatherDelta && Codec::kExchanges ? 2 : Codec::kMinBlocks;
 template <typename T, class Codec, int FORM>
-__global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollectiveKernel(const __grid_constant__ CollArgs a) {
+__global__ void __launch_bounds__(kTileThreads, kFusedBlocks<Codec, FORM>) fusedCollectiveKernel(const __grid_constant__ CollArgs a) {
   __shared__ TileStage<T> stage[FORM == kFormGatherDelta ? 1 : kEncodeStages<T, Codec>];
   __shared__ float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
@@ -290,14 +294,15 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) fusedCollecti
           float acc[32];
 #pragma unroll
           for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-          decodeSum<Codec>(myWs, a.slotBytes, N, L, c, e, FORM == kFormTwoShot ? 1.f : Codec::finishScale(c), acc, sm, aligned);
+          decodeSum<Codec>(myWs, a.slotBytes, N, L, c, e, FORM == kFormTwoShot ? 1.f : Codec::finishScale(c), acc, sm, aligned,
+                           FORM != kFormTwoShot);
           if constexpr (FORM == kFormTwoShot) {
             // stay in the rotated domain: the sum of rotated values is the rotation of the sum
             const typename Codec::Enc enc = Codec::encode(acc, c, false, sm, ((uint64_t)(0x80 + rank) << 40) + (uint64_t)e);
             if (COCCL_CHUNK_RANGE_OK(Codec, L, c, e, 3))
               for (int d = 0; d < N; ++d) Codec::store(enc, a.ws[peerAt(d)] + a.regionBOffset + (long)rank * a.slotBytes, L, c, e);
           } else {
-            Codec::finish(acc, c);
+            Codec::finish(acc, c, TileIO<T, false>::window(stage[0]));
             TileIO<T, false>::storeTile(out + e0, left, TileIO<T, false>::fast(out + e0, left), stage[0], acc);
           }
         }
@@ -419,7 +424,7 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKern
     float v[32];
     TileIO<T>::take(tile, left, e0 == 0, TileIO<T>::fast(tile, left), stage[s], v);
     const long e = e0 + (long)threadIdx.x * kElemsPerThread;
-    const typename Codec::Enc enc = Codec::encode(v, a.codec, true, sm, ((uint64_t)ch << 40) + (uint64_t)e);
+    const typename Codec::Enc enc = Codec::encode(v, a.codec, true, sm, ((uint64_t)ch << 40) + (uint64_t)e, TileIO<T>::window(stage[s]));
     if (COCCL_CHUNK_RANGE_OK(Codec, L, a.codec, e, 1)) Codec::store(enc, out, L, a.codec, e);
   }
 }
@@ -453,7 +458,7 @@ __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const
         src.next(w);
         dst.next(w);
         if (w.more()) r = fetch();
-        Codec::finish(acc, a.codec);
+        Codec::finish(acc, a.codec, TileIO<T>::window(stage));
         TileIO<T>::storeTile(tile, left, TileIO<T>::fast(tile, left), stage, acc);
       }
       return;
@@ -465,8 +470,8 @@ __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const
     float acc[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-    decodeSum<Codec>(src.p, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, Codec::finishScale(a.codec), acc, sm, encodedAligned(a));
-    Codec::finish(acc, a.codec);
+    decodeSum<Codec>(src.p, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, Codec::finishScale(a.codec), acc, sm, encodedAligned(a), true);
+    Codec::finish(acc, a.codec, TileIO<T>::window(stage));
     TileIO<T>::storeTile(dst.p, left, TileIO<T>::fast(dst.p, left), stage, acc);
   }
 }
@@ -487,7 +492,7 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) decodeReduceE
     float acc[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-    decodeSum<Codec>(src.p, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, 1.f, acc, sm, encodedAligned(a));
+    decodeSum<Codec>(src.p, a.chunks * a.encStrideIn, (int)a.reduce, L, a.codec, e, 1.f, acc, sm, encodedAligned(a), false);
     const typename Codec::Enc o = Codec::encode(acc, a.codec, false, sm, ((uint64_t)(0x40 + w.ch) << 40) + (uint64_t)e);
     Codec::store(o, dst.p, L, a.codec, e);
   }

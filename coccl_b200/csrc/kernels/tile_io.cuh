@@ -106,6 +106,8 @@ struct TileIO {
     return k32 ? r * 8 + (c ^ (r & 7)) : r * 4 + (c ^ ((r >> 1) & 3));
   }
 
+  // the warp's window: at least 2 KiB
+  static __device__ __forceinline__ uint4* window(TileStage<T>& st) { return st.buf + (threadIdx.x >> 5) * kWarpChunks; }
   // position of vector vi (0 .. kWarpChunks) of the warp's window
   static __device__ __forceinline__ uint4* place(TileStage<T>& st, int warp, int vi) {
     return vi == kWarpChunks ? st.extra + warp : st.buf + warp * kWarpChunks + slot(vi / kChunksPerRun, vi % kChunksPerRun);
