@@ -1109,8 +1109,8 @@ struct ZfpCodec {
   }
   // Every thread of the CTA calls this once, followed by a __syncthreads(), before any encode or fetch.
   static __device__ __forceinline__ void initShared(float* sm) {
-    zfp1d::PlaneTables& t = *reinterpret_cast<zfp1d::PlaneTables*>(sm + 8);
-    for (int i = threadIdx.x; i < zfp1d::kPlaneTableWork; i += blockDim.x) zfp1d::fillPlaneTables(t, i);
+    const uint4* t = reinterpret_cast<const uint4*>(&zfp1d::kPlaneTables);
+    for (int i = threadIdx.x; i < (int)(sizeof(zfp1d::PlaneTables) / 16); i += blockDim.x) reinterpret_cast<uint4*>(sm + 8)[i] = __ldg(t + i);
   }
 
   struct Enc { uint32_t w[RATE]; };

@@ -207,7 +207,7 @@ constexpr int kFusedBlocks = FORM == kFormGatherDelta && Codec::kExchanges ? 2 :
 template <typename T, class Codec, int FORM>
 __global__ void __launch_bounds__(kTileThreads, kFusedBlocks<Codec, FORM>) fusedCollectiveKernel(const __grid_constant__ CollArgs a) {
   __shared__ TileStage<T> stage[FORM == kFormGatherDelta ? 1 : kEncodeStages<T, Codec>];
-  __shared__ float sm[Codec::kSmemFloats];
+  __shared__ __align__(16) float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
   __syncthreads();
 
@@ -397,7 +397,7 @@ template <typename T, class Codec>
 __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKernel(const CodecArgs a) {
   constexpr int S = kEncodeStages<T, Codec>;
   __shared__ TileStage<T> stage[S];
-  __shared__ float sm[Codec::kSmemFloats];
+  __shared__ __align__(16) float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
   __syncthreads();
   const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);
@@ -433,7 +433,7 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKern
 template <typename T, class Codec, int BLOCKS>
 __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const CodecArgs a) {
   __shared__ TileStage<T> stage;
-  __shared__ float sm[Codec::kSmemFloats];
+  __shared__ __align__(16) float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
   __syncthreads();
   const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);
@@ -480,7 +480,7 @@ __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const
 // (reference kernel: sdp4bit/quantization/dequant_reduce_quant.cu:14-179).
 template <class Codec>
 __global__ void __launch_bounds__(kTileThreads, Codec::kMinBlocks) decodeReduceEncodeKernel(const CodecArgs a) {
-  __shared__ float sm[Codec::kSmemFloats];
+  __shared__ __align__(16) float sm[Codec::kSmemFloats];
   Codec::initShared(sm);
   __syncthreads();
   const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);

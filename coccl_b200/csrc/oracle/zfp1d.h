@@ -270,7 +270,7 @@ constexpr int kPlaneEncEntries = 5 * 16;    // [n][x]
 constexpr int kPlaneDecEntries = 5 * 128;   // [n][next 7 bits]
 
 // bits 0-7: code, LSB first; bits 8-11: length; bits 12-14: n after the plane
-COCCL_HD uint16_t planeCode(int n, uint32_t x) {
+COCCL_HD constexpr uint16_t planeCode(int n, uint32_t x) {
   uint32_t code = x & ((1u << n) - 1u);
   int len = n;
   uint32_t r = x >> n;
