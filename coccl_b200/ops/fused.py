@@ -9,6 +9,8 @@ accumulate epilogue) and returns None for that parameter.
 """
 from __future__ import annotations
 
+import threading
+
 import torch
 import torch.nn.functional as F
 
@@ -26,6 +28,44 @@ def scratch(device, nfloats: int, tag: str = "") -> torch.Tensor:
         t = torch.empty(max(nfloats, 1 << 16), dtype=torch.float32, device=device)
         _scratch[key] = t
     return t
+
+
+class Branch:
+    """A second stream for backward work that only ends in gradient buffers (weight and bias gradients, embedding tables) while a
+    forward and backward pass is captured into a graph: small products fill a fraction of the GPU and nothing waits for these, yet
+    in one stream they stand between the kernels that do wait for one another. All such work of a pass goes through one branch in
+    its old order, so every buffer sees its sums in the order of the launched pass. The tensors it reads are kept until `join`:
+    the allocator knows the main stream only and would hand their memory out again."""
+
+    _of_thread = threading.local()
+
+    def __init__(self, device):
+        self.stream, self.keep, self.used = torch.cuda.Stream(device), [], False
+
+    @classmethod
+    def current(cls):
+        """The branch of the pass that this thread is capturing (None: everything in one stream)."""
+        return getattr(cls._of_thread, "branch", None)
+
+    def __enter__(self):
+        self._of_thread.branch = self
+        return self
+
+    def __exit__(self, *exc):
+        self._of_thread.branch = None
+
+    def run(self, work, *reads):
+        """work() behind what the current stream holds so far, beside what it gets from now on."""
+        self.stream.wait_stream(torch.cuda.current_stream(self.stream.device))
+        self.keep.append(reads)
+        self.used = True
+        with torch.cuda.stream(self.stream):
+            return work()
+
+    def join(self, stream):
+        if self.used:
+            stream.wait_stream(self.stream)
+        self.keep = []
 
 
 def _accum_param_grad(p: torch.Tensor, g_fp32_or_none, compute):
@@ -146,6 +186,7 @@ class _Embed(torch.autograd.Function):
         # saved-tensor hook would hand back as plain tensors
         ctx.tables = (wte, wpe)
         ctx.meta = (b, s, first)
+        ctx.branch = Branch.current()
         return e
 
     @staticmethod
@@ -165,14 +206,21 @@ class _Embed(torch.autograd.Function):
                 grads[1] = F.pad(dy.reshape(b, s, H).sum(0), (0, 0, first, wpe.shape[0] - first - s))
         if any(straight):
             dy = dy.contiguous() if aligned16(dy) else dy.clone(memory_format=torch.contiguous_format)
-        lib, st = _lib.lib(), _lib.cur_stream()
-        if straight[0]:
-            sc = torch.empty(lib.cocclkEmbedScratchBytes(T, H), dtype=torch.uint8, device=dy.device)
-            _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), flat.data_ptr(), sc.data_ptr(), wte.main_grad.data_ptr(), T, H,
-                                          wte.shape[0], st), "cocclkEmbedBwd")
-        if straight[1]:
-            g = wpe.main_grad[first:first + s]
-            _lib.check(lib.cocclkEmbedPositionsBwd(dy.data_ptr(), g.data_ptr(), b, s, H, st), "cocclkEmbedPositionsBwd")
+        lib = _lib.lib()
+        sc = torch.empty(lib.cocclkEmbedScratchBytes(T, H), dtype=torch.uint8, device=dy.device) if straight[0] else None
+
+        def into_buffers():
+            st = _lib.cur_stream()
+            if straight[0]:
+                _lib.check(lib.cocclkEmbedBwd(dy.data_ptr(), flat.data_ptr(), sc.data_ptr(), wte.main_grad.data_ptr(), T, H,
+                                              wte.shape[0], st), "cocclkEmbedBwd")
+            if straight[1]:
+                g = wpe.main_grad[first:first + s]
+                _lib.check(lib.cocclkEmbedPositionsBwd(dy.data_ptr(), g.data_ptr(), b, s, H, st), "cocclkEmbedPositionsBwd")
+        if ctx.branch is not None:   # behind the gradient of a tied output head, which goes into the same buffer
+            ctx.branch.run(into_buffers, dy, flat, sc)
+        else:
+            into_buffers()
         return grads[0], grads[1], None, None
 
 
@@ -438,6 +486,7 @@ class _Linear(torch.autograd.Function):
         ctx.gelu = gelu
         ctx.has_bias = bias is not None
         ctx.in_shape = x.shape
+        ctx.branch = Branch.current()
         return y.reshape(*x.shape[:-1], N)
 
     @staticmethod
@@ -453,16 +502,25 @@ class _Linear(torch.autograd.Function):
                 rc = _lib.lib().cocclkGeluBwd(dy2.data_ptr(), z.data_ptr(), dz.data_ptr(), dz.numel(), _lib.cur_stream())
                 _lib.check(rc, "cocclkGeluBwd")
                 dy2 = dz
+
+            def parameter_grads():
+                dw = _accum_param_grad(w, None, lambda out, acc: G.gemm(dy2.t(), x2.t(), out=out, accumulate=acc))
+                db = None
+                if ctx.has_bias:
+                    def colsum(out, acc):
+                        sc = scratch(dy2.device, _lib.lib().cocclkColSumBlocks(M) * N, "colsum")
+                        rc = _lib.lib().cocclkColSum(dy2.data_ptr(), out.data_ptr(), int(acc), sc.data_ptr(), M, N,
+                                                     _lib.cur_stream())
+                        _lib.check(rc, "cocclkColSum")
+                    db = _accum_param_grad(bias, None, colsum)
+                return dw, db
+            buffers = all(p is None or getattr(p, "main_grad", None) is not None for p in (w, bias))
+            beside = ctx.branch is not None and buffers
+            if beside:
+                dw, db = ctx.branch.run(parameter_grads, dy2, x2)
             dx = G.gemm(dy2, w.t()) if ctx.needs_input_grad[0] else None
-            dw = _accum_param_grad(w, None, lambda out, acc: G.gemm(dy2.t(), x2.t(), out=out, accumulate=acc))
-            db = None
-            if ctx.has_bias:
-                def colsum(out, acc):
-                    sc = scratch(dy2.device, _lib.lib().cocclkColSumBlocks(M) * N, "colsum")
-                    rc = _lib.lib().cocclkColSum(dy2.data_ptr(), out.data_ptr(), int(acc), sc.data_ptr(), M, N,
-                                                 _lib.cur_stream())
-                    _lib.check(rc, "cocclkColSum")
-                db = _accum_param_grad(bias, None, colsum)
+            if not beside:
+                dw, db = parameter_grads()
         else:
             d = dy2.float()
             if ctx.gelu:

@@ -113,7 +113,7 @@ _shape_of, _type_of, _trains = map(operator.attrgetter, ("shape", "dtype", "requ
 
 class MicroBatchGraph:
     """Forward and backward of one micro-batch as a CUDA graph, for models whose kernels are shorter than the host code that
-    launches them.
+    launches them, with the parameters' gradients as a branch of their own beside the backward pass (`fused.Branch`).
 
     A micro-batch is about 35 launches a layer through autograd, 1.2 ms of host time a layer; below that much device work a
     layer the GPU waits (2 layers 512 wide, two micro-batches of 512 tokens: 5.0 ms a step for 1.4 ms of kernels). Replayed,
@@ -141,11 +141,16 @@ class MicroBatchGraph:
         self.launches = 0
 
     @classmethod
+    def pool_bytes(cls, cfg: GPTConfig, n_tokens: int, branch: bool) -> float:
+        # bf16 values a token leaves behind: 12 rows of the hidden size and 4 of the MLP's a layer, and its logits; with the
+        # gradients that a branch of the backward pass reads, 6 and 2 more
+        rows = (18 * cfg.hidden + 6 * cfg.ffn) if branch else (12 * cfg.hidden + 4 * cfg.ffn)
+        return 2.0 * n_tokens * (cfg.n_layer * rows + cfg.vocab)
+
+    @classmethod
     def worth_it(cls, cfg: GPTConfig, n_tokens: int) -> bool:
-        # bf16 values a token leaves behind: 12 rows of the hidden size and 4 of the MLP's a layer, and its logits
-        pool = 2.0 * n_tokens * (cfg.n_layer * (12 * cfg.hidden + 4 * cfg.ffn) + cfg.vocab)
         return (n_tokens <= cls.MAX_TOKENS and cfg.flops_per_token() * n_tokens <= cls.MAX_LAYER_FLOPS * max(1, cfg.n_layer) and
-                pool <= cls.MAX_POOL_BYTES)
+                cls.pool_bytes(cfg, n_tokens, False) <= cls.MAX_POOL_BYTES)
 
     @staticmethod
     def own_code(stage) -> bool:
@@ -229,7 +234,12 @@ class MicroBatchGraph:
             with torch.cuda.stream(side):
                 graph.capture_begin(capture_error_mode="thread_local")
                 try:
-                    t._micro_batch(tokens, scale)
+                    if self.pool_bytes(t.cfg, shape[0] * (shape[1] - 1), True) <= self.MAX_POOL_BYTES:
+                        with fused.Branch(t.device) as branch:
+                            t._micro_batch(tokens, scale)
+                        branch.join(side)
+                    else:
+                        t._micro_batch(tokens, scale)
                 finally:
                     graph.capture_end()
             if any(p.grad is not None for p in params):
