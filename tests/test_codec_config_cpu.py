@@ -1,0 +1,30 @@
+"""What a codec configuration keeps for its calls stays out of its identity."""
+import copy
+import dataclasses
+import pickle
+
+import torch
+
+from coccl_b200.ops.codec import CodecConfig
+
+
+def test_layouts_are_no_part_of_a_configuration():
+    a, b = CodecConfig("sdp4bit", 4, 128, False, True, seed=7), CodecConfig("sdp4bit", 4, 128, False, True, seed=7)
+    n32, n16 = a.encoded_chunk_bytes(1000, torch.float32), a.encoded_chunk_bytes(1000, torch.bfloat16)
+    assert (n32, n16) == (8 * 64 + 8 * 4, 8 * 64 + 8 * 8)
+    assert a == b and hash(a) == hash(b) and repr(a) == repr(b) and dataclasses.asdict(a) == dataclasses.asdict(b)
+    for c in (copy.copy(a), copy.deepcopy(a), pickle.loads(pickle.dumps(a))):
+        assert c == a and "_layouts" not in vars(c)
+        assert c.encoded_chunk_bytes(1000, torch.float32) == n32
+    wider = dataclasses.replace(a, group=64)
+    assert wider.encoded_chunk_bytes(1000, torch.float32) == 16 * 32 + 16 * 4
+    assert a.layout(torch.float32)[0].paramBytes == 4 and a.layout(torch.float16)[0].paramBytes == 8
+    assert a.layout(torch.float32)[0].seed == 7
+
+
+def test_encoded_sizes_of_every_kind():
+    want = {("zfp", 4): 500, ("zfp", 16): 2000, ("mxfp8", 8): 1024 + 32, ("taco", 8): 8 * 128 + 8 * 8}
+    for (kind, bits), n in want.items():
+        cfg = CodecConfig(kind, bits, {"zfp": 4, "mxfp8": 32, "taco": 128}[kind], False, False)
+        assert cfg.encoded_chunk_bytes(1000, torch.float32) == n
+    assert CodecConfig("zfp", 5, 4, False, False).encoded_chunk_bytes(1002, torch.float32) == -(-(251 * 20 // 8) // 4) * 4

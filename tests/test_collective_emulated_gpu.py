@@ -162,3 +162,22 @@ def test_all_gather_delta_tracks_slowly_moving_parameters(cuda, dtype):
             plain_err = (plain.float() - exact).abs().max().item()
     if dtype == torch.float32:
         assert err < 0.2 * plain_err, (err, plain_err)
+
+
+def test_one_state_serves_calls_of_different_kinds(cuda):
+    """Operations, sizes, types, codecs and slices in turn through one state: what each gives with a state of its own; results of
+    earlier calls stay as they are."""
+    from coccl_b200.ops import codec as C
+    torch.manual_seed(3)
+    calls = [("reduce_scatter", torch.float32, 4 * 10004, C.SDP4BIT_G128, None), ("all_gather", torch.bfloat16, 5003, C.MXFP8, None),
+             ("reduce_scatter", torch.float32, 4 * 10004, C.SDP4BIT_G128, None), ("all_reduce_twoshot", torch.bfloat16, 4 * 9001, C.SDP4BIT_G128, 1),
+             ("all_reduce_twoshot", torch.bfloat16, 4 * 9001, C.TACO_G128, None), ("reduce_scatter", torch.bfloat16, 4 * 10004, C.SDP4BIT_G128, None)]
+    state, kept = {}, []
+    for epoch, (op, dtype, numel, cfg, tiles) in enumerate(calls, 1):
+        xs = [torch.randn(numel, device=cuda).to(dtype) for _ in range(4)]
+        outs = K.emulate_collective(op, xs, cfg, epoch=epoch, state=state, slice_tiles=tiles)
+        want = K.emulate_collective(op, xs, cfg, slice_tiles=tiles)
+        kept.append((outs, want))
+        assert all(o.data_ptr() % 16 == 0 and o.is_contiguous() and o.dim() == 1 for o in outs)
+    for outs, want in kept:
+        assert all(torch.equal(a, b) for a, b in zip(outs, want))
