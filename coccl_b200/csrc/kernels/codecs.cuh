@@ -1038,8 +1038,10 @@ struct TacoCodec {
       sumBatches<E, ALIGN, 2>(r, L.groups, stride, n, mul, (c.aux & 1) != 0, acc);
       sumBatches<E, ALIGN, 1>(r, L.groups, stride, n, mul, (c.aux & 1) != 0, acc);
     };
-    auto byAlign = [&](auto lanesTag) {
-      if (aligned) go(lanesTag, std::integral_constant<int, 16>{});
+    auto byAlign = [&](auto lanesTag) {   // four lanes' places are eight bytes, others' whole vectors
+      constexpr int WIDE = decltype(lanesTag)::value == 4 ? 8 : 16;
+      const bool wide = aligned || (WIDE == 8 && ((reinterpret_cast<uintptr_t>(base) | (uintptr_t)stride) & 7u) == 0);
+      if (wide) go(lanesTag, std::integral_constant<int, WIDE>{});
       else go(lanesTag, std::integral_constant<int, 4>{});
     };
     if (spread) byLanes(c, byAlign);
@@ -1056,8 +1058,9 @@ struct TacoCodec {
     if (elem >= L.payloadBytes || !COCCL_CHUNK_RANGE_OK(TacoCodec, L, c, elem, 2)) return r;
     byLanes(c, [&](auto n) {
       constexpr int E = decltype(n)::value;
+      constexpr int WIDE = E == 4 ? 8 : 16;
       const uint8_t* p = base + placesAt<E>(elem);
-      if ((reinterpret_cast<uintptr_t>(base) & 15u) == 0) loadPlaces<E, 16>(p, r.w);
+      if ((reinterpret_cast<uintptr_t>(base) & (WIDE - 1)) == 0) loadPlaces<E, WIDE>(p, r.w);
       else loadPlaces<E, 4>(p, r.w);
     });
     const float* ps = reinterpret_cast<const float*>(base + L.payloadBytes) + (elem >> groupShift(c));
