@@ -5,6 +5,7 @@
 // change, so here the work is one read of the output gradient and one read-modify-write of those rows (167 MB, 26 us to
 // copy): 38 us, with 9 us for the order of the tokens and 15 us for the positions. Rows are summed in a fixed order,
 // whatever the launch: the result does not depend on scheduling.
+#include "dependent_launch.h"
 #include "launch_count.h"
 #include "common.cuh"
 #include "train_api.h"
@@ -20,6 +21,8 @@ constexpr int kEmbCols = kEmbLanes * 8;
 // equal ids and the run's length. places[rank] = {token, place in the run, length of the run, id (-1: not one of a table)}.
 // A warp per token compares its id with all others (T^2 comparisons in all). The counters of embedRowsKernel are zeroed on the way.
 __global__ void __launch_bounds__(256) embedOrderKernel(const long* ids, int4* places, unsigned* counters, int nCounters, int T) {
+  releaseNext();
+  awaitPrevious();
   for (int i = blockIdx.x * 256 + threadIdx.x; i < nCounters; i += gridDim.x * 256) counters[i] = 0u;
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= T) return;
@@ -69,6 +72,8 @@ __global__ void __launch_bounds__(256) embedOrderKernel(const long* ids, int4* p
 constexpr int kEmbPiece = 64;
 __global__ void __launch_bounds__(kEmbThreads, 6) embedRowsKernel(const bf16* dy, const int4* places, float* parts,
                                                                unsigned* counters, float* grad, int T, int H, long vocab) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float other[kEmbLanes][9];
   __shared__ bool last;
   const int i0 = blockIdx.x;
@@ -165,6 +170,8 @@ __global__ void __launch_bounds__(kEmbThreads, 6) embedRowsKernel(const bf16* dy
 
 // grad[s] += sum over the batch of dy[b][s], for the `seq` positions of dy [batch][seq][H]
 __global__ void __launch_bounds__(256) embedPositionsKernel(const bf16* dy, float* grad, int batch, long n) {
+  releaseNext();
+  awaitPrevious();
   const long i = ((long)blockIdx.x * 256 + threadIdx.x) * 8;   // n = seq * H, a multiple of 8
   if (i >= n) return;
   float acc[8], v[8];
@@ -202,8 +209,8 @@ extern "C" int cocclkEmbedBwd(const void* dy, const long* ids, void* scratch, fl
   char* b = (char*)scratch;
   int4* places = (int4*)b;
   unsigned* counters = (unsigned*)(b + L.countersAt);
-  embedOrderKernel<<<(T + 7) / 8, 256, 0, s>>>(ids, places, counters, (int)(L.windows * L.colBlocks), T);
-  embedRowsKernel<<<dim3((unsigned)T, (unsigned)L.colBlocks), kEmbThreads, 0, s>>>((const bf16*)dy, places, (float*)(b + L.partsAt), counters,
+  launchAfter(embedOrderKernel, (T + 7) / 8, 256, 0, s, ids, places, counters, (int)(L.windows * L.colBlocks), T);
+  launchAfter(embedRowsKernel, dim3((unsigned)T, (unsigned)L.colBlocks), kEmbThreads, 0, s, (const bf16*)dy, places, (float*)(b + L.partsAt), counters,
                                                                             grad, T, H, vocab);
   cocclkCountLaunches(2);
   return (int)cudaGetLastError();
@@ -212,7 +219,7 @@ extern "C" int cocclkEmbedBwd(const void* dy, const long* ids, void* scratch, fl
 extern "C" int cocclkEmbedPositionsBwd(const void* dy, float* grad, int batch, int seq, int H, cudaStream_t s) {
   if (batch <= 0 || seq <= 0 || H <= 0 || H % 8) return -1;
   const long n = (long)seq * H;
-  embedPositionsKernel<<<(unsigned)((n / 8 + 255) / 256), 256, 0, s>>>((const bf16*)dy, grad, batch, n);
+  launchAfter(embedPositionsKernel, (unsigned)((n / 8 + 255) / 256), 256, 0, s, (const bf16*)dy, grad, batch, n);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }

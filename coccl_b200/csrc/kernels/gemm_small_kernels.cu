@@ -12,6 +12,7 @@
 // 512 x 512 x 2048: 8.0 us (4 ranks) against 15.7 us with pair tiles; the rule and the sweep behind it are in gemm_kernels.cu.
 // Waits are bounded as in gemm_kernels.cu; every thread reaches both cluster barriers whatever happened before.
 #include "gemm_epilogue.cuh"
+#include "dependent_launch.h"
 #include "launch_count.h"
 #include "per_device.h"
 
@@ -76,6 +77,8 @@ gemmSmallKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
   __syncthreads();
   tcFenceAfter();
   const uint32_t tmem = bars->tmemBase;
+  releaseNext();
+  awaitPrevious();   // nothing above reads or writes what another kernel may
 
   if (warp == 0) {
     {
@@ -260,13 +263,15 @@ extern "C" int cocclkGemmBf16Small(const void* A, long lda, int aMN, const void*
   cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = (size_t)smemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)ranks;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)ranks;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = ranks > 1 ? 1 : 0;
+  cfg.numAttrs = ranks > 1 ? 2 : 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, gemmSmallKernel, ta, tb, g, ranks);
   cocclkCountLaunches(1);
   return (int)e;

@@ -5,6 +5,7 @@
 // moves every byte once. As PyTorch operations the same work was about fifty launches a layer and several fp32 passes over
 // the activations: at 4096 wide, 32 + 8 heads of 128 with norms, ffn 12288 and 4096 tokens 5.3 ms of device time for two
 // layers forward and backward, 0.42 ms here.
+#include "dependent_launch.h"
 #include "launch_count.h"
 #include "common.cuh"
 #include "train_api.h"
@@ -54,6 +55,8 @@ __device__ __forceinline__ float groupSum(float x) {
 // 128 with norms: 20 us forward (100 MB, 15 us to copy), 46 us backward (151 MB, 23 us; 127 registers, two CTAs an SM).
 template <int D, bool NORM, bool BWD>
 __global__ void __launch_bounds__(256) rotateKernel(const RotateArgs a) {
+  releaseNext();
+  awaitPrevious();
   constexpr int G = D / 16, H2 = D / 2;
   __shared__ float red[BWD && NORM ? 2 * D * 8 : 1];
   const int slot = threadIdx.x % G, hl = threadIdx.x / G;
@@ -202,6 +205,8 @@ __global__ void __launch_bounds__(256) rotateKernel(const RotateArgs a) {
 // copy), backward 85 us for 503 MB (77 us).
 template <bool BWD>
 __global__ void __launch_bounds__(256) swigluKernel(const bf16* z, const bf16* dy, bf16* out, int M, int F) {
+  releaseNext();
+  awaitPrevious();
   const int nvec = F / 8;
   const int v = blockIdx.x * blockDim.x + threadIdx.x;
   if (v >= nvec) return;
@@ -241,7 +246,7 @@ static int launchSwiglu(const void* z, const void* dy, void* out, int M, int F, 
   const int bx = (F / 8 + 255) / 256;
   // two waves of resident CTAs (8 of 256 threads an SM) walk the rows; fewer rows: one CTA a row and column block
   const int by = 148 * 16 / bx > 0 ? 148 * 16 / bx : 1;
-  swigluKernel<BWD><<<dim3(bx, M < by ? M : by), 256, 0, s>>>((const bf16*)z, (const bf16*)dy, (bf16*)out, M, F);
+  launchAfter(swigluKernel<BWD>, dim3(bx, M < by ? M : by), 256, 0, s, (const bf16*)z, (const bf16*)dy, (bf16*)out, M, F);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
@@ -263,7 +268,7 @@ static int launchRotate(RotateArgs a, int D, cudaStream_t s) {
   a.perIter = (heads + a.iters - 1) / a.iters;
   const int threads = (a.perIter * G + 31) / 32 * 32;
   const int grid = BWD ? cocclkRotateBwdGrid(a.tokens) : (a.tokens < 148 * 8 ? a.tokens : 148 * 8);
-#define ROT(DD) (norm ? rotateKernel<DD, true, BWD><<<grid, threads, 0, s>>>(a) : rotateKernel<DD, false, BWD><<<grid, threads, 0, s>>>(a))
+#define ROT(DD) (norm ? launchAfter(rotateKernel<DD, true, BWD>, grid, threads, 0, s, a) : launchAfter(rotateKernel<DD, false, BWD>, grid, threads, 0, s, a))
   switch (D) {
     case 32: ROT(32); break;
     case 64: ROT(64); break;

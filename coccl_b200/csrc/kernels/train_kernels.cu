@@ -6,6 +6,7 @@
 // The reference ships no trainer (its training layer is an empty submodule,
 // .gitmodules:1-3); these kernels belong to the framework layer that drives the
 // compressed collectives. Each kernel touches every byte once.
+#include "dependent_launch.h"
 #include "launch_count.h"
 #include "common.cuh"
 #include "train_api.h"
@@ -60,6 +61,8 @@ template <int NV, bool RMS>
 __global__ void __launch_bounds__(kLnThreads) normFwdKernel(const bf16* x, const bf16* res, const bf16* gamma,
                                                             const bf16* beta, bf16* y, bf16* xOut, float* mean,
                                                             float* rstd, int M, int H, float eps) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float sm[32];
   const int nvec = H / 8;
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
@@ -140,6 +143,8 @@ template <int NV, bool RMS>
 __global__ void __launch_bounds__(kLnThreads) normBwdKernel(const bf16* dy, const bf16* x, const float* mean,
                                                             const float* rstd, const bf16* gamma, const bf16* dres,
                                                             bf16* dx, float* partial, int M, int H) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float2 sm[2][8];
   const int nvec = H / 8, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   float dg[NV][8], db[RMS ? 1 : NV][8];
@@ -240,6 +245,8 @@ template <bool RMS>
 __global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf16* dy, const bf16* x, const float* mean,
                                                                        const float* rstd, const bf16* gamma, const bf16* dres,
                                                                        bf16* dx, float* partial, int M, int H) {
+  releaseNext();
+  awaitPrevious();
   extern __shared__ float4 lnSums[];   // [dgamma | dbeta][vector of the thread][half][thread]
   __shared__ float2 sm[2][kLnWideThreads / 32];
   const int nvec = H / 8, warp = threadIdx.x >> 5, sums = (nvec + kLnWideThreads - 1) / kLnWideThreads * 2;
@@ -351,6 +358,8 @@ constexpr int kColReduceCols = 32;
 template <int WARPS>
 __global__ void __launch_bounds__(32 * WARPS) colReduceKernel(const float* partial, float* out, float* out2, long split, int rows,
                                                              long cols, long stride, int accumulate) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float red[WARPS][33];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const long c = (long)blockIdx.x * kColReduceCols + lane;
@@ -382,8 +391,8 @@ __global__ void __launch_bounds__(32 * WARPS) colReduceKernel(const float* parti
 void launchColReduce(const float* partial, float* out, float* out2, long split, int rows, long cols, long stride, int accumulate,
                      cudaStream_t s) {
   const unsigned grid = (unsigned)((cols + kColReduceCols - 1) / kColReduceCols);
-  if (rows > 64 && grid <= 2 * 148) colReduceKernel<32><<<grid, 32 * 32, 0, s>>>(partial, out, out2, split, rows, cols, stride, accumulate);
-  else colReduceKernel<8><<<grid, 32 * 8, 0, s>>>(partial, out, out2, split, rows, cols, stride, accumulate);
+  if (rows > 64 && grid <= 2 * 148) launchAfter(colReduceKernel<32>, grid, 32 * 32, 0, s, partial, out, out2, split, rows, cols, stride, accumulate);
+  else launchAfter(colReduceKernel<8>, grid, 32 * 8, 0, s, partial, out, out2, split, rows, cols, stride, accumulate);
   cocclkCountLaunches(1);
 }
 
@@ -392,6 +401,8 @@ void launchColReduce(const float* partial, float* out, float* out2, long split, 
 // A CTA owns 256 columns (32 lanes x 8) and `rowsPerBlock` rows; its 8 warps take every 8th row, four rows in
 // flight per thread, and fold their sums through shared memory. A warp reads 512 contiguous bytes of one row.
 __global__ void __launch_bounds__(256) colSumPartialKernel(const bf16* x, float* partial, int M, int N, int rowsPerBlock) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float red[8][32][9];
   const int lane = threadIdx.x & 31, wy = threadIdx.x >> 5;
   const int col = (blockIdx.x * 32 + lane) * 8;
@@ -448,6 +459,8 @@ __device__ __forceinline__ float geluGrad(float x) {
 }
 // y = gelu(z (+ bias)); zOut = z + bias (optional)
 __global__ void __launch_bounds__(256) geluFwdKernel(const bf16* z, const bf16* bias, bf16* y, bf16* zOut, long n, int N) {
+  releaseNext();
+  awaitPrevious();
   for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += (long)gridDim.x * blockDim.x * 8) {
     float v[8];
     Vec8<bf16>::load(z + i, 8, true, v);
@@ -469,6 +482,8 @@ __global__ void __launch_bounds__(256) geluFwdKernel(const bf16* z, const bf16* 
 }
 // dz = dy * gelu'(z)
 __global__ void __launch_bounds__(256) geluBwdKernel(const bf16* dy, const bf16* z, bf16* dz, long n) {
+  releaseNext();
+  awaitPrevious();
   for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += (long)gridDim.x * blockDim.x * 8) {
     float d[8], v[8];
     Vec8<bf16>::load(dy + i, 8, true, d);
@@ -501,6 +516,8 @@ __device__ __forceinline__ void cpAsync16(uint32_t smem, const void* g) {
 template <int THREADS, int VECS>
 __global__ void __launch_bounds__(THREADS) crossEntropyKernel(bf16* logits, const long* targets, float* loss,
                                                                  int M, int V, long ld, float gscale) {
+  releaseNext();
+  awaitPrevious();
   extern __shared__ __align__(16) uint8_t ceRow[];
   __shared__ float sm[32];
   const int nvec = V / 8;
@@ -577,6 +594,8 @@ __global__ void __launch_bounds__(THREADS) crossEntropyKernel(bf16* logits, cons
 // (softmax - onehot) * gscale. Rows with target < 0 get loss 0 and a zero gradient.
 __global__ void __launch_bounds__(kCeThreads) ceStatsKernel(const bf16* logits, const long* targets, float4* stats,
                                                             int M, int V, long ld, long vocabOffset) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float sm[32];
   const int nvec = V / 8;
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
@@ -614,6 +633,8 @@ __global__ void __launch_bounds__(kCeThreads) ceStatsKernel(const bf16* logits, 
 // statsAll: [tp][M] entries of pass 1 from every rank (this rank's included).
 __global__ void __launch_bounds__(kCeThreads) ceFinishKernel(bf16* logits, const long* targets, const float4* statsAll, int tp,
                                                              float* loss, int M, int V, long ld, long vocabOffset, float gscale) {
+  releaseNext();
+  awaitPrevious();
   const int nvec = V / 8;
   for (int row = blockIdx.x; row < M; row += gridDim.x) {
     bf16* lr = logits + (long)row * ld;
@@ -655,6 +676,8 @@ template <typename G>
 __global__ void __launch_bounds__(256) adamKernel(float* master, float* m, float* v, const G* grad, bf16* param,
                                                   long n, float lr, float b1, float b2, float eps, float wd,
                                                   float bc1, float bc2, const float* gradScale) {
+  releaseNext();
+  awaitPrevious();
   const float gs = gradScale ? *gradScale : 1.f;
   for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += (long)gridDim.x * blockDim.x * 8) {
     const long left = n - i;
@@ -681,6 +704,8 @@ __global__ void __launch_bounds__(256) adamKernel(float* master, float* m, float
 
 template <typename G>
 __global__ void __launch_bounds__(256) sumSqPartialKernel(const G* x, long n, float* partial) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float sm[32];
   float s = 0.f;
   for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += (long)gridDim.x * blockDim.x * 8) {
@@ -695,6 +720,8 @@ __global__ void __launch_bounds__(256) sumSqPartialKernel(const G* x, long n, fl
 }
 // out[0] (+)= sum(partial)
 __global__ void __launch_bounds__(256) sumFinalKernel(const float* partial, int n, float* out, int accumulate) {
+  releaseNext();
+  awaitPrevious();
   __shared__ float sm[32];
   float s = 0.f;
   for (int i = threadIdx.x; i < n; i += blockDim.x) s += partial[i];
@@ -703,6 +730,8 @@ __global__ void __launch_bounds__(256) sumFinalKernel(const float* partial, int 
 }
 // coef = gradScaleIn * min(1, maxNorm / (sqrt(sumsq) * gradScaleIn + 1e-6))
 __global__ void clipCoefKernel(const float* sumsq, float maxNorm, float gradScaleIn, float* coef, float* normOut) {
+  releaseNext();
+  awaitPrevious();
   const float norm = sqrtf(sumsq[0]) * gradScaleIn;
   if (normOut) normOut[0] = norm;
   float c = 1.f;
@@ -712,6 +741,8 @@ __global__ void clipCoefKernel(const float* sumsq, float maxNorm, float gradScal
 
 // dst(fp32) += src(bf16)  /  dst = src
 __global__ void __launch_bounds__(256) accumBf16Kernel(float* dst, const bf16* src, long n, int accumulate) {
+  releaseNext();
+  awaitPrevious();
   for (long i = ((long)blockIdx.x * blockDim.x + threadIdx.x) * 8; i < n; i += (long)gridDim.x * blockDim.x * 8) {
     const long left = n - i;
     const bool vec = left >= 8;
@@ -748,7 +779,7 @@ static int launchNormFwd(const void* x, const void* res, const void* gamma, cons
   if (H % 8 || H <= 0 || H > kLnThreads * kLnMaxVec * 8 || M <= 0) return -1;
   const int threads = normThreads(H), cap = 148 * 8 * (kLnThreads / threads), grid = M < cap ? M : cap;
   const int nv = (H / 8 + threads - 1) / threads;
-#define NORM_FWD(NV) normFwdKernel<NV, RMS><<<grid, threads, 0, s>>>((const bf16*)x, (const bf16*)res, (const bf16*)gamma, \
+#define NORM_FWD(NV) launchAfter(normFwdKernel<NV, RMS>, grid, threads, 0, s, (const bf16*)x, (const bf16*)res, (const bf16*)gamma, \
       (const bf16*)beta, (bf16*)y, (bf16*)xOut, mean, rstd, M, H, eps)
   if (nv <= 1) NORM_FWD(1); else if (nv <= 2) NORM_FWD(2); else if (nv <= 4) NORM_FWD(4); else NORM_FWD(8);
 #undef NORM_FWD
@@ -765,7 +796,7 @@ static int launchNormBwd(const void* dy, const void* x, const float* mean, const
   if (H % 8 || H <= 0 || H > kLnThreads * kLnMaxVec * 8 || M <= 0) return -1;
   int grid = cocclkLayerNormBwdGrid(M);
   const int threads = normThreads(H), nv = (H / 8 + threads - 1) / threads;
-#define NORM_BWD(NV) normBwdKernel<NV, RMS><<<grid, threads, 0, s>>>((const bf16*)dy, (const bf16*)x, mean, rstd, \
+#define NORM_BWD(NV) launchAfter(normBwdKernel<NV, RMS>, grid, threads, 0, s, (const bf16*)dy, (const bf16*)x, mean, rstd, \
       (const bf16*)gamma, (const bf16*)dres, (bf16*)dx, scratch, M, H)
   if (nv <= 1) NORM_BWD(1);
   else if (nv <= 2) NORM_BWD(2);
@@ -775,7 +806,7 @@ static int launchNormBwd(const void* dy, const void* x, const float* mean, const
     grid = (M + rounds - 1) / rounds;   // one CTA an SM, as many rows for each
     const cudaError_t e = cudaFuncSetAttribute(normBwdWideKernel<RMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return (int)e;   // per device: a process may use several
-    normBwdWideKernel<RMS><<<grid, kLnWideThreads, smem, s>>>((const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)gamma,
+    launchAfter(normBwdWideKernel<RMS>, grid, kLnWideThreads, smem, s, (const bf16*)dy, (const bf16*)x, mean, rstd, (const bf16*)gamma,
                                                               (const bf16*)dres, (bf16*)dx, scratch, M, H);
   }
 #undef NORM_BWD
@@ -821,7 +852,7 @@ extern "C" int cocclkColSum(const void* x, float* out, int accumulate, float* sc
   const int by = colSumBlocks(M, N);
   const int rowsPer = (M + by - 1) / by;
   dim3 grid((N / 8 + 31) / 32, by);
-  colSumPartialKernel<<<grid, 256, 0, s>>>((const bf16*)x, scratch, M, N, rowsPer);
+  launchAfter(colSumPartialKernel, grid, 256, 0, s, (const bf16*)x, scratch, M, N, rowsPer);
   launchColReduce(scratch, out, nullptr, N, by, N, N, accumulate, s);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
@@ -829,13 +860,13 @@ extern "C" int cocclkColSum(const void* x, float* out, int accumulate, float* sc
 
 extern "C" int cocclkGeluFwd(const void* z, const void* bias, void* y, void* zOut, long n, int N, cudaStream_t s) {
   if (n % 8 || N % 8) return -1;
-  geluFwdKernel<<<gridForElems(n, 2048), 256, 0, s>>>((const bf16*)z, (const bf16*)bias, (bf16*)y, (bf16*)zOut, n, N);
+  launchAfter(geluFwdKernel, gridForElems(n, 2048), 256, 0, s, (const bf16*)z, (const bf16*)bias, (bf16*)y, (bf16*)zOut, n, N);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
 extern "C" int cocclkGeluBwd(const void* dy, const void* z, void* dz, long n, cudaStream_t s) {
   if (n % 8) return -1;
-  geluBwdKernel<<<gridForElems(n, 2048), 256, 0, s>>>((const bf16*)dy, (const bf16*)z, (bf16*)dz, n);
+  launchAfter(geluBwdKernel, gridForElems(n, 2048), 256, 0, s, (const bf16*)dy, (const bf16*)z, (bf16*)dz, n);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
@@ -850,8 +881,8 @@ extern "C" int cocclkCrossEntropy(void* logits, const long* targets, float* loss
     const cudaError_t e = cudaFuncSetAttribute(crossEntropyKernel<kCeThreads, kCeMaxVec>, cudaFuncAttributeMaxDynamicSharedMemorySize, kCeThreads * kCeMaxVec * 16);
     if (e != cudaSuccess) return (int)e;
   }
-  if (narrow) crossEntropyKernel<256, 4><<<grid, 256, (size_t)V * 2, s>>>((bf16*)logits, targets, loss, M, V, ld, gscale);
-  else crossEntropyKernel<kCeThreads, kCeMaxVec><<<grid, kCeThreads, (size_t)V * 2, s>>>((bf16*)logits, targets, loss, M, V, ld, gscale);
+  if (narrow) launchAfter(crossEntropyKernel<256, 4>, grid, 256, (size_t)V * 2, s, (bf16*)logits, targets, loss, M, V, ld, gscale);
+  else launchAfter(crossEntropyKernel<kCeThreads, kCeMaxVec>, grid, kCeThreads, (size_t)V * 2, s, (bf16*)logits, targets, loss, M, V, ld, gscale);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
@@ -860,7 +891,7 @@ extern "C" int cocclkCrossEntropyStats(const void* logits, const long* targets, 
                                        long vocabOffset, cudaStream_t s) {
   if (V % 8 || V > kCeThreads * kCeMaxVec * 8 || ld % 8 || M <= 0) return -1;
   const int grid = M < 148 * 2 ? M : 148 * 2;
-  ceStatsKernel<<<grid, kCeThreads, 0, s>>>((const bf16*)logits, targets, reinterpret_cast<float4*>(stats), M, V, ld, vocabOffset);
+  launchAfter(ceStatsKernel, grid, kCeThreads, 0, s, (const bf16*)logits, targets, reinterpret_cast<float4*>(stats), M, V, ld, vocabOffset);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
@@ -868,7 +899,7 @@ extern "C" int cocclkCrossEntropyFinish(void* logits, const long* targets, const
                                         int V, long ld, long vocabOffset, float gscale, cudaStream_t s) {
   if (V % 8 || V > kCeThreads * kCeMaxVec * 8 || ld % 8 || M <= 0 || tp < 1) return -1;
   const int grid = M < 148 * 2 ? M : 148 * 2;
-  ceFinishKernel<<<grid, kCeThreads, 0, s>>>((bf16*)logits, targets, reinterpret_cast<const float4*>(statsAll), tp, loss, M, V, ld,
+  launchAfter(ceFinishKernel, grid, kCeThreads, 0, s, (bf16*)logits, targets, reinterpret_cast<const float4*>(statsAll), tp, loss, M, V, ld,
                                              vocabOffset, gscale);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
@@ -881,9 +912,9 @@ extern "C" int cocclkAdam(float* master, float* m, float* v, const void* grad, i
   const float bc1 = 1.f - powf(b1, (float)step), bc2 = 1.f - powf(b2, (float)step);
   const int grid = gridForElems(n, 2048);
   if (gradIsBf16)
-    adamKernel<bf16><<<grid, 256, 0, s>>>(master, m, v, (const bf16*)grad, (bf16*)param, n, lr, b1, b2, eps, wd, bc1, bc2, gradScale);
+    launchAfter(adamKernel<bf16>, grid, 256, 0, s, master, m, v, (const bf16*)grad, (bf16*)param, n, lr, b1, b2, eps, wd, bc1, bc2, gradScale);
   else
-    adamKernel<float><<<grid, 256, 0, s>>>(master, m, v, (const float*)grad, (bf16*)param, n, lr, b1, b2, eps, wd, bc1, bc2, gradScale);
+    launchAfter(adamKernel<float>, grid, 256, 0, s, master, m, v, (const float*)grad, (bf16*)param, n, lr, b1, b2, eps, wd, bc1, bc2, gradScale);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
@@ -894,23 +925,23 @@ extern "C" int cocclkSumSq(const void* x, int isBf16, long n, float* out, int ac
                            cudaStream_t s) {
   if (n <= 0) return -1;
   const int grid = cocclkSumSqBlocks(n);
-  if (isBf16) sumSqPartialKernel<bf16><<<grid, 256, 0, s>>>((const bf16*)x, n, scratch);
-  else sumSqPartialKernel<float><<<grid, 256, 0, s>>>((const float*)x, n, scratch);
-  sumFinalKernel<<<1, 256, 0, s>>>(scratch, grid, out, accumulate);
+  if (isBf16) launchAfter(sumSqPartialKernel<bf16>, grid, 256, 0, s, (const bf16*)x, n, scratch);
+  else launchAfter(sumSqPartialKernel<float>, grid, 256, 0, s, (const float*)x, n, scratch);
+  launchAfter(sumFinalKernel, 1, 256, 0, s, scratch, grid, out, accumulate);
   cocclkCountLaunches(2);
   return (int)cudaGetLastError();
 }
 
 extern "C" int cocclkClipCoef(const float* sumsq, float maxNorm, float gradScaleIn, float* coef, float* normOut,
                               cudaStream_t s) {
-  clipCoefKernel<<<1, 1, 0, s>>>(sumsq, maxNorm, gradScaleIn, coef, normOut);
+  launchAfter(clipCoefKernel, 1, 1, 0, s, sumsq, maxNorm, gradScaleIn, coef, normOut);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
 
 extern "C" int cocclkAccumBf16(float* dst, const void* src, long n, int accumulate, cudaStream_t s) {
   if (n <= 0) return -1;
-  accumBf16Kernel<<<gridForElems(n, 2048), 256, 0, s>>>(dst, (const bf16*)src, n, accumulate);
+  launchAfter(accumBf16Kernel, gridForElems(n, 2048), 256, 0, s, dst, (const bf16*)src, n, accumulate);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();
 }
@@ -968,7 +999,7 @@ extern "C" int cocclkColSumNoAlloc(const void* x, float* out, int accumulate, in
   const int by = colSumBlocks(M, N);  // <= kNoAllocRows
   const int rowsPer = (M + by - 1) / by;
   dim3 grid((N / 8 + 31) / 32, by);
-  colSumPartialKernel<<<grid, 256, 0, s>>>((const bf16*)x, scratch, M, N, rowsPer);
+  launchAfter(colSumPartialKernel, grid, 256, 0, s, (const bf16*)x, scratch, M, N, rowsPer);
   launchColReduce(scratch, out, nullptr, N, by, N, N, accumulate, s);
   cocclkCountLaunches(1);
   return (int)cudaGetLastError();

@@ -280,8 +280,8 @@ def test_not_a_number_counts_in_no_maximum(cuda, asym):
 
 @pytest.mark.parametrize("cfg", [C.SDP4BIT_G128, C.ZFP_RATE8], ids=lambda c: c.kind)
 @pytest.mark.parametrize("count", [4099, 8192 * 300 + 5])
-def test_launches_that_overlap_see_one_another(cuda, cfg, count):
-    """Kernels start while the one before them ends: a chain through the same two buffers, each read by one kernel and overwritten
+def test_launches_in_a_chain_see_one_another(cuda, cfg, count):
+    """Back-to-back launches without a wait: a chain through the same two buffers, each read by one kernel and overwritten
     by the next but one, gives what it gives with a wait behind every launch; in a stream and in a graph."""
     x = torch.randn(6, count, device=cuda)
     nb = cfg.encoded_chunk_bytes(count, torch.float32)
