@@ -1097,7 +1097,8 @@ struct ZfpCodec {
   static constexpr int kWords = RATE;
   static constexpr bool kRotated = false;
   static constexpr int kMinBlocks = 2;
-  // The coder is a chain of dependent integer work that neither warps nor registers shorten by much: eight chunks of 4 Mi fp32,
+  // The coder is a chain of dependent integer work that neither warps nor registers shorten by much (CTA counts compared before
+  // several planes went through one look-up; the ranking was not taken again): eight chunks of 4 Mi fp32,
   // encode 72.5 us at rate 8 with four CTAs an SM and 71.3 with three, decode 122.0 and 122.7; rate 4 56.0 and 56.0, 77.2 and
   // 76.2; rate 16 103.5 and 104.2, 189.0 and 186.7 (64 registers spill there: 8 x 4096 values 15.3 against 13.5 us). Sums, which
   // hold a second run: 79.0 and 73.2 at rate 4, 130.2 and 126.3 at 8, 207.1 and 201.5 at 16.
