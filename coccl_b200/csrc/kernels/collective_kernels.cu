@@ -24,6 +24,12 @@ extern "C" int cocclkFusedCollective(const cocclkCollArgs* args, int emulatedRan
   memcpy(&a, args, sizeof(a));
   if (a.nRanks < 1 || a.nRanks > kMaxRanks || a.count <= 0 || a.sliceTiles <= 0) return -1;
   if (emulatedRanks != 1 && emulatedRanks != a.nRanks) return -1;
+  // what the kernel follows without looking: every rank's workspace and flags, and the tensors of the ranks played here
+  if (a.rankBase < 0 || a.rankBase + emulatedRanks > a.nRanks) return -1;
+  for (int r = 0; r < a.nRanks; ++r) {
+    const bool here = r >= a.rankBase && r < a.rankBase + emulatedRanks;
+    if (!a.ws[r] || !a.flags[r] || (here && (!a.in[r] || !a.out[r]))) return -1;
+  }
   if (!tileCodecSupported(a.codec)) return -1;
   switch (a.dtype) {
     case kF32: return launchFusedF32(a, emulatedRanks, maxCtas, stream);

@@ -103,9 +103,11 @@ def emulate_collective(op: str, inputs: list[torch.Tensor], cfg: CodecConfig, *,
     a.epoch = epoch
     a.timeoutNs = int(timeout_ms * 1e6)
     trace = state.get("trace")   # list of int64 [TRACE_MAX_CTAS, 4] tensors, one per rank
-    rows = zip(inputs, outs, state["ws"], state["flags"], state["status"])
+    rows = (inputs, outs, state["ws"], state["flags"], state["status"])
+    if any(len(row) < n for row in rows):
+        raise IndexError(f"{n} ranks, but a state with buffers for {min(map(len, rows))}")
     inp, out, ws, flags, status = a.inp, a.out, a.ws, a.flags, a.status
-    for r, (x, o, w, f, s) in enumerate(rows):
+    for r, (x, o, w, f, s) in enumerate(zip(*rows)):
         assert x.is_contiguous() and x.numel() == numel
         inp[r], out[r], ws[r], flags[r], status[r] = x.data_ptr(), o.data_ptr(), w.data_ptr(), f.data_ptr(), s.data_ptr()
         a.trace[r] = None if trace is None else trace[r].data_ptr()
