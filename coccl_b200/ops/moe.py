@@ -94,6 +94,9 @@ def emulate_dispatch(xs, ids, n_experts, *, capacity=None, state=None, max_ctas=
     topk = ids[0].shape[1]
     dev = xs[0].device
     le = n_experts // n
+    if any(i.numel() < tokens * topk for i in ids[:n]):
+        raise ValueError(f"{tokens} tokens a rank with {topk} choices, got tables of {[tuple(i.shape) for i in ids[:n]]}")
+    alike = all(i.numel() == tokens * topk for i in ids[:n])   # one size serves every rank's layout; longer tables have their own
     capacity = capacity or tokens * topk
     state = _state(state if state is not None else {}, n, dev, ws_bytes(n, capacity, hidden, le))
     a = _base_args(n, tokens, hidden, topk, n_experts, capacity, state, timeout_ms)
@@ -101,7 +104,10 @@ def emulate_dispatch(xs, ids, n_experts, *, capacity=None, state=None, max_ctas=
     for r in range(n):
         assert ids[r].dtype == torch.int32 and n_experts % n == 0
         routed = ids[r].contiguous()
-        pos, counts = torch.empty_like(routed), torch.empty(n_experts, dtype=torch.int32, device=dev)
+        if alike:
+            pos, counts = torch.empty_like(routed), torch.empty(n_experts, dtype=torch.int32, device=dev)
+        else:
+            pos, counts = route_layout(routed, n_experts, n)
         recv = torch.empty(n * capacity, hidden, dtype=torch.bfloat16, device=dev)
         roff = torch.empty(le + 1, dtype=torch.int32, device=dev)   # both written in full by the kernel
         rcnt = torch.empty(n, le, dtype=torch.int32, device=dev)
@@ -110,7 +116,8 @@ def emulate_dispatch(xs, ids, n_experts, *, capacity=None, state=None, max_ctas=
         keep.append((routed, pos, counts))
         recvs.append(recv)
         handles.append(Handle(routed, pos, rcnt, roff, capacity, n_experts))
-    _lib.check(_lib.lib().cocclkMoeLayoutRanks(a, _lib.cur_stream()), "cocclkMoeLayoutRanks")
+    if alike:
+        _lib.check(_lib.lib().cocclkMoeLayoutRanks(a, _lib.cur_stream()), "cocclkMoeLayoutRanks")
     _lib.check(_lib.lib().cocclkMoeDispatch(a, n, max_ctas, _lib.cur_stream()), "cocclkMoeDispatch")
     return recvs, handles, state
 
