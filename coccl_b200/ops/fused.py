@@ -35,7 +35,8 @@ class Branch:
     forward and backward pass is captured into a graph: small products fill a fraction of the GPU and nothing waits for these, yet
     in one stream they stand between the kernels that do wait for one another. All such work of a pass goes through one branch in
     its old order, so every buffer sees its sums in the order of the launched pass. The tensors it reads are kept until `join`:
-    the allocator knows the main stream only and would hand their memory out again."""
+    the allocator knows the main stream only and would hand their memory out again. Leaving the context joins, also on an error: a
+    capture with a stream that has not come back cannot even be ended."""
 
     _of_thread = threading.local()
 
@@ -51,8 +52,13 @@ class Branch:
         self._of_thread.branch = self
         return self
 
-    def __exit__(self, *exc):
+    def __exit__(self, error, *_):
         self._of_thread.branch = None
+        try:
+            self.join(torch.cuda.current_stream(self.stream.device))
+        except RuntimeError:   # of a capture that the error in flight has broken
+            if error is None:
+                raise
 
     def run(self, work, *reads):
         """work() behind what the current stream holds so far, beside what it gets from now on."""
@@ -63,9 +69,11 @@ class Branch:
             return work()
 
     def join(self, stream):
-        if self.used:
-            stream.wait_stream(self.stream)
-        self.keep = []
+        try:
+            if self.used:
+                stream.wait_stream(self.stream)
+        finally:
+            self.keep = []
 
 
 def _accum_param_grad(p: torch.Tensor, g_fp32_or_none, compute):

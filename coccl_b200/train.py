@@ -235,9 +235,8 @@ class MicroBatchGraph:
                 graph.capture_begin(capture_error_mode="thread_local")
                 try:
                     if self.pool_bytes(t.cfg, shape[0] * (shape[1] - 1), True) <= self.MAX_POOL_BYTES:
-                        with fused.Branch(t.device) as branch:
+                        with fused.Branch(t.device):
                             t._micro_batch(tokens, scale)
-                        branch.join(side)
                     else:
                         t._micro_batch(tokens, scale)
                 finally:

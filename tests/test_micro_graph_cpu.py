@@ -101,3 +101,96 @@ def test_size_rule():
     assert MicroBatchGraph.worth_it(small, 192)
     assert not MicroBatchGraph.worth_it(small, 16385)
     assert not MicroBatchGraph.worth_it(GPTConfig(), 4096)
+
+
+class _Streams:
+    """Streams, events and captures of torch.cuda as far as a capture sees them: a stream that has waited for one in a capture is in
+    it too, and has to come back to the stream that the capture began in before that can end."""
+
+    def __init__(self, monkeypatch):
+        outer = self
+        self.current, self.away, self.origin, self.ended = None, set(), None, 0
+
+        class Stream:
+            def __init__(self, device=None):
+                self.device = device
+
+            def wait_stream(self, other):
+                if other is outer.origin or other in outer.away:
+                    outer.away.add(self)
+                if self is outer.origin:
+                    outer.away.discard(other)
+                    outer.away.discard(self)
+
+        class use:
+            def __init__(self, stream):
+                self.stream = stream
+
+            def __enter__(self):
+                self.before, outer.current = outer.current, self.stream
+
+            def __exit__(self, *_):
+                outer.current = self.before
+
+        class Graph:
+            def capture_begin(self, **_):
+                outer.origin = outer.current
+
+            def capture_end(self):
+                outer.origin = None
+                outer.ended += 1
+                if outer.away:
+                    raise RuntimeError("capture ended with a stream that has not joined")
+
+        self.current = Stream()
+        for name, fake in (("Stream", Stream), ("stream", use), ("CUDAGraph", Graph), ("current_stream", lambda device=None: outer.current)):
+            monkeypatch.setattr(torch.cuda, name, fake)
+
+
+@pytest.mark.parametrize("error", [ValueError("in the pass"), KeyboardInterrupt("in the pass"), None], ids=["error", "interrupt", "none"])
+@pytest.mark.parametrize("in_branch", [False, True])
+def test_an_error_inside_a_captured_pass_stays_that_error(monkeypatch, error, in_branch):
+    """The branch of parameter gradients joins whatever happens, so that the capture can be ended and what the caller sees is what went
+    wrong."""
+    from coccl_b200.ops import fused
+    t = _trainer()
+    streams = _Streams(monkeypatch)
+
+    def fail():
+        if error is not None:
+            raise error
+
+    def micro_batch(tokens, scale):
+        branch = fused.Branch.current()
+        branch.run(lambda: None, tokens)
+        if in_branch:
+            branch.run(fail, tokens)
+        fail()
+    monkeypatch.setattr(t, "_micro_batch", micro_batch, raising=False)
+    if error is None:
+        t.micro_graph._capture(t, (2, 9), 1.0)
+    else:
+        with pytest.raises(type(error), match="in the pass"):
+            t.micro_graph._capture(t, (2, 9), 1.0)
+    assert (t.micro_graph.graph is not None) == (error is None)
+    assert streams.ended == 1 and not streams.away and fused.Branch.current() is None and t.micro_graph.enabled
+
+
+def test_a_broken_capture_is_reported_with_its_own_error(monkeypatch):
+    """An error that also breaks the capture: the streams can neither join nor end, and that is what is reported, as ever."""
+    from coccl_b200.ops import fused
+    t = _trainer()
+    streams = _Streams(monkeypatch)
+
+    def micro_batch(tokens, scale):
+        branch = fused.Branch.current()
+        branch.run(lambda: None, tokens)
+
+        def broken(stream):
+            raise RuntimeError("cannot join")
+        monkeypatch.setattr(branch, "join", broken)
+        raise RuntimeError("out of memory")
+    monkeypatch.setattr(t, "_micro_batch", micro_batch, raising=False)
+    with pytest.warns(UserWarning, match="not joined"):
+        t.micro_graph._capture(t, (2, 9), 1.0)
+    assert streams.ended == 1 and t.micro_graph.graph is None and not t.micro_graph.enabled
