@@ -77,9 +77,7 @@ def emulate_collective(op: str, inputs: list[torch.Tensor], cfg: CodecConfig, *,
         assert state is not None and "outs" in state, "all_gather_delta needs state['outs'] from an exact first gather"
         outs = state["outs"]
     else:
-        # the ranks' results side by side in one allocation, each on 16 bytes
-        row = -(-out_numel * x0.element_size() // 16) * 16 // x0.element_size()
-        outs = list(torch.empty((n, row), dtype=dtype, device=dev)[:, :out_numel].unbind(0))
+        outs = [torch.empty(out_numel, dtype=dtype, device=dev) for _ in range(n)]
     if state is None:
         state = {}
     # sizes, and the part of the arguments that a call of the same kind leaves alone (20 us of a small call without them)

@@ -86,3 +86,14 @@ def test_the_library_refuses_arguments_without_a_buffer(recorder, missing, rank)
     args, ranks = recorder.launched[-1]
     getattr(args, missing)[rank] = None
     assert recorder.real.cocclkFusedCollective(args, ranks, 0, None) == -1
+
+
+def test_every_rank_s_result_is_a_tensor_of_its_own(recorder):
+    """Of its own memory (kept, saved or resized by itself) and no view, which autograd would not let a caller change in place."""
+    outs = K.emulate_collective("all_gather", _inputs(4, 1003), C.SDP4BIT_G128)
+    assert all(o._base is None and o.is_contiguous() and o.storage_offset() == 0 and o.untyped_storage().nbytes() == o.nbytes for o in outs)
+    outs[1].zero_()
+    outs[0].resize_(2 * outs[0].numel()).fill_(7.0)
+    assert not outs[1].any()
+    outs[2].mul_(torch.ones_like(outs[2], requires_grad=True))
+    assert outs[2].requires_grad
