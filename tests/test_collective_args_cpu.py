@@ -1,6 +1,8 @@
 """The arguments that `emulate_collective` hands to the kernel library, recorded in its place (no GPU): every rank's entries are
 filled, or the call is refused before anything is launched."""
+import copy
 import ctypes
+import io
 
 import pytest
 import torch
@@ -97,3 +99,53 @@ def test_every_rank_s_result_is_a_tensor_of_its_own(recorder):
     assert not outs[1].any()
     outs[2].mul_(torch.ones_like(outs[2], requires_grad=True))
     assert outs[2].requires_grad
+
+
+def test_a_state_can_be_copied_and_saved(recorder):
+    """It holds buffers and their sizes, which a program may keep with its checkpoints; a copy serves as well as the original."""
+    state = {}
+    K.emulate_collective("reduce_scatter", _inputs(4), C.SDP4BIT_G128, state=state)
+    assert set(state) == {"flags", "status", "ws", "ws_bytes"}
+    file = io.BytesIO()
+    torch.save(state, file)
+    file.seek(0)
+    for other in (copy.deepcopy(state), torch.load(file, weights_only=True)):
+        K.emulate_collective("reduce_scatter", _inputs(4), C.SDP4BIT_G128, state=other)
+        args, _ = recorder.launched[-1]
+        assert args.ws[3] == other["ws"][3].data_ptr() != state["ws"][3].data_ptr()
+
+
+def test_kinds_in_turn_and_what_they_share(recorder):
+    """A call's own values (buffers, epoch, time limit, trace) are in its own arguments only."""
+    kinds = [("reduce_scatter", 4, 64 * 8, C.SDP4BIT_G128, None), ("all_gather", 2, 64, C.MXFP8, 3), ("reduce_scatter", 4, 64 * 8, C.TACO_G128, None)]
+    state, first = {}, []
+    for turn in range(2):
+        for i, (op, n, numel, cfg, tiles) in enumerate(kinds):
+            if turn == 0 and i == 0:
+                state["trace"] = [torch.zeros(8, dtype=torch.int64) for _ in range(4)]
+            xs = _inputs(n, numel)
+            outs = K.emulate_collective(op, xs, cfg, slice_tiles=tiles, epoch=1 + turn, timeout_ms=5.0 + i, state=state)
+            state.pop("trace", None)
+            a, ranks = recorder.launched[-1]
+            alone = K._arguments(K.OP_NAMES[op], n, xs[0].dtype, numel, tiles, None, cfg)[0]
+            for field in ("op", "nRanks", "rankBase", "dtype", "count", "sliceTiles", "slotBytes", "regionBOffset"):
+                assert getattr(a, field) == getattr(alone, field), field
+            assert bytes(a.codec) == bytes(cfg.to_c(xs[0].dtype)) and ranks == n
+            assert a.epoch == 1 + turn and a.timeoutNs == int((5.0 + i) * 1e6)
+            assert [a.inp[r] for r in range(n)] == [x.data_ptr() for x in xs] and [a.out[r] for r in range(n)] == [o.data_ptr() for o in outs]
+            assert (a.trace[0] is not None) == (turn == 0 and i == 0)
+            assert all(a.inp[r] is None for r in range(n, _lib.MAX_RANKS))
+
+
+def test_a_codec_described_by_another_object_is_asked_each_time(recorder):
+    class Described:
+        group = 128
+
+        def to_c(self, dtype):
+            return C.CodecConfig("sdp4bit", 4, self.group).to_c(dtype)
+    cfg, state = Described(), {}
+    for group in (128, 32):
+        cfg.group = group
+        K.emulate_collective("reduce_scatter", _inputs(4), cfg, state=state)
+        args, _ = recorder.launched[-1]
+        assert args.codec.group == group and args.slotBytes == K.slot_bytes(cfg, 128, torch.float32)
