@@ -59,13 +59,13 @@ class CodecConfig:
                           int(self.stochastic), self.param_bytes(dtype), self.seed & 0xFFFFFFFF)
 
     def encoded_chunk_bytes(self, count: int, dtype: torch.dtype) -> int:
-        _, _, g, group_bits, group_params = self.layout(dtype)
+        _, g, group_bits, group_params = self.layout(dtype)
         groups = -(-count // g)
         total = groups * group_bits // 8 + groups * group_params
         return -(-total // 4) * 4
 
     def layout(self, dtype: torch.dtype) -> tuple:
-        """(C struct, the kernels' code of `dtype`, values, payload bits and parameter bytes of a group): what every call needs of
+        """(C struct, values, payload bits and parameter bytes of a group): what every call needs of
         this configuration, which cannot change, worked out once (4 us of the 13 that a small call took on the host). The struct
         is only read."""
         known = self.__dict__.setdefault("_layouts", {})
@@ -73,7 +73,7 @@ class CodecConfig:
         if got is None:
             g = {"mxfp8": 32, "zfp": 4}.get(self.kind, self.group)
             bits = 8 if self.kind in ("mxfp8", "taco") else self.bits
-            got = known[dtype] = (self.to_c(dtype), DTYPE_CODE.get(dtype), g, g * bits, self.param_bytes(dtype))
+            got = known[dtype] = (self.to_c(dtype), g, g * bits, self.param_bytes(dtype))
         return got
 
     def __getstate__(self):   # copies and pickles are the fields
@@ -93,8 +93,9 @@ def encode(x: torch.Tensor, cfg: CodecConfig, chunks: int = 1) -> torch.Tensor:
     count = x.numel() // chunks
     nbytes = cfg.encoded_chunk_bytes(count, x.dtype)
     out = torch.empty((chunks, nbytes), dtype=torch.uint8, device=x.device)
-    c, code = cfg.layout(x.dtype)[:2]
-    rc = _lib.lib().cocclkEncode(x.data_ptr(), out.data_ptr(), count, chunks, count, nbytes, code, c, _lib.cur_stream())
+    c = cfg.layout(x.dtype)[0]
+    rc = _lib.lib().cocclkEncode(x.data_ptr(), out.data_ptr(), count, chunks, count, nbytes, DTYPE_CODE[x.dtype],
+                                 c, _lib.cur_stream())
     _lib.check(rc, "cocclkEncode")
     return out
 
@@ -104,9 +105,9 @@ def decode_reduce(enc: torch.Tensor, cfg: CodecConfig, count: int, dtype: torch.
     """out[j] = sum_i decode(enc[i*chunks + j]) for j < chunks; enc is uint8 [reduce*chunks, chunk_bytes]."""
     assert enc.is_cuda and enc.is_contiguous() and enc.shape[0] == chunks * reduce
     out = torch.empty((chunks, count), dtype=dtype, device=enc.device)
-    c, code = cfg.layout(dtype)[:2]
-    rc = _lib.lib().cocclkDecodeReduce(enc.data_ptr(), out.data_ptr(), count, chunks, reduce, count, enc.shape[1], code, c,
-                                       _lib.cur_stream())
+    c = cfg.layout(dtype)[0]
+    rc = _lib.lib().cocclkDecodeReduce(enc.data_ptr(), out.data_ptr(), count, chunks, reduce, count, enc.shape[1],
+                                       DTYPE_CODE[dtype], c, _lib.cur_stream())
     _lib.check(rc, "cocclkDecodeReduce")
     return out
 

@@ -3,6 +3,7 @@ import copy
 import dataclasses
 import pickle
 
+import pytest
 import torch
 
 from coccl_b200.ops.codec import CodecConfig
@@ -28,3 +29,21 @@ def test_encoded_sizes_of_every_kind():
         cfg = CodecConfig(kind, bits, {"zfp": 4, "mxfp8": 32, "taco": 128}[kind], False, False)
         assert cfg.encoded_chunk_bytes(1000, torch.float32) == n
     assert CodecConfig("zfp", 5, 4, False, False).encoded_chunk_bytes(1002, torch.float32) == -(-(251 * 20 // 8) // 4) * 4
+
+
+def test_a_type_that_the_kernels_do_not_know_is_a_key_error(monkeypatch):
+    """As a look-up of the type gives it, before anything is launched; sizes are known for every type."""
+    from coccl_b200 import _lib
+    from coccl_b200.ops import codec as C
+    monkeypatch.setattr(_lib, "lib", lambda: type("", (), {"__getattr__": lambda self, name: lambda *a: 1 / 0})())
+    monkeypatch.setattr(_lib, "cur_stream", lambda: 0)
+
+    class OnGpu(torch.Tensor):
+        is_cuda = True
+    x = torch.zeros(256, dtype=torch.float64).as_subclass(OnGpu)
+    enc = torch.zeros(1, 144, dtype=torch.uint8).as_subclass(OnGpu)
+    assert C.SDP4BIT_G128.encoded_chunk_bytes(256, torch.float64) == 128 + 2 * 8
+    with pytest.raises(KeyError):
+        C.encode(x, C.SDP4BIT_G128, 1)
+    with pytest.raises(KeyError):
+        C.decode(enc, C.SDP4BIT_G128, 256, torch.float64, 1)
