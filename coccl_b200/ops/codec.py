@@ -19,8 +19,13 @@ DTYPE_CODE = {torch.float32: 0, torch.float16: 1, torch.bfloat16: 2}
 KIND_SDP4BIT, KIND_MXFP8, KIND_TACO, KIND_ZFP = 0, 1, 3, 4
 
 
+class _Layouts:
+    """A place beside a configuration's fields: what is kept there is in neither `vars` nor any comparison."""
+    __slots__ = ("_layouts",)
+
+
 @dataclass(frozen=True)
-class CodecConfig:
+class CodecConfig(_Layouts):
     kind: str = "sdp4bit"          # "sdp4bit" | "mxfp8" | "taco" | "zfp"
     bits: int = 4                  # sdp4bit: 4 | 8; zfp: the rate in bits per value (4 | 8 | 16); taco: 8
     group: int = 128               # elements per quantisation group (mxfp8: 32; zfp: 4, one block; taco: 32..512)
@@ -65,10 +70,13 @@ class CodecConfig:
         return -(-total // 4) * 4
 
     def layout(self, dtype: torch.dtype) -> tuple:
-        """(C struct, values, payload bits and parameter bytes of a group): what every call needs of
-        this configuration, which cannot change, worked out once (4 us of the 13 that a small call took on the host). The struct
-        is only read."""
-        known = self.__dict__.setdefault("_layouts", {})
+        """(C struct, values, payload bits and parameter bytes of a group): what every call needs of this configuration, which
+        cannot change, worked out once. The struct is only read."""
+        try:
+            known = self._layouts
+        except AttributeError:
+            known = {}
+            object.__setattr__(self, "_layouts", known)
         got = known.get(dtype)
         if got is None:
             g = {"mxfp8": 32, "zfp": 4}.get(self.kind, self.group)
@@ -77,7 +85,7 @@ class CodecConfig:
         return got
 
     def __getstate__(self):   # copies and pickles are the fields
-        return {k: v for k, v in self.__dict__.items() if k != "_layouts"}
+        return dict(self.__dict__)
 
 
 SDP4BIT_G128 = CodecConfig("sdp4bit", 4, 128, False, True)

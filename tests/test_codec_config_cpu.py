@@ -31,6 +31,16 @@ def test_encoded_sizes_of_every_kind():
     assert CodecConfig("zfp", 5, 4, False, False).encoded_chunk_bytes(1002, torch.float32) == -(-(251 * 20 // 8) // 4) * 4
 
 
+def test_calls_leave_a_configuration_s_fields_alone():
+    """`vars` are the fields, before and after a call: they build an equal configuration, and snapshots of them stay equal."""
+    cfg = CodecConfig("taco", 8, 64, False, False)
+    before = dict(vars(cfg))
+    cfg.encoded_chunk_bytes(1000, torch.float32)
+    assert vars(cfg) == before == dataclasses.asdict(cfg)
+    assert CodecConfig(**vars(cfg)) == cfg
+    assert cfg.layout(torch.float32)[0] is cfg.layout(torch.float32)[0]
+
+
 def test_a_type_that_the_kernels_do_not_know_is_a_key_error(monkeypatch):
     """As a look-up of the type gives it, before anything is launched; sizes are known for every type."""
     from coccl_b200 import _lib
