@@ -180,3 +180,75 @@ def test_gradients_that_autograd_hands_over_are_not_left_to_a_capture(cuda):
         ga, gb = a.stage.wte.main_grad, b.stage.wte.main_grad
         assert gb.norm() > 0 and (ga - gb).norm() <= 3e-2 * gb.norm(), step
     assert a.micro_graph.graph is None
+
+
+@pytest.mark.parametrize("arch", ["gpt", "llama"])
+def test_every_gradient_of_a_replayed_step(cuda, arch):
+    """Parameter by parameter, from equal parameters: what the backward pass forms ahead of its first attention (head, last norm, the
+    last layer's second half) bit for bit, the others up to the order of the attention's atomic sums."""
+    a, b = _pair(arch)
+    for step in range(5):
+        a.stage.store.flat_param.copy_(b.stage.store.flat_param)
+        a.train_step(_tokens(step))
+        b.train_step(_tokens(step))
+        if step < 2:
+            continue
+        assert a.micro_graph.graph is not None
+        ours = dict(a.stage.named_parameters())
+        for name, p in b.stage.named_parameters():
+            got, want = ours[name].main_grad, p.main_grad
+            assert want.norm() > 0, name
+            if name.startswith(("lnf", "lm_head", "layers.1.fc", "layers.1.gate", "layers.1.up", "layers.1.w_gate", "layers.1.down", "layers.1.ln2")):
+                assert torch.equal(got, want), (step, name)
+            else:
+                assert (got - want).norm() <= 2e-2 * want.norm(), (step, name)
+
+
+def test_a_bound_on_the_pool_leaves_the_branch_out(cuda, monkeypatch):
+    """Between the two sizes of the pool the graph is captured in one stream, with the same gradients."""
+    from coccl_b200.ops import fused
+    from coccl_b200.train import MicroBatchGraph
+    a, b = _pair("gpt")
+    n = 2 * 96
+    small, large = (MicroBatchGraph.pool_bytes(a.cfg, n, branch) for branch in (False, True))
+    monkeypatch.setattr(MicroBatchGraph, "MAX_POOL_BYTES", (small + large) // 2)
+    made = []
+    init = fused.Branch.__init__
+
+    def counted(self, device):
+        made.append(device)
+        init(self, device)
+    monkeypatch.setattr(fused.Branch, "__init__", counted)
+    for bound, branches in (((small + large) // 2, 0), (large, 1)):
+        monkeypatch.setattr(MicroBatchGraph, "MAX_POOL_BYTES", bound)
+        a.micro_graph._drop()
+        for step in range(3):
+            a.stage.store.flat_param.copy_(b.stage.store.flat_param)
+            a.train_step(_tokens(step))
+            b.train_step(_tokens(step))
+        assert a.micro_graph.graph is not None and len(made) == branches
+        ga, gb = a.stage.store.flat_grad, b.stage.store.flat_grad
+        assert (ga - gb).norm() <= 2e-2 * gb.norm()
+
+
+def test_an_error_inside_a_captured_pass_reaches_the_caller(cuda):
+    """On the host, behind work of the gradients' branch; the next steps are launched and captured as if nothing had been."""
+    from coccl_b200.ops import fused
+    from coccl_b200.train import Trainer
+    a, b = _pair("gpt")
+
+    def fail(tokens, scale):
+        Trainer._micro_batch(a, tokens, scale)
+        assert fused.Branch.current().used
+        raise ValueError("inside the pass")
+    for step in range(5):
+        if step == 2:
+            a._micro_batch = fail
+            with pytest.raises(ValueError, match="inside the pass"):
+                a.micro_graph._capture(a, (2, 97), 1.0)
+            del a._micro_batch
+            assert a.micro_graph.graph is None and a.micro_graph.enabled
+        la, lb = a.train_step(_tokens(step)).item(), b.train_step(_tokens(step)).item()
+        assert abs(la - lb) <= 2e-3 * abs(lb), step
+    assert a.micro_graph.graph is not None
+    a.check_health()
