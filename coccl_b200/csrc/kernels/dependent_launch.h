@@ -7,6 +7,10 @@
 // this must therefore call it. All CTAs of a kernel have started before any of the next one does, so nothing can be held up.
 // Launched in the ordinary way both calls do nothing.
 //
+// What an earlier kernel of the stream may have written is read with loadOrdered (common.cuh) or plain dereferences, behind
+// awaitPrevious(). Loads that take memory to be read-only for the kernel's whole life (__ldg, ld.global.nc, const pointers with
+// __restrict__) are not ordered by the wait: the compiler may move them ahead of it, and that life begins while earlier kernels write.
+//
 // The trainers' short kernels and small GEMMs are launched like this: a chain of them is bound by launch latency, and a replayed
 // training step of two layers, 512 wide, takes 666 us instead of 750 (steps 4096 wide: 17.4 against 17.5 ms and 18.39 against 18.37, no
 // difference). The codec kernels are not. They fill the chip for tens of microseconds with a fixed share of the tiles for

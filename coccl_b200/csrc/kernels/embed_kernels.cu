@@ -27,7 +27,7 @@ __global__ void __launch_bounds__(256) embedOrderKernel(const long* ids, int4* p
   const int t = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= T) return;
   // the low words: valid ids have no others
-  auto idOf = [&](int i) { return __ldg(reinterpret_cast<const int*>(ids + i)); };
+  auto idOf = [&](int i) { return *(reinterpret_cast<const int*>(ids) + 2L * i); };
   const int id = idOf(t), strip = t & ~31;
   int rank = 0, earlier = 0, equal = 0;
 #pragma unroll 4
@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kEmbThreads, 6) embedRowsKernel(const bf16* dy
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int k = i + 2 * u;
-        raw[u] = k < end ? __ldg(reinterpret_cast<const uint4*>(dy + (long)places[k].x * H + col)) : make_uint4(0, 0, 0, 0);
+        raw[u] = k < end ? loadOrdered(dy + (long)places[k].x * H + col) : make_uint4(0, 0, 0, 0);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {

@@ -201,7 +201,7 @@ gemmSmallKernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         *reinterpret_cast<uint4*>(p) = make_uint4(o[0], o[1], o[2], o[3]);
       };
       if (g.epi == GEMM_EPI_BIAS || g.epi == GEMM_EPI_BIAS_GELU) {
-        const uint4 bw = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(g.bias) + col));
+        const uint4 bw = *reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(g.bias) + col);
         const uint32_t w[4] = {bw.x, bw.y, bw.z, bw.w};
 #pragma unroll
         for (int j = 0; j < 4; ++j) {

@@ -66,10 +66,10 @@ __global__ void __launch_bounds__(256) rotateKernel(const RotateArgs a) {
     float t[8];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      unpack8(__ldg(reinterpret_cast<const uint4*>(a.qw + h * H2) + slot), t);
+      unpack8(loadOrdered(reinterpret_cast<const uint4*>(a.qw + h * H2) + slot), t);
 #pragma unroll
       for (int i = 0; i < 8; ++i) wq[8 * h + i] = t[i];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(a.kw + h * H2) + slot), t);
+      unpack8(loadOrdered(reinterpret_cast<const uint4*>(a.kw + h * H2) + slot), t);
 #pragma unroll
       for (int i = 0; i < 8; ++i) wk[8 * h + i] = t[i];
     }
@@ -94,12 +94,12 @@ __global__ void __launch_bounds__(256) rotateKernel(const RotateArgs a) {
       uint4 lo = make_uint4(0, 0, 0, 0), hi = lo, glo = lo, ghi = lo;
       if (valid) {
         if (!BWD || (NORM && !isV)) {
-          lo = __ldg(reinterpret_cast<const uint4*>(a.qkv + packed));
-          hi = __ldg(reinterpret_cast<const uint4*>(a.qkv + packed + H2));
+          lo = loadOrdered(reinterpret_cast<const uint4*>(a.qkv + packed));
+          hi = loadOrdered(reinterpret_cast<const uint4*>(a.qkv + packed + H2));
         }
         if (BWD) {
-          glo = __ldg(reinterpret_cast<const uint4*>(split));
-          ghi = __ldg(reinterpret_cast<const uint4*>(split + H2));
+          glo = loadOrdered(reinterpret_cast<const uint4*>(split));
+          ghi = loadOrdered(reinterpret_cast<const uint4*>(split + H2));
         }
       }
       float x[16];
@@ -213,9 +213,9 @@ __global__ void __launch_bounds__(256) swigluKernel(const bf16* z, const bf16* d
   for (int row = blockIdx.y; row < M; row += gridDim.y) {
     const uint4* zr = reinterpret_cast<const uint4*>(z + (long)row * 2 * F);
     float g[8], u[8], d[8], a[8], b[8];
-    const uint4 rg = __ldg(zr + v), ru = __ldg(zr + nvec + v);
+    const uint4 rg = loadOrdered(zr + v), ru = loadOrdered(zr + nvec + v);
     uint4 rd = make_uint4(0, 0, 0, 0);
-    if (BWD) rd = __ldg(reinterpret_cast<const uint4*>(dy + (long)row * F) + v);
+    if (BWD) rd = loadOrdered(reinterpret_cast<const uint4*>(dy + (long)row * F) + v);
     unpack8(rg, g);
     unpack8(ru, u);
     unpack8(rd, d);

@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(kLnThreads) normBwdKernel(const bf16* dy, cons
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
     const int vi = threadIdx.x + i * blockDim.x;
-    gm[i] = vi < nvec ? __ldg(reinterpret_cast<const uint4*>(gamma) + vi) : make_uint4(0, 0, 0, 0);
+    gm[i] = vi < nvec ? loadOrdered(reinterpret_cast<const uint4*>(gamma) + vi) : make_uint4(0, 0, 0, 0);
     nd[i] = nx[i] = nr[i] = make_uint4(0, 0, 0, 0);
 #pragma unroll
     for (int j = 0; j < 8; ++j) { dg[i][j] = 0.f; if (!RMS) db[i][j] = 0.f; }
@@ -164,9 +164,9 @@ __global__ void __launch_bounds__(kLnThreads) normBwdKernel(const bf16* dy, cons
     for (int i = 0; i < NV; ++i) {
       const int vi = threadIdx.x + i * blockDim.x;
       if (vi < nvec) {
-        nd[i] = __ldg(reinterpret_cast<const uint4*>(dy) + base + vi);
-        nx[i] = __ldg(reinterpret_cast<const uint4*>(x) + base + vi);
-        if (dres) nr[i] = __ldg(reinterpret_cast<const uint4*>(dres) + base + vi);
+        nd[i] = loadOrdered(reinterpret_cast<const uint4*>(dy) + base + vi);
+        nx[i] = loadOrdered(reinterpret_cast<const uint4*>(x) + base + vi);
+        if (dres) nr[i] = loadOrdered(reinterpret_cast<const uint4*>(dres) + base + vi);
       }
     }
     if (!RMS) nmu = mean[row];
@@ -261,8 +261,8 @@ __global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf1
     for (int i = 0; i < kLnWideVec; ++i) {
       const int vi = threadIdx.x + i * kLnWideThreads;
       if (vi < nvec) {
-        nd[i] = __ldg(reinterpret_cast<const uint4*>(dy) + base + vi);
-        nx[i] = __ldg(reinterpret_cast<const uint4*>(x) + base + vi);
+        nd[i] = loadOrdered(reinterpret_cast<const uint4*>(dy) + base + vi);
+        nx[i] = loadOrdered(reinterpret_cast<const uint4*>(x) + base + vi);
       }
     }
     if (!RMS) nmu = mean[row];
@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf1
       const int vi = threadIdx.x + i * kLnWideThreads;
       cd[i] = nd[i];
       cx[i] = nx[i];
-      if (dres && vi < nvec) cr[i] = __ldg(reinterpret_cast<const uint4*>(dres) + base + vi);
+      if (dres && vi < nvec) cr[i] = loadOrdered(reinterpret_cast<const uint4*>(dres) + base + vi);
     }
     const float mu = nmu, rs = nrs;
     if (row + (int)gridDim.x < M) fetch(row + gridDim.x);
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf1
         float d[8], xv[8], g[8], p[8];
         unpackBf16x8(cd[i], d);
         unpackBf16x8(cx[i], xv);
-        unpackBf16x8(__ldg(gv + vi), g);
+        unpackBf16x8(loadOrdered(gv + vi), g);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const float xh = RMS ? xv[j] * rs : (xv[j] - mu) * rs, t = d[j] * g[j];
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(kLnWideThreads, 1) normBwdWideKernel(const bf1
         float d[8], xv[8], g[8], r[8], o[8];
         unpackBf16x8(cd[i], d);
         unpackBf16x8(cx[i], xv);
-        unpackBf16x8(__ldg(gv + vi), g);
+        unpackBf16x8(loadOrdered(gv + vi), g);
         if (dres) unpackBf16x8(cr[i], r);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
