@@ -15,7 +15,8 @@
 // training step of two layers, 512 wide, takes 666 us instead of 750 (steps 4096 wide: 17.4 against 17.5 ms and 18.39 against 18.37, no
 // difference). The codec kernels are not. They fill the chip for tens of microseconds with a fixed share of the tiles for
 // each CTA, and CTAs that move in early share an SM with the last ones of the kernel before: a stochastic 4-bit encode + sum of
-// 8 x 8 Mi fp32 took 84.7 us instead of 77.3, although the shorter codec chains gained (49.9 -> 45.5 us for 8 x 5,000,003 bf16).
+// 8 x 8 Mi fp32 took 84.7 us instead of 77.3, although the shorter codec chains gained (49.9 -> 45.5 us for 8 x 5,000,003 bf16). For
+// the same reason launchIfEarly leaves out norm backwards and rotations of several rows a CTA.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -26,7 +27,8 @@ __device__ __forceinline__ void releaseNext() { asm volatile("griddepcontrol.lau
 __device__ __forceinline__ void awaitPrevious() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class... Params, class... Args>
-static inline cudaError_t launchAfter(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+static inline cudaError_t launchIfEarly(bool early, void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                        Args... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -36,8 +38,12 @@ static inline cudaError_t launchAfter(void (*kern)(Params...), dim3 grid, dim3 b
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = early ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<Params>(args)...);
+}
+template <class... Params, class... Args>
+static inline cudaError_t launchAfter(void (*kern)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+  return launchIfEarly(true, kern, grid, block, smem, stream, args...);
 }
 #endif
 

@@ -65,6 +65,8 @@ __global__ void __launch_bounds__(256) embedOrderKernel(const long* ids, int4* p
 // the CTA that finds all of them there, whichever it is, adds them up in order: the result does not depend on scheduling.
 // One CTA for a whole run summed 16384 equal ids in 1.5 ms (512 wide) and 2.4 ms (4096 wide), in pieces they take 45 and 97 us.
 // 40 registers keep six CTAs on an SM, which is what ids that differ need (50304 x 4096, 4096 of them: 38 us, 50 with 51 registers).
+// No dependent launch: most CTAs leave after one look at their place, and the two instructions of such a launch cost each of them more
+// than the early start gains (4096 x 4096, equal ids: 39.0 us with them, 33.2 without; 512 x 512: 4.9 and 4.8).
 //
 // parts: a row per window of kEmbPiece places and kind of piece (first of its run or not). Two pieces of one kind, both of long
 // runs, never start in the same window: later pieces of a run are kEmbPiece apart, a run's later piece and the next run's lie
@@ -72,8 +74,6 @@ __global__ void __launch_bounds__(256) embedOrderKernel(const long* ids, int4* p
 constexpr int kEmbPiece = 64;
 __global__ void __launch_bounds__(kEmbThreads, 6) embedRowsKernel(const bf16* dy, const int4* places, float* parts,
                                                                unsigned* counters, float* grad, int T, int H, long vocab) {
-  releaseNext();
-  awaitPrevious();
   __shared__ float other[kEmbLanes][9];
   __shared__ bool last;
   const int i0 = blockIdx.x;
@@ -210,7 +210,7 @@ extern "C" int cocclkEmbedBwd(const void* dy, const long* ids, void* scratch, fl
   int4* places = (int4*)b;
   unsigned* counters = (unsigned*)(b + L.countersAt);
   launchAfter(embedOrderKernel, (T + 7) / 8, 256, 0, s, ids, places, counters, (int)(L.windows * L.colBlocks), T);
-  launchAfter(embedRowsKernel, dim3((unsigned)T, (unsigned)L.colBlocks), kEmbThreads, 0, s, (const bf16*)dy, places, (float*)(b + L.partsAt), counters,
+  embedRowsKernel<<<dim3((unsigned)T, (unsigned)L.colBlocks), kEmbThreads, 0, s>>>((const bf16*)dy, places, (float*)(b + L.partsAt), counters,
                                                                             grad, T, H, vocab);
   cocclkCountLaunches(2);
   return (int)cudaGetLastError();

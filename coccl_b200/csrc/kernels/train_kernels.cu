@@ -796,7 +796,12 @@ static int launchNormBwd(const void* dy, const void* x, const float* mean, const
   if (H % 8 || H <= 0 || H > kLnThreads * kLnMaxVec * 8 || M <= 0) return -1;
   int grid = cocclkLayerNormBwdGrid(M);
   const int threads = normThreads(H), nv = (H / 8 + threads - 1) / threads;
-#define NORM_BWD(NV) launchAfter(normBwdKernel<NV, RMS>, grid, threads, 0, s, (const bf16*)dy, (const bf16*)x, mean, rstd, \
+  // Many rows for each of a fixed number of CTAs: those that move in early share an SM with the last ones of the kernel before, and the
+  // slowest SM counts (in a graph of such calls, early and in turn: 4096 x 1024 LayerNorm 19.0 and 14.7 us, 4096 x 2048 RMSNorm 21.9
+  // and 16.8, 1024 x 768 7.8 and 7.2). Few rows gain (512 x 512: 5.1 and 5.5 us), and so do wide ones, which take an SM's
+  // registers anyway (4096 x 4096 with a residual: 36.2 and 37.0).
+  const bool early = M <= 2 * grid || H > 2048;
+#define NORM_BWD(NV) launchIfEarly(early, normBwdKernel<NV, RMS>, grid, threads, 0, s, (const bf16*)dy, (const bf16*)x, mean, rstd, \
       (const bf16*)gamma, (const bf16*)dres, (bf16*)dx, scratch, M, H)
   if (nv <= 1) NORM_BWD(1);
   else if (nv <= 2) NORM_BWD(2);
