@@ -290,7 +290,7 @@ struct SdpCodec {
   // parameters do not fit 80 registers beside a run: 35.6 (three) and 39.8 (four), 28.9 (two) and 32.8 (three).
   static constexpr int kEncodeBlocks = SMALLG ? 3 : 4, kDecodeBlocks = BITS == 8 && SMALLG && ASYM ? 2 : 3, kSumBlocks = 2;
   static constexpr bool kExchanges = false;   // runs of neighbouring lanes through the window
-  static constexpr bool kEncodeAhead = !(SMALLG && BITS == 8);   // collective_kernels.cuh
+  static constexpr bool kEncodeAhead = !SMALLG;   // collective_kernels.cuh: kEncodeStages
   static constexpr int kSmemFloats = 8; // shared scratch every kernel passes as `sm` (group reductions wider than a warp)
   static __device__ __forceinline__ void initShared(float*) {}
   static constexpr uint32_t kSignBits = BITS == 4 ? 0x88888888u : 0x80808080u;

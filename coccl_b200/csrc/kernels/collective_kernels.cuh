@@ -72,7 +72,7 @@ __device__ __forceinline__ unsigned int* flagPtr(unsigned int* base, int region,
 // Stages of raw values: for codecs that are bound by instructions the next tile's are on their way to shared memory while this one
 // is encoded, except for fp32, where the loads alone take 0.95 of the copy rate with four CTAs an SM and a second stage leaves
 // room for three (4 bits, groups of 128, 8 x 8 Mi: fp32 48.1 us with one stage, 52.9 with two; bf16 38.5 and 35.6; 8 bits in
-// groups of 8, bound by stores: bf16 63.7 and 84.3).
+// groups of 8, bound by stores: bf16 63.7 and 84.3; 4 bits in groups of 8: 53.9 and 71.7).
 template <typename T, class Codec>
 constexpr int kEncodeStages = sizeof(T) == 2 && Codec::kEncodeAhead ? 2 : 1;
 
