@@ -1038,11 +1038,12 @@ struct TacoCodec {
       sumBatches<E, ALIGN, 2>(r, L.groups, stride, n, mul, (c.aux & 1) != 0, acc);
       sumBatches<E, ALIGN, 1>(r, L.groups, stride, n, mul, (c.aux & 1) != 0, acc);
     };
+    const uintptr_t address = reinterpret_cast<uintptr_t>(base) | (uintptr_t)stride;
     auto byAlign = [&](auto lanesTag) {   // four lanes' places are eight bytes, others' whole vectors
-      constexpr int WIDE = decltype(lanesTag)::value == 4 ? 8 : 16;
-      const bool wide = aligned || (WIDE == 8 && ((reinterpret_cast<uintptr_t>(base) | (uintptr_t)stride) & 7u) == 0);
-      if (wide) go(lanesTag, std::integral_constant<int, WIDE>{});
-      else go(lanesTag, std::integral_constant<int, 4>{});
+      constexpr int E = decltype(lanesTag)::value;
+      if (E != 4 && aligned) go(lanesTag, std::integral_constant<int, 16>{});
+      else if (E != 1 && (address & 7u) == 0) go(lanesTag, std::integral_constant<int, 8>{});
+      else go(lanesTag, std::integral_constant<int, 4>{});   // of one lane: 32 bytes, as their address allows
     };
     if (spread) byLanes(c, byAlign);
     else byAlign(std::integral_constant<int, 1>{});
@@ -1058,9 +1059,10 @@ struct TacoCodec {
     if (elem >= L.payloadBytes || !COCCL_CHUNK_RANGE_OK(TacoCodec, L, c, elem, 2)) return r;
     byLanes(c, [&](auto n) {
       constexpr int E = decltype(n)::value;
-      constexpr int WIDE = E == 4 ? 8 : 16;
       const uint8_t* p = base + placesAt<E>(elem);
-      if ((reinterpret_cast<uintptr_t>(base) & (WIDE - 1)) == 0) loadPlaces<E, WIDE>(p, r.w);
+      const uintptr_t address = reinterpret_cast<uintptr_t>(base);
+      if (E != 4 && (address & 15u) == 0) loadPlaces<E, 16>(p, r.w);
+      else if (E != 1 && (address & 7u) == 0) loadPlaces<E, 8>(p, r.w);
       else loadPlaces<E, 4>(p, r.w);
     });
     const float* ps = reinterpret_cast<const float*>(base + L.payloadBytes) + (elem >> groupShift(c));
