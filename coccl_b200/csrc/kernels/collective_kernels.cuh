@@ -429,6 +429,38 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKern
   }
 }
 
+// out chunk j = decode(in chunk j): one copy (all-gather, all-to-all), for codecs with direct sums. The next tile's words are loaded
+// before this one is transformed and stored (4 bits, groups of 128, rotated: 8 x 8 Mi bf16 40.3 -> 33.0 us, 8 x 5,000,003 29.4 ->
+// 23.9 us). A kernel of its own: in one with the sums' code both spilled (TACO fp32 88 bytes, asymmetric 4 bits 28).
+template <typename T, class Codec>
+__global__ void __launch_bounds__(kTileThreads, Codec::kDecodeBlocks) decodeKernel(const CodecArgs a) {
+  __shared__ TileStage<T> stage;
+  __shared__ __align__(16) float sm[Codec::kSmemFloats];
+  Codec::initShared(sm);
+  __syncthreads();
+  const ChunkLayout L = makeChunkLayout(a.codec, a.count, 4);
+  TileWalk w(a.count, a.chunks);
+  Along<const uint8_t> src(reinterpret_cast<const uint8_t*>(a.in), a.encStrideIn, 0, w);
+  Along<T> dst(reinterpret_cast<T*>(a.out), a.rawPitch, kTileElems, w);
+  auto fetch = [&] { return Codec::ahead(src.p, L, a.codec, (long)w.t * kTileElems + (long)threadIdx.x * kElemsPerThread); };
+  typename Codec::Ahead r;
+  if (w.more()) r = fetch();
+  while (w.more()) {
+    T* tile = dst.p;
+    const long left = L.count - (long)w.t * kTileElems;
+    float acc[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) acc[i] = 0.f;
+    Codec::addAhead(r, a.codec, Codec::finishScale(a.codec), acc);
+    w.next();
+    src.next(w);
+    dst.next(w);
+    if (w.more()) r = fetch();
+    Codec::finish(acc, a.codec, TileIO<T>::window(stage));
+    TileIO<T>::storeTile(tile, left, TileIO<T>::fast(tile, left), stage, acc);
+  }
+}
+
 // out chunk j = sum_{i<reduce} decode(in chunk i*chunks + j)
 template <typename T, class Codec, int BLOCKS>
 __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const CodecArgs a) {
@@ -440,30 +472,6 @@ __global__ void __launch_bounds__(kTileThreads, BLOCKS) decodeReduceKernel(const
   TileWalk w(a.count, a.chunks);
   Along<const uint8_t> src(reinterpret_cast<const uint8_t*>(a.in), a.encStrideIn, 0, w);
   Along<T> dst(reinterpret_cast<T*>(a.out), a.rawPitch, kTileElems, w);
-  if constexpr (HasDirectSums<Codec>::value) {
-    // One copy (all-gather, all-to-all): the next tile's words are loaded before this one is transformed and stored (4 bits,
-    // groups of 128, rotated: 8 x 8 Mi bf16 40.3 -> 33.0 us, 8 x 5,000,003 29.4 -> 23.9 us).
-    if (a.reduce == 1) {
-      auto fetch = [&] { return Codec::ahead(src.p, L, a.codec, (long)w.t * kTileElems + (long)threadIdx.x * kElemsPerThread); };
-      typename Codec::Ahead r;
-      if (w.more()) r = fetch();
-      while (w.more()) {
-        T* tile = dst.p;
-        const long left = L.count - (long)w.t * kTileElems;
-        float acc[32];
-#pragma unroll
-        for (int i = 0; i < 32; ++i) acc[i] = 0.f;
-        Codec::addAhead(r, a.codec, Codec::finishScale(a.codec), acc);
-        w.next();
-        src.next(w);
-        dst.next(w);
-        if (w.more()) r = fetch();
-        Codec::finish(acc, a.codec, TileIO<T>::window(stage));
-        TileIO<T>::storeTile(tile, left, TileIO<T>::fast(tile, left), stage, acc);
-      }
-      return;
-    }
-  }
   for (; w.more(); w.next(), src.next(w), dst.next(w)) {
     const long e0 = (long)w.t * kTileElems, left = L.count - e0;
     const long e = e0 + (long)threadIdx.x * kElemsPerThread;

@@ -310,3 +310,24 @@ def test_launches_in_a_chain_see_one_another(cuda, cfg, count):
     for _ in range(3):
         graph.replay()
         assert all(torch.equal(a, b) for a, b in zip(outs, want))
+
+
+@pytest.mark.parametrize("cfg", [C.SDP4BIT_G128, C.CodecConfig("sdp4bit", 4, 128, True, True), C.CodecConfig("sdp4bit", 8, 128, False, True),
+                                 C.CodecConfig("sdp4bit", 4, 8, False, False), C.MXFP8, *(C.CodecConfig("taco", 8, g, False, False) for g in (32, 64, 128, 512))],
+                         ids=lambda c: f"{c.kind}{c.bits}g{c.group}{'a' if c.asym else 's'}")
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("chunks,count", [(3, 8192 * 3 + 512), (1, 512), (600, 8192)])
+def test_one_copy_decodes_alike_wherever_it_is_put(cuda, cfg, dtype, chunks, count):
+    """Aligned fp32 goes through another kernel than everything else: the same values, bit for bit, one element further on."""
+    torch.manual_seed(count)
+    x = torch.randn(chunks * count, device=cuda).to(dtype)
+    enc = C.encode(x, cfg, chunks)
+    room = torch.full((chunks * count + 16,), float("nan"), dtype=dtype, device=cuda)
+    want = C.decode(enc, cfg, count, dtype, chunks).reshape(-1)
+    for first in (0, 1, 3):
+        out = room[first:first + chunks * count].fill_(float("nan"))
+        _lib.check(_lib.lib().cocclkDecodeReduce(enc.data_ptr(), out.data_ptr(), count, chunks, 1, count, enc.shape[1], C.DTYPE_CODE[dtype],
+                                                 cfg.to_c(dtype), _lib.cur_stream()), "cocclkDecodeReduce")
+        assert torch.equal(out, want), first
+        assert room[first + chunks * count:].isnan().all() and room[:first].isnan().all()
+        room.fill_(float("nan"))
