@@ -113,13 +113,15 @@ def emulate_collective(op: str, inputs: list[torch.Tensor], cfg: CodecConfig, *,
     a.timeoutNs = int(timeout_ms * 1e6)
     trace = state.get("trace")   # list of int64 [TRACE_MAX_CTAS, 4] tensors, one per rank
     rows = (inputs, outs, state["ws"], state["flags"], state["status"])
-    if any(len(row) < n for row in rows):
+    if min(map(len, rows)) < n:
         raise IndexError(f"{n} ranks, but a state with buffers for {min(map(len, rows))}")
     inp, out, ws, flags, status = a.inp, a.out, a.ws, a.flags, a.status
     for r, (x, o, w, f, s) in enumerate(zip(*rows)):
         assert x.is_contiguous() and x.numel() == numel
         inp[r], out[r], ws[r], flags[r], status[r] = x.data_ptr(), o.data_ptr(), w.data_ptr(), f.data_ptr(), s.data_ptr()
-        a.trace[r] = None if trace is None else trace[r].data_ptr()
+    if trace is not None:
+        for r in range(n):
+            a.trace[r] = trace[r].data_ptr()
     rc = _lib.lib().cocclkFusedCollective(a, n, max_ctas, _lib.cur_stream())
     _lib.check(rc, f"cocclkFusedCollective({op})")
     return outs
