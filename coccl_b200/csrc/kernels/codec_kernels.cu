@@ -84,10 +84,10 @@ extern "C" int cocclkDecodeReduce(const void* in, void* out, long count, long ch
   const long tiles = (count + kTileElems - 1) / kTileElems;
   bool ok = dispatchCodec(a.codec, [&](auto codecTag) {
     using C = decltype(codecTag);
-    // Sums hold the words of several copies in flight and are faster with the registers of one CTA an SM fewer (8 x 262,147 bf16:
-    // 4 bits, groups of 128 6.4 -> 5.9 us, asymmetric groups of 16 8.3 -> 5.8, TACO 7.5 -> 6.6), unless that means one more round
-    // of tiles (8 x 3,000,008 fp16 TACO, 367 tiles on 296 places: 13.2 us, on 444 10.5) or, for 4-bit digits in groups of 32 and
-    // more, more than one round (8 x 4 Mi bf16, 512 tiles: 12.9 us, 12.5 with three). ZFP, integer work throughout: always.
+    // Sums hold the words of several copies in flight and are faster with the registers of one CTA an SM fewer (8 x 4 Mi bf16,
+    // asymmetric groups of 16 18.7 -> 14.7 us), unless that means one more round of tiles (8 x 3,000,008 bf16, 367 tiles: 4 bits, groups
+    // of 8 14.6 us on 296 places, 12.6 on 444; block-scaled FP8 10.5 and 9.4). Since sums settle their addresses once, the difference
+    // is within 0.2 us for 4-bit digits in groups of 32 and more, and for TACO. ZFP, integer work throughout: always.
     const long items = tiles * chunks, few = (long)smCount() * C::kSumBlocks, many = (long)smCount() * C::kDecodeBlocks;
     const bool sum = reduce > 1 && (a.codec.kind == kCodecZfp || items <= few ||
                                     (!kSumsOneRound<C> && (items + few - 1) / few == (items + many - 1) / many));

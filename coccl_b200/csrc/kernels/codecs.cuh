@@ -285,9 +285,9 @@ struct SdpCodec {
   static constexpr bool kRotated = HAD;
   static constexpr int kMinBlocks = 3;  // resident CTAs per SM the fused kernels are compiled for
   // The same for the stand-alone kernels: encode, decode of one copy, sum of several (codec_kernels.cu says which sums). Eight
-  // chunks of 4 Mi bf16, one CTA an SM fewer against these: 4 bits, groups of 128: encode 19.4 against 19.1 us, decode 22.2
-  // against 20.3; 4 bits, groups of 8: 29.5 (three) and 31.2 (four), 26.1 and 23.1; 8 bits, asymmetric groups of 8, whose
-  // parameters do not fit 80 registers beside a run: 35.6 (three) and 39.8 (four), 28.9 (two) and 32.8 (three).
+  // chunks of 4 Mi bf16, one CTA an SM fewer, these, one more: 4 bits, groups of 128: encode 20.8, 20.9, 20.9 us, decode 16.9, 16.7, 16.7
+  // (four chunks of 16 Mi 37.6, 33.6, 33.1); 4 bits, groups of 8: 31.3, 29.9, 31.1 and 26.9, 24.8, 22.9 (3,000,008 values 16.7, 17.0, 17.2);
+  // 8 bits, asymmetric groups of 8, whose parameters do not fit 80 registers beside a run: 36.5, 37.4, 40.8 and 39.3, 30.9, 34.3.
   static constexpr int kEncodeBlocks = SMALLG ? 3 : 4, kDecodeBlocks = BITS == 8 && SMALLG && ASYM ? 2 : 3, kSumBlocks = 2;
   static constexpr bool kExchanges = false;   // runs of neighbouring lanes through the window
   static constexpr bool kEncodeAhead = !SMALLG;   // collective_kernels.cuh: kEncodeStages
@@ -564,7 +564,7 @@ struct SdpCodec {
 
   // Sum of n copies whose runs and parameters start at pw and pp, `stride` bytes apart, all aligned to ALIGN bytes. Alignment
   // and addresses are settled once per run instead of once per copy. Sums of eight copies with groups of 128, 4 bits, rotated:
-  // 224 -> 146 instructions a run and copy; 8 x 8 Mi fp32 23.5 -> 16.2 us, 8 x 5,000,003 bf16 16.2 -> 11.1 us.
+  // 224 -> 146 instructions a run and copy; 8 x 8 Mi fp32 24.6 -> 16.7 us, 8 x 5,000,003 bf16 16.2 -> 11.5 us.
   static constexpr bool kDirectSums = !SMALLG;
   template <int ALIGN, int B>
   static __device__ __forceinline__ void sumBatches(const uint8_t*& pw, const uint8_t*& pp, long stride, int& n, float mul, uint32_t magic,
@@ -649,7 +649,8 @@ struct MxFp8Codec {
   static constexpr int kWords = 8;
   static constexpr bool kRotated = false;
   static constexpr int kMinBlocks = 3;
-  // 4 x 16 Mi bf16: decode 42.8 us with four, 35.7 with three; 8 x 4 Mi encode 15.7 us with three, 14.6 with four
+  // 4 x 16 Mi bf16: decode 39.2 us with two, 35.7 with three, 39.4 with four; encode 35.4 with three, 34.4 with four, 33.3 with five
+  // (8 x 3,000,008 fp32 22.1, 21.2, 22.9)
   static constexpr int kEncodeBlocks = 4, kDecodeBlocks = 3, kSumBlocks = 2;
   static constexpr bool kExchanges = false;
   static constexpr bool kEncodeAhead = false;
@@ -710,19 +711,6 @@ struct MxFp8Codec {
     uint32_t biased;
     bool valid;
   };
-  static constexpr int kBatch = 2;
-
-  static __device__ __forceinline__ Raw fetch(const uint8_t* chunk, const ChunkLayout& L, const CodecCfg& /*c*/, long elem,
-                                              float /*mul*/, const float* /*sm*/ = nullptr) {
-    Raw r;
-    r.valid = elem < L.groups * 32;
-    if (!r.valid) return r;
-    const uint8_t* pw = chunk + elem;
-    loadWords(pw, r.w);
-    r.biased = __ldcg(chunk + L.payloadBytes + elem / 32);
-    return r;
-  }
-
   static __device__ __forceinline__ void accumulate(const Raw& r, float (&acc)[32]) {
     if (!r.valid) return;
     addRun(r.w, r.biased, acc);
@@ -794,8 +782,8 @@ struct MxFp8Codec {
 // For the next two, E = min(4, G/32) lanes exchange their runs through shared memory, so that each holds the same 32/E places
 // of E runs (the "spread" ownership) and finds its partners in its own registers: 16 vector accesses instead of 64 shuffles
 // and as many multiply-adds, and what follows (maxima, FP8, stores) is as easy there. Wider groups use shuffles for the rest.
-// Groups of 128, 8 x 8 Mi fp16: encode 65.3 -> 51.3 us, sum 21.8 -> 19.4 us, re-encoding sum 24.3 -> 15.7 us; 8 x 3,000,008:
-// encode 26.0 -> 21.4 us. (Groups of 64 with their one stage by shuffles: sum of 8 x 3,000,008 12.3 us, 9.2 with the exchange.)
+// Groups of 128, 8 x 8 Mi fp16: encode 65.3 -> 53.7 us, sum 21.8 -> 20.8 us, re-encoding sum 24.3 -> 16.7 us; 8 x 3,000,008:
+// encode 26.0 -> 22.9 us. (Groups of 64 with their one stage by shuffles: sum of 8 x 3,000,008 12.3 us, 9.2 with the exchange.)
 // The group statistics are warp shuffles, so every lane of the warp must call encode() and finish() together. "Rotated domain"
 // here is y / ada = H_G(x) / sqrt(G): independent of the sender's ada, so copies from different ranks add up there and one
 // inverse transform serves the sum; the transform is orthonormal, so mean(x^2) for a re-encode is available without leaving the
@@ -1099,11 +1087,10 @@ struct ZfpCodec {
   static constexpr int kWords = RATE;
   static constexpr bool kRotated = false;
   static constexpr int kMinBlocks = 2;
-  // The coder is a chain of dependent integer work that neither warps nor registers shorten by much (CTA counts compared before
-  // several planes went through one look-up; the ranking was not taken again): eight chunks of 4 Mi fp32,
-  // encode 72.5 us at rate 8 with four CTAs an SM and 71.3 with three, decode 122.0 and 122.7; rate 4 56.0 and 56.0, 77.2 and
-  // 76.2; rate 16 103.5 and 104.2, 189.0 and 186.7 (64 registers spill there: 8 x 4096 values 15.3 against 13.5 us). Sums, which
-  // hold a second run: 79.0 and 73.2 at rate 4, 130.2 and 126.3 at 8, 207.1 and 201.5 at 16.
+  // The coder is a chain of dependent integer work that neither warps nor registers shorten by much: eight chunks of 4 Mi fp32,
+  // encode 71.5 us at rate 8 with four CTAs an SM and 70.0 with three (3,000,008 values 53.8 and 55.4), decode 90.4 and 89.8 (68.0 and
+  // 70.0); rate 4 53.9 and 54.1, 65.3 and 63.8; rate 16 102.7 and 102.9, 139.8 and 138.4 (64 registers spill there: 8 x 262,147 values
+  // 17.8 against 16.5 us). Sums, which hold a second run: 63.9 and 61.8 at rate 4, 92.5 and 86.4 at 8.
   static constexpr int kEncodeBlocks = 4, kDecodeBlocks = RATE == 16 ? 3 : 4, kSumBlocks = 3;
   static constexpr int kMaxBits = 4 * RATE;
   // the plane tables of oracle/zfp1d_planes.h live in the kernel's shared scratch, behind its first 8 floats
@@ -1246,7 +1233,6 @@ __device__ __forceinline__ void decodeSum(const uint8_t* base, long stride, int 
   if constexpr (HasDirectSums<Codec>::value) {
     Codec::sum(base, stride, n, L, c, elem, mul, aligned, spread, acc);
   } else {
-    if constexpr (Codec::kBatch >= 4) decodeBatches<Codec, 4>(base, stride, n, L, c, elem, mul, acc, sm);
     if constexpr (Codec::kBatch >= 2) decodeBatches<Codec, 2>(base, stride, n, L, c, elem, mul, acc, sm);
     decodeBatches<Codec, 1>(base, stride, n, L, c, elem, mul, acc, sm);
   }

@@ -357,8 +357,8 @@ struct CodecArgs {
 
 // These kernels are bound by instruction issue, then by the loads in flight. With packed fp32 arithmetic, digits dequantised
 // where they stand, no divisions and four copies in flight (8 chunks, 4-bit groups of 128, rotated): encode of 256 MiB fp32
-// with stochastic rounding 68.6 -> 54.6 us (290 MB: 44 us to copy), decode + sum 30.6 -> 26.4 us; chunks of 5,000,003 bf16
-// elements (misaligned: see tile_io.cuh) 74.4 -> 30.0 us.
+// with stochastic rounding 68.6 -> 54.6 us, now 52.3 (290 MB: 44 us to copy), decode + sum 30.6 -> 26.4 us, now 16.7 (codecs.cuh, sums);
+// chunks of 5,000,003 bf16 elements (misaligned: see tile_io.cuh) 74.4 -> 30.0 us, now 29.0.
 //
 // whether every encoded input chunk starts on 16 bytes
 __device__ __forceinline__ bool encodedAligned(const CodecArgs& a) {
@@ -430,8 +430,8 @@ __global__ void __launch_bounds__(kTileThreads, Codec::kEncodeBlocks) encodeKern
 }
 
 // out chunk j = decode(in chunk j): one copy (all-gather, all-to-all), for codecs with direct sums. The next tile's words are loaded
-// before this one is transformed and stored (4 bits, groups of 128, rotated: 8 x 8 Mi bf16 40.3 -> 33.0 us, 8 x 5,000,003 29.4 ->
-// 23.9 us). A kernel of its own: in one with the sums' code both spilled (TACO fp32 88 bytes, asymmetric 4 bits 28).
+// before this one is transformed and stored (4 bits, groups of 128, rotated: 8 x 8 Mi bf16 41.5 -> 33.6 us, 8 x 5,000,003 35.1 ->
+// 24.9 us, of which tile_io.cuh has the greater part). A kernel of its own: in one with the sums' code both spilled (TACO fp32 88 bytes, asymmetric 4 bits 28).
 template <typename T, class Codec>
 __global__ void __launch_bounds__(kTileThreads, Codec::kDecodeBlocks) decodeKernel(const CodecArgs a) {
   __shared__ TileStage<T> stage;
