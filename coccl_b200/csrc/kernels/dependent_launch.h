@@ -1,6 +1,6 @@
 // Launches that overlap the end of the kernel before them (programmatic dependent launch).
 //
-// A kernel calls releaseNext() at its start and awaitPrevious() before it touches anything that an earlier kernel of the
+// A kernel calls releaseNext() at its start (the small GEMM behind its main loop) and awaitPrevious() before it touches anything that an earlier kernel of the
 // stream may read or write. Its CTAs then take the places that the CTAs of the kernel before it leave, and set themselves up
 // while the last of those run. awaitPrevious() returns when that kernel has completed and its memory is visible; since that
 // one waited in the same way, everything before it has completed too. Every thread of every kernel that is launched like
